@@ -206,7 +206,7 @@ def autotune_report() -> dict:
 
 
 OPERATOR_FORMS = ("none", "tensor-core split-BF16 product", "FP32 CUDA-core product", "FP64 CUDA-core product",
-                  "FP32 FFT convolution")
+                  "FP32 FFT convolution", "FP64 FFT convolution")
 
 
 def kernel_launch_count() -> int:

@@ -176,6 +176,12 @@ cudaError_t MatFreeOperator<S>::contract_z(int N, cudaStream_t s, bool t_kn) {
                              reinterpret_cast<float*>(Tm), t_kn ? Npad : Kpad, t_kn, s);
     return cudaErrorInvalidValue;
   }
+  if (kind == GEMM_FFT_F64) {
+    if constexpr (sizeof(S) == 8)
+      return launch_fft64_conv(plan64, reinterpret_cast<const double*>(Zr), Kpad, N / 2, spec64,
+                               reinterpret_cast<double*>(Tm), Npad, s);
+    return cudaErrorInvalidValue;
+  }
   return launch_simt_gemm_tn<S>(Vr, Kpad, Zr, Kpad, reinterpret_cast<S*>(Tm), Npad, nk, N, Kpad, s);
 }
 
@@ -187,6 +193,7 @@ double MatFreeOperator<S>::contraction_flops(int N) const {
     const double lg = std::log2((double)fft_p);
     return (N / 2) * ((2.0 * mesh1 + 2.0 * fft_p) * 5.0 * fft_p * lg + 6.0 * fft_p * fft_p);
   }
+  if (kind == GEMM_FFT_F64) return (N / 2) * fft64_column;
   return 2.0 * nk * (double)N * nk;
 }
 
@@ -195,6 +202,7 @@ double MatFreeOperator<S>::contraction_flops(int N) const {
 template <class S>
 double MatFreeOperator<S>::contraction_bytes(int N) const {
   if (kind == GEMM_FFT_F32) return 4.0 * 2.0 * N * nk + 8.0 * (double)fft_p * fft_p;
+  if (kind == GEMM_FFT_F64) return 8.0 * 2.0 * N * nk + 16.0 * (double)fft64_spec_size(plan64);
   return sizeof(S) * ((double)nk * nk + (double)N * nk + (double)nk * N);
 }
 

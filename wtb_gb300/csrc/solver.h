@@ -115,7 +115,8 @@ struct DenseOperator : Operator<S> {
 };
 
 // GEMM_FFT_F32: the contraction as FP32 FFT convolutions over a two-dimensional mesh (k_fftconv.cu)
-enum GemmKind { GEMM_TC_BF16 = 0, GEMM_SIMT_F32 = 1, GEMM_SIMT_F64 = 2, GEMM_FFT_F32 = 3 };
+// (GEMM_FFT_F64: in FP64 over a mesh of any dimension, k_fft64.cu)
+enum GemmKind { GEMM_TC_BF16 = 0, GEMM_SIMT_F32 = 1, GEMM_SIMT_F64 = 2, GEMM_FFT_F32 = 3, GEMM_FFT_F64 = 4 };
 
 // Event pairs around the contraction launches (enabled by wtb_profile_enable).
 struct KernelProfile {
@@ -165,6 +166,10 @@ struct MatFreeOperator : Operator<S> {
   int mesh1 = 0, mesh2 = 0, fft_p = 0;
   const float2* fft_spec = nullptr;
   const float2* fft_tw = nullptr;
+  // FP64 FFT kind: its plan, spectrum and FP64 instructions per complex column
+  Fft64Plan plan64;
+  const zd* spec64 = nullptr;
+  double fft64_column = 0.0;
   DevStatus* st = nullptr;
   KernelProfile* prof = nullptr;
   std::map<long, TcGemmPlan*> plans;  // keyed by (N of the chunk, slice products)
@@ -195,7 +200,8 @@ struct MatFreeOperator : Operator<S> {
                           (uint64_t)(uintptr_t)Vs, (uint64_t)(uintptr_t)Zs,
                           (uint64_t)(uintptr_t)Vr, (uint64_t)(uintptr_t)Zr, (uint64_t)(uintptr_t)Tm,
                           (uint64_t)(uintptr_t)st, (uint64_t)mesh1, (uint64_t)mesh2, (uint64_t)fft_p,
-                          (uint64_t)(uintptr_t)fft_spec, (uint64_t)(uintptr_t)fft_tw};
+                          (uint64_t)(uintptr_t)fft_spec, (uint64_t)(uintptr_t)fft_tw, (uint64_t)(uintptr_t)spec64,
+                          (uint64_t)plan64.m[0], (uint64_t)plan64.m[1], (uint64_t)plan64.m[2]};
     sig->insert(sig->end(), v, v + sizeof(v) / sizeof(v[0]));
   }
   // launches the contraction of an ncol-column application (the first phase's slice products) reps times

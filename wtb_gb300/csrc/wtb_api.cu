@@ -406,12 +406,60 @@ int make_operator(wtb_ctx* c, const wtb_bse_params* p, int nbmax, OpBundle* ob, 
     return WTB_OK;
   }
   c->last_form = WTB_FORM_NONE;
+  // FP64 matrix-free operator on a Monkhorst-Pack mesh of any dimension: the same contraction in FP64, faster than the
+  // product at every size measured (9.0 against 75 us at 2 x 2 and w = 6, 17 / 76 at 6 x 6, 79 / 212 at 12 x 12 and
+  // w = 8, 105 / 144 at 5^3, 3.04 / 37.3 ms at 48 x 45 and w = 12).  The rule is one of reproducibility.  A 2D solve
+  // for many excitons takes a dozen iterations or more, and the search directions of its early converged columns
+  // are then rounding noise that the late ones use: any other rounding of T moves the activities by 1e-9 to 3e-8
+  // relative (within what the 1e-8 residual leaves open, and the same between the dense and the matrix-free product),
+  // on 14 % of the strained systems at 24 x 24 with 10 excitons and 80 % at 32 x 33 with 12.  With up to 6 excitons,
+  // and on 3D meshes, the solve ends before that (differences of 1e-13 to 1e-10), and from 1,800 k-points on the
+  // product costs 0.3 s a solve and more.  Elsewhere the product stays, and with it every digit of its results.
+  const bool fp64 = p->precision == WTB_PREC_FP64;
+  const bool mesh = c->mesh_mp && p->ngrid[0] == c->ngrid[0] && p->ngrid[1] == c->ngrid[1] &&
+                    p->ngrid[2] == c->ngrid[2] && (long)p->ngrid[0] * p->ngrid[1] * p->ngrid[2] == nk;
+  Fft64Plan plan64;
+  double col64 = 0.0;
+  const bool three_d = p->ngrid[0] > 1 && p->ngrid[1] > 1 && p->ngrid[2] > 1;
+  if (p->op == WTB_OP_MATFREE && fp64 && mesh && (three_d || p->nev <= 6 || nk >= 1800) && !(fft_env && std::strcmp(fft_env, "0") == 0) &&
+      fft64_plan(p->ngrid[0], p->ngrid[1], p->ngrid[2], &plan64, &col64)) {
+    const double* dbl = c->ws.find<double>("recip", 9);
+    if (!dbl) return set_err(c, WTB_ESTATE, "reciprocal vectors not staged");
+    CoulParams cpar = coul_of(c, p);
+    cpar.deriv_r0 = deriv_r0 ? 1 : 0;
+    const long ns = (2L * p->ngrid[0] - 1) * (2L * p->ngrid[1] - 1) * (2L * p->ngrid[2] - 1);
+    double* stn = c->ws.get<double>("vstencil" + tag, ns, &err);
+    zd* work = c->ws.get<zd>("fft64_work", fft64_work_size(plan64), &err);
+    zd* spec = c->ws.get<zd>("fft64_spec" + tag, fft64_spec_size(plan64), &err);
+    CKC(err);
+    CKC(launch_coulomb_stencil(cpar, dbl, stn, c->s));
+    CKC(launch_fft64_spectrum(plan64, stn, work, spec, c->s));
+    const int N = 2 * w * w * nbmax;
+    const int Npad = (N + 255) / 256 * 256;
+    auto op = new MatFreeOperator<double>();
+    ob->o64.reset(op);
+    ob->dE = dE;
+    ob->dim = dim;
+    op->kind = GEMM_FFT_F64;
+    op->nk = nk; op->nv = nv; op->nc = nc; op->w = w; op->nbmax = nbmax;
+    op->vec_win = vec_win; op->dE = dE; op->st = c->st; op->msg = &ob->msg; op->prof = &c->prof;
+    op->vec_s = vec_win;
+    op->dE_s = dE;
+    op->Kpad = Kpad; op->Mpad = Mpad; op->Npad = Npad;
+    op->plan64 = plan64;
+    op->spec64 = spec;
+    op->fft64_column = col64;
+    op->Zr = c->ws.get<double>("Zr64", (size_t)Npad * Kpad, &err, true);
+    op->Tm = c->ws.get<double>("T64", (size_t)Mpad * Npad, &err);
+    CKC(err);
+    c->last_form = WTB_FORM_FFT_F64;
+    return WTB_OK;
+  }
   double* V = c->ws.get<double>("V" + tag, (size_t)Mpad * Kpad, &err, true);
   CKC(err);
   CKR(coulomb_table_into(c, p, V, Kpad, deriv_r0));
   ob->dE = dE;
   ob->dim = dim;
-  const bool fp64 = p->precision == WTB_PREC_FP64;
   if (p->op == WTB_OP_DENSE) {
     if (fp64) {
       zd* H = c->ws.get<zd>("H64", (size_t)dim * dim, &err);

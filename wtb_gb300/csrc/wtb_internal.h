@@ -143,6 +143,22 @@ cudaError_t launch_fft_spectrum(const double* stencil, int n1, int n2, int P, zd
                                 cudaStream_t s);
 cudaError_t launch_fft_conv(const float* Z, int ldz, int npairs, int n1, int n2, int P, const float2* spec,
                             const float2* tw, float* T, int ldt, bool t_kn, cudaStream_t s);
+// FP64 form of the contraction on a one-, two- or three-dimensional mesh (k_fft64.cu): the mesh with unit dimensions
+// dropped (m[0] = outermost), the transform lengths P = R1 R2 per dimension, the planes a batch and the shared memory
+// of a CTA.  fft64_plan: false where the mesh does not fit; *per_column the FP64 instructions of one complex column.
+// spec: fft64_spec_size complex, work: fft64_work_size complex; the conv takes Z as launch_fft_conv does and writes
+// T[k][2q + (0, 1)] (row k at T + k ldt).
+struct Fft64Plan {
+  int m[3] = {1, 1, 1}, P[3] = {1, 1, 1}, R1[3] = {1, 1, 1}, R2[3] = {1, 1, 1};
+  int batch = 1;
+  size_t smem = 0;
+};
+bool fft64_plan(int n1, int n2, int n3, Fft64Plan* pl, double* per_column);
+size_t fft64_spec_size(const Fft64Plan& pl);
+size_t fft64_work_size(const Fft64Plan& pl);
+cudaError_t launch_fft64_spectrum(const Fft64Plan& pl, const double* stencil, zd* work, zd* spec, cudaStream_t s);
+cudaError_t launch_fft64_conv(const Fft64Plan& pl, const double* Z, int ldz, int npairs, const zd* spec, double* T,
+                              int ldt, cudaStream_t s);
 cudaError_t launch_coulomb_mesh(const CoulParams& p, const double* bl, double* stencil, double* V, int ldv,
                                 cudaStream_t s);
 // Transition energies dE[I] = E_c - E_v.
