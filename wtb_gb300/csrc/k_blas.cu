@@ -205,6 +205,128 @@ __global__ void __launch_bounds__(256) gram_pair_partial_kernel(const cplx<S>* _
     }
 }
 
+// FP64 Grams: out = A^H B, or with PAIR A^H A and A^H B in one launch (out2 the second).  The FP64 pipe (2 multiply-adds
+// a clock and SM, a warp instruction occupies a quarter of it for 64 clocks) bounds them, so what counts is that every
+// SM has entries to add up, not the loads: the grid is reduction part x chunk of the output's entries, each CTA
+// which stages its part's rows for 256 threads of NE entries (NC = 2), or for small problems of one real component of an
+// entry (NC = 1: a part's chain of 192 rows then takes two multiply-adds a row, and a single part of a 48-column
+// pair spreads over 36 CTAs).  Every component is added in the row order of gram_partial_kernel with the same
+// operations, so the partials are bitwise those of one CTA per part.  Pair of 48 columns: 2,304 rows 868 -> 75 us
+// (12 parts: 12 CTAs before; a floor of 68), 34,560 rows 1,727 -> 1,063 us (a floor of 1,010); X^H [W P] there
+// 388 -> 128 us (112).
+template <int NC, int NE, bool PAIR>
+__global__ void __launch_bounds__(256) gram64_kernel(const zd* __restrict__ A, int lda, int p, const zd* __restrict__ B,
+                                                     int ldb, int q, int nrow, double* __restrict__ partial,
+                                                     int rows_per_part, int npart, BatchMap bm, int RT) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int W = p + q, tid = threadIdx.x;
+  zd* rows = reinterpret_cast<zd*>(smem_raw);  // two stages of RT rows: [2][RT][p of A, then q of B]
+  const float r_W = 1.0f / (float)W;
+  long r_begin, r_end;
+  const int sys = bm_part(bm, blockIdx.x, nrow, rows_per_part, &r_begin, &r_end);
+  if (bm_frozen(bm, sys)) return;
+  auto stage = [&](int buf, long r0) {
+    const int nr = (int)min((long)RT, r_end - r0);
+    for (int e = tid; e < nr * W; e += blockDim.x) {
+      const int rr = qdiv(e, r_W), c = e - rr * W;
+      cp_async_elem<16>(rows + (buf * RT + rr) * W + c, c < p ? A + (r0 + rr) * lda + c : B + (r0 + rr) * ldb + c - p);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // entry t of this thread: columns ia of A and jb of the staged row (A's again for the first matrix of a pair)
+  const int n = p * q, items = (PAIR ? 2 : 1) * n * (NC == 1 ? 2 : 1);
+  int ia[NE], jb[NE], im[NE];
+  double re[NE], imv[NE];
+#pragma unroll
+  for (int t = 0; t < NE; ++t) {
+    const int e = (blockIdx.y * NE + t) * blockDim.x + tid;
+    int x = e < items ? e : 0;
+    im[t] = 0;
+    if (NC == 1) {
+      im[t] = x >= items / 2;
+      x -= im[t] * (items / 2);
+    }
+    const bool second = !PAIR || x >= n;
+    if (PAIR && second) x -= n;
+    ia[t] = x / q;
+    jb[t] = x - ia[t] * q + (second ? p : 0);
+    re[t] = imv[t] = 0.0;
+  }
+  const long nst = (r_end - r_begin + RT - 1) / RT;
+  if (nst > 0) stage(0, r_begin);
+  for (long s = 0; s < nst; ++s) {
+    const int buf = (int)(s & 1);
+    if (s + 1 < nst) {
+      stage(buf ^ 1, r_begin + (s + 1) * RT);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const int nr = (int)min((long)RT, r_end - (r_begin + s * RT));
+    const zd* row = rows + buf * RT * W;
+#pragma unroll 4
+    for (int rr = 0; rr < nr; ++rr, row += W) {
+#pragma unroll
+      for (int t = 0; t < NE; ++t) {
+        const zd a = row[ia[t]];
+        if (NC == 2) {
+          const zd b = row[jb[t]];
+          re[t] = fma(a.re, b.re, re[t]);
+          re[t] = fma(a.im, b.im, re[t]);
+          imv[t] = fma(a.re, b.im, imv[t]);
+          imv[t] = fma(-a.im, b.re, imv[t]);
+        } else {
+          // one component, (re, re) + (im, im) or (re, im) - (im, re): chosen by address, and the sign of a.im by its
+          // sign bit, so that no FP64 instruction is spent on either
+          const double* b = reinterpret_cast<const double*>(row + jb[t]);
+          const double ai = __hiloint2double(__double2hiint(a.im) ^ (im[t] << 31), __double2loint(a.im));
+          re[t] = fma(a.re, b[im[t]], re[t]);
+          re[t] = fma(ai, b[im[t] ^ 1], re[t]);
+        }
+      }
+    }
+    __syncthreads();  // the next stage's copies overwrite this buffer
+  }
+#pragma unroll
+  for (int t = 0; t < NE; ++t) {
+    const int e = (blockIdx.y * NE + t) * blockDim.x + tid;
+    if (e >= items) continue;
+    const int jj = jb[t] < p && PAIR ? jb[t] : jb[t] - p;
+    const bool second = PAIR && jb[t] >= p;
+    double* out = partial + ((size_t)(second ? npart : 0) + blockIdx.x) * n * 2 + 2 * (ia[t] * q + jj);
+    if (NC == 2) {
+      out[0] = re[t];
+      out[1] = imv[t];
+    } else {
+      out[im[t]] = re[t];
+    }
+  }
+}
+
+// Entries in twos where that still gives every SM eight CTAs, single ones where it gives six, else components.
+template <bool PAIR>
+cudaError_t run_gram64(const zd* A, int lda, int p, const zd* B, int ldb, int q, int nrow, double* partial, int rpp,
+                       int npart, cudaStream_t s, const BatchMap& bm) {
+  const int n = (PAIR ? 2 : 1) * p * q;
+  auto run = [&](auto kernel, int per_thread, int nt, int total, int rt) {
+    const size_t smem = (size_t)2 * rt * (p + q) * sizeof(zd);
+    const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(kernel), smem);
+    if (e != cudaSuccess) return e;
+    const int chunk = per_thread * nt;
+    kernel<<<dim3(npart, (total + chunk - 1) / chunk), nt, smem, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, npart,
+                                                                      bm, rt);
+    ++g_launch_count;
+    return cudaGetLastError();
+  };
+  if ((long)npart * ((n + 511) / 512) >= 152 * 8) return run(gram64_kernel<2, 2, PAIR>, 2, 256, n, 8);
+  if ((long)npart * ((n + 255) / 256) >= 152 * 6) return run(gram64_kernel<2, 1, PAIR>, 1, 256, n, 8);
+  // few parts: 16 rows a stage, since a stage's copies take longer than its multiply-adds; for one or two parts a
+  // warp or two on every SM rather than eight on a few, and 32 rows (as far as 192 columns: 196 KB)
+  if ((long)npart * n >= 152 * 64) return run(gram64_kernel<1, 1, PAIR>, 1, 256, 2 * n, 16);
+  return run(gram64_kernel<1, 1, PAIR>, 1, 64, 2 * n, 32);
+}
+
 // The Gram pair for 33..48 FP32 columns over the upper triangle only (M and G are Hermitian: the lower triangle is
 // the conjugate, written by sum_partials_herm_kernel).  The 48 x 48 matrices are 16 x 16 blocks of 3 x 3; thread
 // t < 136 owns upper block t (block row a <= block column b) of both, so a staged row costs it the same 9
@@ -1029,17 +1151,22 @@ cudaError_t launch_gram(const cplx<S>* A, int lda, int p, const cplx<S>* B, int 
   if (p > 96 || q > 96) return cudaErrorInvalidValue;
   if (bm.parts) npart = bm.nparts;
   const int rpp = (nrow + npart - 1) / npart;
-  const int ti = (std::max(p, q) + 15) / 16;
-  switch (ti) {
-    case 1: gram_partial_kernel<S, 1><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
-    case 2: gram_partial_kernel<S, 2><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
-    case 3: gram_partial_kernel<S, 3><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
-    case 4: gram_partial_kernel<S, 4><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
-    case 5: gram_partial_kernel<S, 5><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
-    default: gram_partial_kernel<S, 6><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
-  }
-  ++g_launch_count;
   const int n = p * q * 2;
+  if constexpr (sizeof(S) == 8) {
+    const cudaError_t e = run_gram64<false>(A, lda, p, B, ldb, q, nrow, partial, rpp, npart, s, bm);
+    if (e != cudaSuccess) return e;
+  } else {
+    const int ti = (std::max(p, q) + 15) / 16;
+    switch (ti) {
+      case 1: gram_partial_kernel<S, 1><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
+      case 2: gram_partial_kernel<S, 2><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
+      case 3: gram_partial_kernel<S, 3><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
+      case 4: gram_partial_kernel<S, 4><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
+      case 5: gram_partial_kernel<S, 5><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
+      default: gram_partial_kernel<S, 6><<<npart, 256, 0, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, bm); break;
+    }
+    ++g_launch_count;
+  }
   sum_partials_kernel<<<dim3((n + 31) / 32, bm.nsys), 256, 0, s>>>(partial, npart, n, reinterpret_cast<double*>(out),
                                                                     bm, 2 * out_stride);
   ++g_launch_count;
@@ -1063,13 +1190,18 @@ cudaError_t launch_gram_pair(const cplx<S>* A, const cplx<S>* B, int ld, int p, 
       return cudaGetLastError();
     }
   }
-  const int ti = (p + 15) / 16;
-  switch (ti) {
-    case 1: gram_pair_partial_kernel<S, 1><<<npart, 256, 0, s>>>(A, B, ld, p, nrow, partial, rpp, npart, bm); break;
-    case 2: gram_pair_partial_kernel<S, 2><<<npart, 256, 0, s>>>(A, B, ld, p, nrow, partial, rpp, npart, bm); break;
-    default: gram_pair_partial_kernel<S, 3><<<npart, 256, 0, s>>>(A, B, ld, p, nrow, partial, rpp, npart, bm); break;
+  if constexpr (sizeof(S) == 8) {
+    const cudaError_t e = run_gram64<true>(A, ld, p, B, ld, p, nrow, partial, rpp, npart, s, bm);
+    if (e != cudaSuccess) return e;
+  } else {
+    const int ti = (p + 15) / 16;
+    switch (ti) {
+      case 1: gram_pair_partial_kernel<S, 1><<<npart, 256, 0, s>>>(A, B, ld, p, nrow, partial, rpp, npart, bm); break;
+      case 2: gram_pair_partial_kernel<S, 2><<<npart, 256, 0, s>>>(A, B, ld, p, nrow, partial, rpp, npart, bm); break;
+      default: gram_pair_partial_kernel<S, 3><<<npart, 256, 0, s>>>(A, B, ld, p, nrow, partial, rpp, npart, bm); break;
+    }
+    ++g_launch_count;
   }
-  ++g_launch_count;
   const int n = p * p * 2;
   // both sets in one launch (the G partials keep the part numbering, npart parts further on)
   sum_partials_kernel<<<dim3((n + 31) / 32, bm.nsys, 2), 256, 0, s>>>(partial, npart, n,
