@@ -1,0 +1,55 @@
+"""The dense Hermitian eigensolver at the edges of its tiles (64) and panels (32), on matrices that reach its special
+cases: reducible ones, zero columns (reflectors that do nothing), low rank, entries of very different sizes.  Against
+LAPACK; the bound is the backward error of a stable reduction, n eps ||A|| for the eigenvalues and 8 sqrt(n) eps ||A||_F
+for the residuals."""
+import os
+import sys
+
+import numpy as np
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+sys.path.insert(0, ROOT)
+
+from wtb_gb300 import api  # noqa: E402
+
+pytestmark = pytest.mark.gpu
+EPS = np.finfo(np.float64).eps
+
+
+def matrix(n, kind):
+    rng = np.random.default_rng(n)
+    X = rng.normal(size=(n, n)) + 1j * rng.normal(size=(n, n))
+    A = (X + X.conj().T) / 2
+    if kind == "dominant":
+        return 1e-3 * A + np.diag(rng.uniform(1.5, 8.0, n))
+    if kind == "graded":
+        s = 10.0 ** rng.uniform(-8.0, 0.0, n)
+        return A * s[:, None] * s[None]
+    if kind == "low rank":
+        return X[:, :3] @ X[:, :3].conj().T
+    if kind == "reducible":
+        A[: n // 2, n // 2:] = 0.0
+        A[n // 2:, : n // 2] = 0.0
+    if kind == "diagonal":
+        return np.diag(rng.normal(size=n)).astype(complex)
+    return np.zeros_like(A) if kind == "zero" else A
+
+
+@pytest.mark.parametrize("kind", ["random", "dominant", "graded", "low rank", "reducible", "diagonal", "zero"])
+@pytest.mark.parametrize("n", [1, 2, 31, 32, 33, 34, 64, 65, 66, 97, 129, 200])
+def test_eigenvalues(ctx, n, kind):
+    A = matrix(n, kind)
+    W, ref = ctx.zheev(A), np.linalg.eigvalsh(A)
+    assert np.abs(W - ref).max() <= max(n, 4) * EPS * np.abs(ref).max() + 1e-300
+
+
+@pytest.mark.parametrize("kind", ["random", "dominant", "reducible"])
+@pytest.mark.parametrize("n", [2, 33, 65, 200, 333])
+def test_eigenpairs(ctx, n, kind):
+    A = matrix(n, kind)
+    W, Z = ctx.zheev_vectors(A)
+    nrm = np.linalg.norm(A)
+    assert np.linalg.norm(A @ Z - Z * W) <= 8.0 * np.sqrt(n) * EPS * nrm
+    # eigenvectors of values closer than 1e-7 ||A|| are orthogonalised, the others by their gaps (eps / 1e-7)
+    assert np.abs(Z.conj().T @ Z - np.eye(n)).max() <= 1e-8

@@ -1,16 +1,15 @@
 // All eigenvalues of a dense Hermitian matrix on the device: the stand-in for the LAPACK ZHEEV calls of the
 // full-spectrum paths (bsebnds, src/module_bse.F90:1427-1448; the temperature solver's dense path).
 //
-// 1. Householder tridiagonalisation A = Q T Q^H in FP64, the unblocked zhetd2 sequence (lower form): for
-//    column j, the reflector H = I - tau v v^H of zlarfg annihilates A(j+2:n, j); x = tau A22 v;
-//    w = x - (tau/2)(x^H v) v; A22 -= v w^H + w v^H, on the lower triangle only.  Four launches per column:
-//    the reflector (one CTA), the Hermitian product by 64 x 64 lower tiles (each off-diagonal tile staged
-//    in shared memory serves A v and A^H v), the fixed-order sum of the tile partials with the x^H v dots,
-//    and the rank-2 update of the lower tiles.  On this GPU the FP64 pipe, not HBM, bounds both: 8 FMAs per
-//    stored element and column, 8/3 n^3 FMAs in all.
-// 2. Eigenvalues of the real symmetric tridiagonal T by bisection on Sturm counts (dstebz's method), as
-//    multisection with a few lanes per eigenvalue index where n alone would leave SMs idle, the count with
-//    LAPACK's pivot guard pivmin, to the FP64 resolution of the Gershgorin interval.  Backward stable: |lambda - lambda_exact| <~ n eps ||A||.
+// 1. Householder tridiagonalisation A = Q T Q^H, lower form, blocked as LAPACK's zhetrd: within a panel of 32 columns
+//    the trailing matrix is left as it was, a column is brought up to date from the panel's v and w, and its Hermitian
+//    product is corrected by them; after the panel the trailing matrix takes all 32 rank-2 updates at once.  Three
+//    launches a column (the column and the w before it; the Hermitian product by 64 x 64 lower tiles; x) and one a
+//    panel.  8/3 n^3 multiply-adds: on the FP64 pipe 62 ms at n = 2,304, so the Hermitian product and the trailing
+//    update run as exact integer sums of quantised components (below), the rest in FP64.
+// 2. Eigenvalues of the real symmetric tridiagonal T by bisection on Sturm counts, as multisection with a few lanes
+//    per eigenvalue index where n alone would leave SMs idle, to the FP64 resolution of the Gershgorin interval.
+//    Backward stable: |lambda - lambda_exact| <~ n eps ||A||.
 #include <cfloat>
 
 #include "wtb_internal.h"
@@ -19,24 +18,57 @@ namespace wtb {
 
 namespace {
 
-// Tile edge of the Hermitian product and the rank-2 update: 64 while the trailing block gives at least three
-// tiles per SM, then 32, then 16 (the late columns would otherwise run on a handful of CTAs).
-constexpr int kMinTiles = 3 * 152;
-inline int pick_tile(int m) {
-  auto tiles = [m](int t) { const long nt = (m + t - 1) / t; return nt * (nt + 1) / 2; };
-  if (tiles(64) >= kMinTiles) return 64;
-  if (tiles(32) >= kMinTiles) return 32;
-  return 16;
+constexpr int kT = 64;    // tile edge of the Hermitian product and the trailing update (absolute tile grid)
+constexpr int kNB = 32;   // reflectors a panel
+constexpr int kQ = 55;    // bits of a quantised component
+constexpr int kExpBad = 100000, kExpZero = -4096;
+
+inline int tiles_of(int n) { return (n + kT - 1) / kT; }
+inline size_t lower_tiles(int nT) { return (size_t)nT * (nT + 1) / 2; }
+
+// Quantised arithmetic.  An FP64 warp instruction holds the SM's FP64 pipe for 19 clocks (1.7 lanes a clock), a 32 x 32 +
+// 64-bit integer multiply-add for about 1.5, so the products of the reduction run as integers: a component x of a group
+// with a common exponent, |x| < 2^ex, is the integer q = rint(x 2^(55 - ex)) = hi 2^28 + lo, |hi| <= 2^27,
+// |lo| <= 2^27, and a product takes three multiply-adds (hi hi; hi lo + lo hi; lo lo is below 2^-56 of the largest).
+// Every sum of a tile is exact in 64 bits (at most 128 products of 2^54), so the only errors are those of q, 2^-56 of
+// the group's largest component, eight times below FP64's own rounding of one product of that size.
+__device__ __forceinline__ int exponent_of(double x) { return (__double2hiint(x) >> 20) & 0x7ff; }  // biased
+
+// the biased exponent field of the group's largest component -> ex with |x| < 2^ex
+__device__ __forceinline__ int group_ex(int field) {
+  return field == 0x7ff ? kExpBad : field == 0 ? kExpZero : field - 1022;
 }
-// partial-sum buffer: (tiles per column) x m entries, largest over the three tile sizes (from m = 4096 on the
-// tile is always 64)
-inline size_t p_capacity(int n) {
-  size_t cap = (size_t)((n + 63) / 64) * n;
-  for (int m = 1; m < std::min(n, 4096); ++m) {
-    const int t = pick_tile(m);
-    cap = std::max(cap, (size_t)((m + t - 1) / t) * m);
-  }
-  return cap;
+__device__ __forceinline__ int2 quantise(double x, int ex) {
+  const long long b = __double_as_longlong(x);
+  const int f = (int)((b >> 52) & 0x7ff);
+  long long m = (b & 0xfffffffffffffll) | 0x10000000000000ll;  // x = m 2^(f - 1075)
+  const int sh = f - 1075 + kQ - ex;                            // <= 2 for |x| < 2^ex
+  if (f == 0 || ex >= kExpBad || sh < -54) return make_int2(0, 0);
+  if (sh >= 0)
+    m <<= sh;
+  else
+    m = (m + (1ll << (-sh - 1))) >> -sh;
+  if (b < 0) m = -m;
+  const int hi = (int)((m + (1ll << 27)) >> 28);
+  return make_int2(hi, (int)(m - ((long long)hi << 28)));
+}
+__device__ __forceinline__ int4 quantise(zd x, int ex) {
+  const int2 r = quantise(x.re, ex), i = quantise(x.im, ex);
+  return make_int4(r.x, r.y, i.x, i.y);
+}
+// 2^e (0 below the range, infinity above; NaN for a group with a component that is not finite)
+__device__ __forceinline__ double pow2(int e) {
+  if (e > kExpBad / 2) return __longlong_as_double(0x7ff8000000000000ll);
+  return scalbn(1.0, e);
+}
+// an exact sum of products hh 2^56 + cr 2^28 of groups with exponents adding to e, as a double
+__device__ __forceinline__ double from_sums(long long hh, long long cr, double s56, double s28) {
+  return fma((double)hh, s56, (double)cr * s28);
+}
+__device__ __forceinline__ void mac(long long& hh, long long& cr, int ah, int al, int bh, int bl) {
+  hh += (long long)ah * bh;
+  cr += (long long)ah * bl;
+  cr += (long long)al * bh;
 }
 
 // zlarfg for x = A(j+1:n, j): returns tau, beta and the scale 1/(alpha - beta) applied to x(2:m).
@@ -73,150 +105,15 @@ __device__ __forceinline__ void lower_tile(int b, int* R, int* C) {
   *C = b - r * (r + 1) / 2;
 }
 
-// zlarfg on column j (one CTA): v(0) = 1, v(1:) = x(1:) / (alpha - beta), stored in v and below the
-// subdiagonal of column j; tau(j), e(j) = beta.
-__global__ void __launch_bounds__(256) tri_reflector_kernel(zd* __restrict__ A, int n, int lda, int j,
-                                                            zd* __restrict__ v, zd* __restrict__ tau_out,
-                                                            double* __restrict__ e_out) {
-  __shared__ double red[8];
-  __shared__ zd s_scale;
-  __shared__ int s_skip;
-  const int m = n - j - 1;
-  zd* x = A + (size_t)j * lda + j + 1;
-  double s2 = 0.0;
-  for (int i = 1 + threadIdx.x; i < m; i += blockDim.x) s2 = fma(x[i].re, x[i].re, fma(x[i].im, x[i].im, s2));
-  for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s2;
-  __syncthreads();
-  // the scalar FP64 work (sqrt, divisions) on one thread: every warp repeating it would queue on the FP64 pipe
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    const Reflector R = make_reflector(x[0], t);
-    tau_out[j] = R.tau;
-    e_out[j] = R.beta;
-    s_scale = R.scale;
-    s_skip = R.tau.re == 0.0 && R.tau.im == 0.0;
-  }
-  __syncthreads();
-  if (s_skip) return;
-  const zd sc = s_scale;
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    const zd vi = i == 0 ? mk<double>(1.0, 0.0) : cmul(x[i], sc);
-    v[i] = vi;
-    x[i] = vi;
-  }
-}
-
-// Lower-triangle Hermitian product p = A22 v by tiles: an off-diagonal tile (R, C) gives A_RC v_C to the rows of
-// block R and A_RC^H v_R to the rows of block C; a diagonal tile supplies its upper half from the lower one.
-// Each (row block, other block) pair receives exactly one partial, P[other][row], so the sum over the tile
-// index is a fixed-order reduction.  4T threads: row (or column) t % T, a quarter of the tile's width each.
-template <int T>
-__global__ void __launch_bounds__(4 * T) tri_symv_kernel(const zd* __restrict__ A, int n, int lda, int j,
-                                                         const zd* __restrict__ v, const zd* __restrict__ tau_p,
-                                                         zd* __restrict__ P) {
-  constexpr int kSymTile = T, kTPad = T + 1;  // padded column stride: conflict-free transposed reads
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  zd* tile = reinterpret_cast<zd*>(smem_raw);    // [kSymTile][kTPad], column-major
-  zd* vR = tile + kSymTile * kTPad;
-  zd* vC = vR + kSymTile;
-  zd* ry = vC + kSymTile;                         // [4][kSymTile]
-  zd* rz = ry + 4 * kSymTile;                     // [4][kSymTile]
-  const zd tau = tau_p[j];
-  if (tau.re == 0.0 && tau.im == 0.0) return;
-  const int m = n - j - 1;
-  int R, C;
-  lower_tile(blockIdx.x, &R, &C);
-  const int r0 = R * kSymTile, c0 = C * kSymTile;
-  const zd* a22 = A + (size_t)(j + 1) * lda + j + 1;
-  for (int e = threadIdx.x; e < kSymTile * kSymTile; e += blockDim.x) {
-    const int ii = e % kSymTile, jj = e / kSymTile;
-    const int r = r0 + ii, c = c0 + jj;
-    tile[jj * kTPad + ii] = (r < m && c < m) ? a22[(size_t)c * lda + r] : mk<double>(0.0, 0.0);
-  }
-  if (threadIdx.x < kSymTile) {
-    const int r = r0 + threadIdx.x, c = c0 + threadIdx.x;
-    vR[threadIdx.x] = r < m ? v[r] : mk<double>(0.0, 0.0);
-    vC[threadIdx.x] = c < m ? v[c] : mk<double>(0.0, 0.0);
-  }
-  __syncthreads();
-  const bool diag = R == C;
-  const int i = threadIdx.x % kSymTile, g = threadIdx.x / kSymTile;
-  const int q0 = g * (kSymTile / 4), q1 = q0 + kSymTile / 4;
-  zd acc = mk<double>(0.0, 0.0);
-  if (!diag) {
-    for (int jj = q0; jj < q1; ++jj) cfma(acc, tile[jj * kTPad + i], vC[jj]);
-  } else {
-    for (int jj = q0; jj < q1; ++jj) {
-      zd a;
-      if (jj < i)
-        a = tile[jj * kTPad + i];
-      else if (jj == i)
-        a = mk<double>(tile[i * kTPad + i].re, 0.0);
-      else
-        a = cconj(tile[i * kTPad + jj]);
-      cfma(acc, a, vC[jj]);
-    }
-  }
-  ry[g * kSymTile + i] = acc;
-  if (!diag) {
-    zd accz = mk<double>(0.0, 0.0);
-    for (int ii = q0; ii < q1; ++ii) cfmac(accz, tile[i * kTPad + ii], vR[ii]);  // conj(A(ii, i)) vR(ii)
-    rz[g * kSymTile + i] = accz;
-  }
-  __syncthreads();
-  if (threadIdx.x < kSymTile) {
-    const int t = threadIdx.x;
-    zd y = ry[t];
-    for (int q = 1; q < 4; ++q) y = cadd(y, ry[q * kSymTile + t]);
-    if (r0 + t < m) P[(size_t)C * m + r0 + t] = y;
-  } else if (!diag && threadIdx.x < 2 * kSymTile) {
-    const int t = threadIdx.x - kSymTile;
-    zd z = rz[t];
-    for (int q = 1; q < 4; ++q) z = cadd(z, rz[q * kSymTile + t]);
-    if (c0 + t < m) P[(size_t)R * m + c0 + t] = z;
-  }
-}
-
-// x = tau sum_k P[k] and the partial dots conj(x) . v of each CTA.  256 threads = 32 rows x 8 slices of the
-// tile index (slice l sums k = l, l+8, ...), the slices then added in order: a fixed-order sum whose serial
-// chain is nT/8 loads long.
-constexpr int kXRows = 32;
-__global__ void __launch_bounds__(256) tri_x_kernel(const zd* __restrict__ P, int nT, int m,
-                                                    const zd* __restrict__ tau_p, int j, const zd* __restrict__ v,
-                                                    zd* __restrict__ x, zd* __restrict__ dots) {
-  __shared__ zd red[8][kXRows];
-  const zd tau = tau_p[j];
-  if (tau.re == 0.0 && tau.im == 0.0) return;
-  const int rr = threadIdx.x % kXRows, sl = threadIdx.x / kXRows;
-  const int r = blockIdx.x * kXRows + rr;
-  zd p = mk<double>(0.0, 0.0);
-  if (r < m)
-    for (int k = sl; k < nT; k += 8) p = cadd(p, P[(size_t)k * m + r]);
-  red[sl][rr] = p;
-  __syncthreads();
-  if (threadIdx.x < kXRows) {
-    zd t = mk<double>(0.0, 0.0);
-    if (r < m) {
-      zd q = red[0][rr];
-      for (int l = 1; l < 8; ++l) q = cadd(q, red[l][rr]);
-      const zd xr = cmul(tau, q);
-      x[r] = xr;
-      t = cmulc(xr, v[r]);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      t.re += __shfl_xor_sync(0xffffffffu, t.re, o);
-      t.im += __shfl_xor_sync(0xffffffffu, t.im, o);
-    }
-    if (threadIdx.x == 0) dots[blockIdx.x] = t;
-  }
-}
+// The column's reflector: what K2's first CTA leaves for K3.
+struct TriCol {
+  zd tau, sc, om;  // om = 1 - sc alpha: v = sc x + om e_1 for x = A(j+1:n, j)
+};
 
 // alpha = -(tau/2) sum_b dots[b], the sum split over one warp's lanes in a fixed order.
 __device__ __forceinline__ zd her2_alpha(const zd* __restrict__ dots, int ndots, zd tau) {
   zd d = mk<double>(0.0, 0.0);
-  for (int b = threadIdx.x; b < ndots; b += 32) d = cadd(d, dots[b]);
+  for (int b = threadIdx.x & 31; b < ndots; b += 32) d = cadd(d, dots[b]);
   for (int o = 16; o > 0; o >>= 1) {
     d.re += __shfl_xor_sync(0xffffffffu, d.re, o);
     d.im += __shfl_xor_sync(0xffffffffu, d.im, o);
@@ -224,61 +121,383 @@ __device__ __forceinline__ zd her2_alpha(const zd* __restrict__ dots, int ndots,
   return cscale(cmul(tau, d), -0.5);
 }
 
-// A22 -= v w^H + w v^H on the lower triangle, w = x - (tau/2)(x^H v) v formed per tile from x and the dots.
-// Eight FP64 FMAs per element.
-template <int T>
-__global__ void __launch_bounds__(4 * T) tri_her2l_kernel(zd* __restrict__ A, int n, int lda, int j,
-                                                          const zd* __restrict__ tau_p, const zd* __restrict__ v,
-                                                          const zd* __restrict__ x, const zd* __restrict__ dots,
-                                                          int ndots) {
-  constexpr int kSymTile = T;
+__device__ __forceinline__ zd half_warp_sum(zd a) {
+  for (int o = 8; o > 0; o >>= 1) {
+    a.re += __shfl_xor_sync(0xffffffffu, a.re, o);
+    a.im += __shfl_xor_sync(0xffffffffu, a.im, o);
+  }
+  return a;
+}
+
+constexpr int kRows = 16;  // rows of a CTA of the column kernels, 16 lanes each
+
+// K1, column j = j0 + i: w_{i-1} = x - (tau/2)(x^H v) v of the column before, then
+// A(j:n, j) -= sum_{l < i} v_l conj(w_l(j)) + w_l conj(v_l(j)), and the column's norm (rows from j + 2) by CTA.
+__global__ void __launch_bounds__(256) tri_col_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
+                                                      const zd* __restrict__ tau, zd* __restrict__ W,
+                                                      const zd* __restrict__ xw, const zd* __restrict__ dots, int ndots,
+                                                      double* __restrict__ norms) {
+  __shared__ zd vj[kNB], wj[kNB], s_alpha;
+  __shared__ double red[8];
+  const int tid = threadIdx.x, lane = tid & 15, j0 = j - i;
+  if (i > 0 && tid < 32) {
+    const zd al = her2_alpha(dots, ndots, tau[j - 1]);
+    if (tid == 0) s_alpha = al;
+  }
+  __syncthreads();
+  zd alpha = mk<double>(0.0, 0.0);
+  if (i > 0) alpha = s_alpha;
+  if (tid < i) {
+    const zd v = A[(size_t)(j0 + tid) * lda + j];
+    vj[tid] = v;
+    wj[tid] = tid == i - 1 ? cadd(xw[j], cmul(alpha, v)) : W[(size_t)tid * n + j];
+  }
+  __syncthreads();
+  const int r = j + blockIdx.x * kRows + tid / 16;
+  zd acc = mk<double>(0.0, 0.0);
+  if (r < n)
+    for (int l = lane; l < i; l += 16) {
+      const zd v = A[(size_t)(j0 + l) * lda + r];
+      zd w;
+      if (l == i - 1) {
+        w = cadd(xw[r], cmul(alpha, v));
+        W[(size_t)l * n + r] = w;
+      } else {
+        w = W[(size_t)l * n + r];
+      }
+      cfmac(acc, wj[l], v);
+      cfmac(acc, vj[l], w);
+    }
+  acc = half_warp_sum(acc);
+  double s2 = 0.0;
+  if (lane == 0 && r < n) {
+    zd a = csub(A[(size_t)j * lda + r], acc);
+    if (r == j) a.im = 0.0;
+    A[(size_t)j * lda + r] = a;
+    if (r > j + 1) s2 = fma(a.re, a.re, a.im * a.im);
+  }
+  s2 += __shfl_xor_sync(0xffffffffu, s2, 16);
+  if ((tid & 31) == 0) red[tid >> 5] = s2;
+  __syncthreads();
+  if (tid == 0) {
+    double t = red[0];
+    for (int w = 1; w < 8; ++w) t += red[w];
+    norms[blockIdx.x] = t;
+  }
+}
+
+// K2, with x = A(j+1:n, j) (no scaling of the reflector yet: A v = sc A x + om A(:, j+1)).
+//   CTA 0: the reflector's tau, beta, sc and om.  CTAs 1 .. i: v_l^H x and w_l^H x.
+//   The others, one per lower tile (R, C) of the trailing block: the quantised strict lower triangle's A_RC x_C to
+//   the rows of block R and A_RC^H x_R to the rows of block C, as P[other block][row] (a diagonal tile's second
+//   product as P[nT][row]), each (slot, row) written once.  A thread sums one row (or column) over a quarter of the
+//   tile.  Bound by the integer multiply-adds (24 an element, 21 lanes a clock and SM measured): 22 us at m = 2,304
+//   where the FP64 product took 55, 12.6 us averaged over the columns of n = 2,304.
+__global__ void __launch_bounds__(256) tri_symv_kernel(const zd* __restrict__ A, int n, int lda, int j, int i,
+                                                       const zd* __restrict__ W, const double* __restrict__ norms,
+                                                       int nnorms, const int4* __restrict__ Aq,
+                                                       const int* __restrict__ Aex, TriCol* __restrict__ col,
+                                                       zd* __restrict__ tau_out, double* __restrict__ e_out,
+                                                       zd* __restrict__ g, zd* __restrict__ P) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const zd* x = A + (size_t)j * lda;  // by absolute row, from j + 1
+  if ((int)blockIdx.x <= i) {
+    zd* red = reinterpret_cast<zd*>(smem_raw);
+    if (blockIdx.x == 0) {
+      if (warp == 0) {
+        double t = 0.0;
+        for (int b = lane; b < nnorms; b += 32) t += norms[b];
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) {
+          const Reflector R = make_reflector(x[j + 1], t);
+          tau_out[j] = R.tau;
+          e_out[j] = R.beta;
+          col->tau = R.tau;
+          col->sc = R.scale;
+          const zd sa = cmul(R.scale, x[j + 1]);
+          col->om = mk<double>(1.0 - sa.re, -sa.im);
+        }
+      }
+      return;
+    }
+    const int l = blockIdx.x - 1;
+    const zd* v = A + (size_t)(j - i + l) * lda;
+    const zd* w = W + (size_t)l * n;
+    zd gv = mk<double>(0.0, 0.0), gw = gv;
+    for (int r = j + 1 + tid; r < n; r += 256) {
+      cfmac(gv, v[r], x[r]);
+      cfmac(gw, w[r], x[r]);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+      gv.re += __shfl_xor_sync(0xffffffffu, gv.re, o);
+      gv.im += __shfl_xor_sync(0xffffffffu, gv.im, o);
+      gw.re += __shfl_xor_sync(0xffffffffu, gw.re, o);
+      gw.im += __shfl_xor_sync(0xffffffffu, gw.im, o);
+    }
+    if (lane == 0) {
+      red[2 * warp] = gv;
+      red[2 * warp + 1] = gw;
+    }
+    __syncthreads();
+    if (tid < 2) {
+      zd t = red[tid];
+      for (int q = 1; q < 8; ++q) t = cadd(t, red[2 * q + tid]);
+      g[2 * l + tid] = t;
+    }
+    return;
+  }
+  constexpr int kPad = kT + 1;                       // conflict-free columns and rows
+  int4* tile = reinterpret_cast<int4*>(smem_raw);    // [column][row]
+  int4* xR = tile + kT * kPad;
+  int4* xC = xR + kT;
+  long long* sums = reinterpret_cast<long long*>(xC + kT);  // [4 quarters][4][kT]
+  const int nT = (n + kT - 1) / kT, C0 = (j + 1) / kT;
+  int R, C;
+  lower_tile(blockIdx.x - i - 1, &R, &C);
+  R += C0;
+  C += C0;
+  const size_t t = (size_t)R * (R + 1) / 2 + C;
+  const int4* src = Aq + t * kT * kT;
+  for (int e = tid; e < kT * kT; e += 256)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                     (uint32_t)__cvta_generic_to_shared(tile + (e / kT) * kPad + e % kT)),
+                 "l"(src + e)
+                 : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  __shared__ int s_f[4];  // largest exponent fields of x over the halves of the two blocks
+  zd z = mk<double>(0.0, 0.0);
+  if (tid < 2 * kT) {
+    const int r = (tid < kT ? R : C) * kT + tid % kT;
+    if (r > j && r < n) z = x[r];
+    const int f = __reduce_max_sync(0xffffffffu, max(exponent_of(z.re), exponent_of(z.im)));
+    if (lane == 0) s_f[warp] = f;
+  }
+  __syncthreads();
+  const int exR = group_ex(max(s_f[0], s_f[1])), exC = group_ex(max(s_f[2], s_f[3]));
+  if (tid < 2 * kT) (tid < kT ? xR : xC)[tid % kT] = quantise(z, tid < kT ? exR : exC);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  const int row = tid % kT, q0 = (tid / kT) * (kT / 4);
+#pragma unroll 1
+  for (int second = 0; second < 2; ++second) {
+    long long rh = 0, rc = 0, ih = 0, ic = 0;
+    if (!second) {
+#pragma unroll 4
+      for (int c = q0; c < q0 + kT / 4; ++c) {  // a x
+        const int4 a = tile[c * kPad + row], b = xC[c];
+        mac(rh, rc, a.x, a.y, b.x, b.y);
+        mac(rh, rc, -a.z, -a.w, b.z, b.w);
+        mac(ih, ic, a.x, a.y, b.z, b.w);
+        mac(ih, ic, a.z, a.w, b.x, b.y);
+      }
+    } else {
+#pragma unroll 4
+      for (int r = q0; r < q0 + kT / 4; ++r) {  // conj(a) x
+        const int4 a = tile[row * kPad + r], b = xR[r];
+        mac(rh, rc, a.x, a.y, b.x, b.y);
+        mac(rh, rc, a.z, a.w, b.z, b.w);
+        mac(ih, ic, a.x, a.y, b.z, b.w);
+        mac(ih, ic, -a.z, -a.w, b.x, b.y);
+      }
+    }
+    long long* o = sums + (tid / kT) * 4 * kT + row;
+    o[0] = rh;
+    o[kT] = rc;
+    o[2 * kT] = ih;
+    o[3 * kT] = ic;
+    __syncthreads();
+    const int out = (second ? C : R) * kT + row;
+    if (tid < kT && out < n) {
+      const int e_all = Aex[t] + (second ? exR : exC) - 2 * kQ;
+      const double s56 = pow2(e_all + 56), s28 = pow2(e_all + 28);
+      long long s[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) s[c] = (sums[c * kT + row] + sums[(4 + c) * kT + row]) +
+                                         (sums[(8 + c) * kT + row] + sums[(12 + c) * kT + row]);
+      const int slot = second ? (R == C ? nT : R) : C;
+      P[(size_t)slot * n + out] = mk<double>(from_sums(s[0], s[1], s56, s28), from_sums(s[2], s[3], s56, s28));
+    }
+    __syncthreads();
+  }
+}
+
+// K3: x_w = tau (A v - sum_l v_l (w_l^H v) + w_l (v_l^H v)) with A v = sc (P + diag x) + om A(:, j+1), v into column
+// j, and the dots conj(x_w) v by CTA.
+__global__ void __launch_bounds__(256) tri_x_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
+                                                    const zd* __restrict__ W, const zd* __restrict__ P,
+                                                    const TriCol* __restrict__ col, const zd* __restrict__ g,
+                                                    zd* __restrict__ xw, zd* __restrict__ dots) {
+  __shared__ zd gv[kNB], gw[kNB], red[8];
+  const int tid = threadIdx.x, lane = tid & 15, j0 = j - i;
+  const zd tau = col->tau, sc = col->sc, om = col->om;
+  if (tid < 2 * i) {
+    const int l = tid >> 1;
+    const zd at = (tid & 1) ? W[(size_t)l * n + j + 1] : A[(size_t)(j0 + l) * lda + j + 1];
+    zd t = cmul(sc, g[tid]);
+    cfma(t, om, cconj(at));
+    ((tid & 1) ? gw : gv)[l] = t;  // v_l^H v, w_l^H v
+  }
+  __syncthreads();
+  const int r = j + 1 + blockIdx.x * kRows + tid / 16;
+  const int nT = (n + kT - 1) / kT, C0 = (j + 1) / kT;
+  zd acc = mk<double>(0.0, 0.0);
+  if (r < n) {
+    zd y = mk<double>(0.0, 0.0);
+    for (int t = C0 + lane; t <= nT; t += 16) y = cadd(y, P[(size_t)t * n + r]);
+    acc = cmul(sc, y);
+    for (int l = lane; l < i; l += 16) {
+      const zd v = A[(size_t)(j0 + l) * lda + r], w = W[(size_t)l * n + r];
+      cfma(acc, mk<double>(-v.re, -v.im), gw[l]);
+      cfma(acc, mk<double>(-w.re, -w.im), gv[l]);
+    }
+  }
+  acc = half_warp_sum(acc);
+  zd d = mk<double>(0.0, 0.0);
+  if (lane == 0 && r < n) {
+    const zd x = A[(size_t)j * lda + r];
+    const double dg = A[(size_t)r * lda + r].re;
+    zd a1 = A[(size_t)(j + 1) * lda + r];
+    if (r == j + 1) a1.im = 0.0;
+    const zd v = r == j + 1 ? mk<double>(1.0, 0.0) : cmul(sc, x);
+    cfma(acc, sc, cscale(x, dg));
+    cfma(acc, om, a1);
+    const zd xr = cmul(tau, acc);
+    xw[r] = xr;
+    A[(size_t)j * lda + r] = v;
+    d = cmulc(xr, v);
+  }
+  d.re += __shfl_xor_sync(0xffffffffu, d.re, 16);
+  d.im += __shfl_xor_sync(0xffffffffu, d.im, 16);
+  if ((tid & 31) == 0) red[tid >> 5] = d;
+  __syncthreads();
+  if (tid == 0) {
+    zd t = red[0];
+    for (int w = 1; w < 8; ++w) t = cadd(t, red[w]);
+    dots[blockIdx.x] = t;
+  }
+}
+
+// After a panel of kb reflectors (columns j1 - kb .. j1 - 1): A(r, c) -= sum_l v_l(r) conj(w_l(c)) + w_l(r) conj(v_l(c))
+// for r >= c >= j1, one CTA per 64 x 64 tile, the products quantised, then the tile's own quantised form (strict lower
+// triangle) for the next panel's Hermitian products.  kb = 0: only that.  512 threads, 4 x 2 entries each.  Bound by
+// the integer multiply-adds (768 an entry): 404 us at m = 2,304, where 32 FP64 rank-2 updates took 1.6 ms; all panels of
+// n = 2,304 13 ms against 55.
+__global__ void __launch_bounds__(512, 1) tri_update_kernel(zd* __restrict__ A, int n, int lda, int j1, int kb,
+                                                            const zd* __restrict__ tau, const zd* __restrict__ W,
+                                                            const zd* __restrict__ xw, const zd* __restrict__ dots,
+                                                            int ndots, int4* __restrict__ Aq, int* __restrict__ Aex) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  int4* vR = reinterpret_cast<int4*>(smem_raw);  // [kNB][kT] each
+  int4* wR = vR + kNB * kT;
+  int4* vC = wR + kNB * kT;
+  int4* wC = vC + kNB * kT;
   __shared__ zd s_alpha;
-  __shared__ zd vR[kSymTile], wR[kSymTile], vC[kSymTile], wC[kSymTile];
-  const zd tau = tau_p[j];
-  if (tau.re == 0.0 && tau.im == 0.0) return;
-  const int m = n - j - 1;
+  __shared__ int s_exv, s_exw, s_ext;
+  const int tid = threadIdx.x, C0 = j1 / kT;
   int R, C;
   lower_tile(blockIdx.x, &R, &C);
-  const int r0 = R * kSymTile, c0 = C * kSymTile;
-  if (threadIdx.x < 32) {
-    const zd al = her2_alpha(dots, ndots, tau);
-    if (threadIdx.x == 0) s_alpha = al;
+  R += C0;
+  C += C0;
+  if (tid == 0) s_exv = s_exw = s_ext = 0;
+  if (kb > 0 && tid < 32) {
+    const zd al = her2_alpha(dots, ndots, tau[j1 - 1]);
+    if (tid == 0) s_alpha = al;
   }
   __syncthreads();
-  const zd alpha = s_alpha;
-  if (threadIdx.x < kSymTile) {
-    const int t = threadIdx.x, r = r0 + t, c = c0 + t;
-    const zd z = mk<double>(0.0, 0.0);
-    const zd vr = r < m ? v[r] : z, vc = c < m ? v[c] : z;
-    vR[t] = vr;
-    vC[t] = vc;
-    wR[t] = r < m ? cadd(x[r], cmul(alpha, vr)) : z;
-    wC[t] = c < m ? cadd(x[c], cmul(alpha, vc)) : z;
+  const int tr = tid % 16, tc = tid / 16;
+  long long rh[8], rc[8], ih[8], ic[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) rh[e] = rc[e] = ih[e] = ic[e] = 0;
+  double scale = 0.0;
+  if (kb > 0) {
+    const zd alpha = s_alpha;
+    auto w_at = [&](int l, int r) {  // the last column's w is still x - (tau/2)(x^H v) v
+      if (r < j1 || r >= n) return mk<double>(0.0, 0.0);
+      if (l < kb - 1) return W[(size_t)l * n + r];
+      return cadd(xw[r], cmul(alpha, A[(size_t)(j1 - 1) * lda + r]));
+    };
+    auto v_at = [&](int l, int r) {
+      return r >= j1 && r < n ? A[(size_t)(j1 - kb + l) * lda + r] : mk<double>(0.0, 0.0);
+    };
+    int fv = 0, fw = 0;
+    for (int e = tid; e < 2 * kb * kT; e += 512) {
+      const int l = e / (2 * kT), rr = e % (2 * kT), r = (rr < kT ? R : C) * kT + rr % kT;
+      const zd v = v_at(l, r), w = w_at(l, r);
+      fv = max(fv, max(exponent_of(v.re), exponent_of(v.im)));
+      fw = max(fw, max(exponent_of(w.re), exponent_of(w.im)));
+    }
+    fv = __reduce_max_sync(0xffffffffu, fv);
+    fw = __reduce_max_sync(0xffffffffu, fw);
+    if ((tid & 31) == 0) {
+      atomicMax(&s_exv, fv);
+      atomicMax(&s_exw, fw);
+    }
+    __syncthreads();
+    const int exv = group_ex(s_exv), exw = group_ex(s_exw);
+    for (int e = tid; e < 2 * kb * kT; e += 512) {
+      const int l = e / (2 * kT), rr = e % (2 * kT), r = (rr < kT ? R : C) * kT + rr % kT;
+      (rr < kT ? wR : wC)[l * kT + rr % kT] = quantise(w_at(l, r), exw);
+      (rr < kT ? vR : vC)[l * kT + rr % kT] = quantise(v_at(l, r), exv);
+    }
+    __syncthreads();
+    for (int l = 0; l < kb; ++l) {
+      int4 v2[2], w2[2];
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        v2[c] = vC[l * kT + tc + 32 * c];
+        w2[c] = wC[l * kT + tc + 32 * c];
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int4 v = vR[l * kT + tr + 16 * q], w = wR[l * kT + tr + 16 * q];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int e = q * 2 + c;
+          mac(rh[e], rc[e], v.x, v.y, w2[c].x, w2[c].y);
+          mac(rh[e], rc[e], v.z, v.w, w2[c].z, w2[c].w);
+          mac(rh[e], rc[e], w.x, w.y, v2[c].x, v2[c].y);
+          mac(rh[e], rc[e], w.z, w.w, v2[c].z, v2[c].w);
+          mac(ih[e], ic[e], v.z, v.w, w2[c].x, w2[c].y);
+          mac(ih[e], ic[e], -v.x, -v.y, w2[c].z, w2[c].w);
+          mac(ih[e], ic[e], w.z, w.w, v2[c].x, v2[c].y);
+          mac(ih[e], ic[e], -w.x, -w.y, v2[c].z, v2[c].w);
+        }
+      }
+    }
+    scale = pow2(exw + exv - 2 * kQ + 56);
   }
+  // the new entries, and the tile's largest exponent off the diagonal
+  zd a[8];
+  int f = 0;
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int r = R * kT + tr + 16 * (e >> 1), c = C * kT + tc + 32 * (e & 1);
+    a[e] = mk<double>(0.0, 0.0);
+    if (r < n && c >= j1 && r >= c) {
+      zd* p = A + (size_t)c * lda + r;
+      a[e] = *p;
+      if (kb > 0) {  // the low sums carried into the high ones, rounded at 2^-54 of the largest product
+        const long long hr = rh[e] + ((rc[e] + (1ll << 27)) >> 28), hi = ih[e] + ((ic[e] + (1ll << 27)) >> 28);
+        a[e].re = fma(-(double)hr, scale, a[e].re);
+        a[e].im = r == c ? 0.0 : fma(-(double)hi, scale, a[e].im);
+        *p = a[e];
+      }
+      if (r == c)
+        a[e] = mk<double>(0.0, 0.0);
+      else
+        f = max(f, max(exponent_of(a[e].re), exponent_of(a[e].im)));
+    }
+  }
+  f = __reduce_max_sync(0xffffffffu, f);
+  if ((tid & 31) == 0) atomicMax(&s_ext, f);
   __syncthreads();
-  const int i = threadIdx.x % kSymTile, g = threadIdx.x / kSymTile;
-  const int r = r0 + i;
-  if (r >= m) return;
-  zd* a22 = A + (size_t)(j + 1) * lda + j + 1;
-  const zd vr = vR[i], wr = wR[i];
-  const int q0 = g * (kSymTile / 4);
-  const int q1 = min(q0 + kSymTile / 4, R == C ? i + 1 : kSymTile);
-  for (int jj = q0; jj < q1; ++jj) {
-    const int c = c0 + jj;
-    if (c >= m) break;
-    const zd vc = vC[jj], wc = wC[jj];
-    zd a = a22[(size_t)c * lda + r];
-    // a -= vr conj(wc) + wr conj(vc)
-    a.re = fma(-vr.re, wc.re, a.re);
-    a.re = fma(-vr.im, wc.im, a.re);
-    a.re = fma(-wr.re, vc.re, a.re);
-    a.re = fma(-wr.im, vc.im, a.re);
-    a.im = fma(-vr.im, wc.re, a.im);
-    a.im = fma(vr.re, wc.im, a.im);
-    a.im = fma(-wr.im, vc.re, a.im);
-    a.im = fma(wr.re, vc.im, a.im);
-    a22[(size_t)c * lda + r] = a;
-  }
+  const int ex = group_ex(s_ext);
+  const size_t t = (size_t)R * (R + 1) / 2 + C;
+  if (tid == 0) Aex[t] = ex;
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    Aq[t * kT * kT + (tc + 32 * (e & 1)) * kT + tr + 16 * (e >> 1)] = quantise(a[e], ex);
 }
 
 // A(j,i) = conj(A(i,j)) for i < j (the upper triangle is the input, as ZHEEV 'U' reads it); real diagonal.
@@ -290,64 +509,87 @@ __global__ void mirror_upper_kernel(zd* __restrict__ A, int n, int lda) {
   else if (i == j) A[(size_t)j * lda + i].im = 0.0;
 }
 
-// d(i) = Re A(i,i); Gershgorin bounds and pivmin of T (one CTA).
+// d(i) = Re A(i,i); Gershgorin bounds and scale of T (one CTA).
 __global__ void __launch_bounds__(1024) tri_finish_kernel(const zd* __restrict__ A, int n, int lda,
                                                           double* __restrict__ d, const double* __restrict__ e,
                                                           double* __restrict__ bounds) {
-  double lo = INFINITY, hi = -INFINITY, emax2 = 0.0;
+  double lo = INFINITY, hi = -INFINITY;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double di = A[(size_t)i * lda + i].re;
     d[i] = di;
     const double el = i > 0 ? fabs(e[i - 1]) : 0.0, er = i < n - 1 ? fabs(e[i]) : 0.0;
     lo = fmin(lo, di - el - er);
     hi = fmax(hi, di + el + er);
-    if (i < n - 1) emax2 = fmax(emax2, e[i] * e[i]);
   }
   for (int o = 16; o > 0; o >>= 1) {
     lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    emax2 = fmax(emax2, __shfl_xor_sync(0xffffffffu, emax2, o));
   }
-  __shared__ double s_lo[32], s_hi[32], s_e[32];
+  __shared__ double s_lo[32], s_hi[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0) {
     s_lo[warp] = lo;
     s_hi[warp] = hi;
-    s_e[warp] = emax2;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
     for (int i = 1; i < (int)(blockDim.x >> 5); ++i) {
       lo = fmin(lo, s_lo[i]);
       hi = fmax(hi, s_hi[i]);
-      emax2 = fmax(emax2, s_e[i]);
     }
     const double tnorm = fmax(fabs(lo), fabs(hi));
     // widen by a few ulps of the norm so that the end eigenvalues are strictly inside
     const double pad = 2.0 * (double)n * DBL_EPSILON * fmax(tnorm, 1e-300) + DBL_MIN;
     bounds[0] = lo - pad;
     bounds[1] = hi + pad;
-    bounds[2] = DBL_MIN * fmax(1.0, emax2);  // pivmin (dstebz)
+    const int k = min(max(ilogb(fmax(fabs(bounds[0]), fabs(bounds[1]))) + 1, -1000), 1000);
+    bounds[2] = scalbn(1.0, -k);  // T times this has entries and eigenvalues of at most 1
   }
 }
 
-// number of eigenvalues of T below x (Sturm sequence with the pivot guard)
+// Number of eigenvalues of the scaled T below x: the sign changes of p_0 = 1, p_{i+1} = (d_i - x) p_i - e_{i-1}^2 p_{i-1}
+// (the leading minors; Givens' recurrence, each p_i the exact one of a T whose entries differ by a few ulp).  One
+// multiply-add of latency and three FP64 instructions a row, against a division's chain of 460 clocks and eleven
+// instructions for the ratios q_i = p_{i+1} / p_i (all eigenvalues at n = 2,304: 20 -> 6.9 ms).  T is scaled to entries of at most 1, so that the pair (p_i, p_{i-1})
+// can lose at most 53 bits a row and gain two: every eighth row rescales it by a power of two.  A zero counts as
+// of the other sign than its predecessor (a zero pivot replaced by a small negative one).
 __device__ __forceinline__ int sturm_count(const double* __restrict__ d, const double* __restrict__ e2, int n,
-                                           double x, double pivmin) {
-  double q = d[0] - x;
-  if (fabs(q) < pivmin) q = -pivmin;
-  int cnt = q < 0.0;
-  for (int i = 1; i < n; ++i) {
-    q = (d[i] - x) - e2[i - 1] / q;
-    if (fabs(q) < pivmin) q = -pivmin;
-    cnt += q < 0.0;
+                                           double x) {
+  auto nonzero = [](double p, double before) {
+    return (__double_as_longlong(p) << 1) == 0
+               ? __hiloint2double((__double2hiint(before) & 0x80000000) ^ (int)0xb3700000, 0)  // -+ 2^-200
+               : p;
+  };
+  double p0 = 1.0, p1 = nonzero(d[0] - x, 1.0);
+  int cnt = (unsigned)__double2hiint(p1) >> 31;
+  for (int i0 = 1; i0 < n; i0 += 8) {
+    const int e = (max((__double2hiint(p0) >> 20) & 0x7ff, (__double2hiint(p1) >> 20) & 0x7ff));
+    const double sc = __hiloint2double((2046 - e) << 20, 0);  // 2^(1023 - e): the larger one to [1, 2)
+    p0 *= sc;
+    p1 *= sc;
+    const int i1 = min(i0 + 8, n);
+#pragma unroll 8
+    for (int i = i0; i < i1; ++i) {
+      const double p = nonzero(fma(d[i] - x, p1, -(e2[i - 1] * p0)), p1);
+      cnt += (unsigned)(__double2hiint(p) ^ __double2hiint(p1)) >> 31;
+      p0 = p1;
+      p1 = p;
+    }
   }
   return cnt;
 }
 
-__global__ void e2_kernel(const double* __restrict__ e, int n, double* __restrict__ e2) {
+// ds, e2: T scaled by the power of two that brings its Gershgorin interval to at most 1 in magnitude (bounds[2])
+__global__ void tri_scale_kernel(const double* __restrict__ d, const double* __restrict__ e, int n,
+                                 const double* __restrict__ bounds, double* __restrict__ ds, double* __restrict__ e2) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n - 1) e2[i] = e[i] * e[i];
+  if (i >= n) return;
+  const double s = bounds[2];
+  ds[i] = d[i] * s;
+  if (i < n - 1) {
+    const double es = e[i] * s;
+    e2[i] = es * es;
+  }
 }
 
 // The k-th smallest eigenvalue (k = 0..n-1) by multisection with L lanes per k (L a power of two <= 32): the L
@@ -364,16 +606,16 @@ __global__ void __launch_bounds__(128) tri_multisect_kernel(const double* __rest
   const int lane = threadIdx.x & 31;
   const int k = tid / L, g = lane % L, base = lane - g;
   const unsigned gmask = L == 32 ? 0xffffffffu : (((1u << L) - 1u) << base);
-  double lo = bounds[0], hi = bounds[1];
-  const double pivmin = bounds[2];
-  const double tol = 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi)) + pivmin;
+  const double sc = bounds[2];
+  double lo = bounds[0] * sc, hi = bounds[1] * sc;
+  const double tol = 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi));
   bool done = k >= n;
   for (int it = 0; it < 256; ++it) {
     if (!done && !(hi - lo > tol)) done = true;
     if (__all_sync(0xffffffffu, done)) break;
     const double h = (hi - lo) / (double)(L + 1);
     const double x = lo + h * (double)(g + 1);
-    const int cnt = done ? 0 : sturm_count(d, e2, n, x, pivmin);
+    const int cnt = done ? 0 : sturm_count(d, e2, n, x);
     const unsigned bal = __ballot_sync(0xffffffffu, !done && cnt <= k);
     const int nlo = __popc(bal & gmask);
     const double xlo = __shfl_sync(0xffffffffu, x, base + max(nlo - 1, 0));
@@ -389,7 +631,7 @@ __global__ void __launch_bounds__(128) tri_multisect_kernel(const double* __rest
       }
     }
   }
-  if (k < n && g == 0) W[k] = 0.5 * (lo + hi);
+  if (k < n && g == 0) W[k] = 0.5 * (lo + hi) / sc;
 }
 
 // ----------------------------------------------------------------------------- eigenvectors
@@ -558,34 +800,88 @@ __global__ void __launch_bounds__(256) tri_backtransform_kernel(const zd* __rest
 
 }  // namespace
 
-size_t dense_eig_scratch(int n) {
-  // v, x, tau (n each), dots, P, all complex; e, d, e2 (n doubles); bounds
-  const size_t nd = (size_t)(n + kXRows - 1) / kXRows;
-  return sizeof(zd) * ((size_t)3 * n + nd + p_capacity(n)) + sizeof(double) * ((size_t)3 * n + 4);
-}
+// The reduction's buffers in one scratch block.
+struct TriScratch {
+  zd *xw, *tau, *dots, *g, *W, *P;
+  double *norms, *e, *d, *ds, *e2, *bounds;
+  TriCol* col;
+  int* Aex;
+  int4* Aq;
+  size_t bytes;
+  TriScratch(int n, void* base) {
+    const int nT = tiles_of(n);
+    const size_t nd = (size_t)(n + kRows - 1) / kRows, nt = lower_tiles(nT);
+    unsigned char* p = reinterpret_cast<unsigned char*>(base);
+    auto take = [&](size_t b) {
+      unsigned char* q = p;
+      p += (b + 15) & ~(size_t)15;
+      return q;
+    };
+    Aq = reinterpret_cast<int4*>(take(nt * kT * kT * sizeof(int4)));
+    P = reinterpret_cast<zd*>(take((size_t)(nT + 1) * n * sizeof(zd)));
+    W = reinterpret_cast<zd*>(take((size_t)kNB * n * sizeof(zd)));
+    xw = reinterpret_cast<zd*>(take(n * sizeof(zd)));
+    tau = reinterpret_cast<zd*>(take(n * sizeof(zd)));
+    dots = reinterpret_cast<zd*>(take(nd * sizeof(zd)));
+    g = reinterpret_cast<zd*>(take(2 * kNB * sizeof(zd)));
+    col = reinterpret_cast<TriCol*>(take(sizeof(TriCol)));
+    norms = reinterpret_cast<double*>(take(nd * sizeof(double)));
+    e = reinterpret_cast<double*>(take(n * sizeof(double)));
+    d = reinterpret_cast<double*>(take(n * sizeof(double)));
+    ds = reinterpret_cast<double*>(take(n * sizeof(double)));
+    e2 = reinterpret_cast<double*>(take(n * sizeof(double)));
+    bounds = reinterpret_cast<double*>(take(4 * sizeof(double)));
+    Aex = reinterpret_cast<int*>(take(nt * sizeof(int)));
+    bytes = (size_t)(p - reinterpret_cast<unsigned char*>(base));
+  }
+};
+
+size_t dense_eig_scratch(int n) { return TriScratch(n, nullptr).bytes; }
+
+constexpr size_t kSymvSmem = sizeof(int4) * (kT * (kT + 1) + 2 * kT) + sizeof(long long) * 16 * kT;
+constexpr size_t kUpdateSmem = sizeof(int4) * 4 * kNB * kT;
 
 cudaError_t dense_eig_prepare() {
-  cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(tri_symv_kernel<64>), sizeof(zd) * (64 * 65 + 640));
-  if (err == cudaSuccess)
-    err = raise_smem_limit(reinterpret_cast<const void*>(tri_symv_kernel<32>), sizeof(zd) * (32 * 33 + 320));
-  if (err == cudaSuccess)
-    err = raise_smem_limit(reinterpret_cast<const void*>(tri_symv_kernel<16>), sizeof(zd) * (16 * 17 + 160));
+  cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(tri_symv_kernel), kSymvSmem);
+  if (err == cudaSuccess) err = raise_smem_limit(reinterpret_cast<const void*>(tri_update_kernel), kUpdateSmem);
   return err;
 }
 
-template <int T>
-static cudaError_t tri_step(zd* A, int n, int lda, int j, zd* v, zd* tau, zd* P, zd* x, zd* dots, cudaStream_t s) {
-  const int m = n - j - 1;
-  const int nT = (m + T - 1) / T;
-  const unsigned ntiles = (unsigned)((long)nT * (nT + 1) / 2);
-  const int nd = (m + kXRows - 1) / kXRows;
-  const size_t smem = sizeof(zd) * ((size_t)T * (T + 1) + 10 * T);
-  cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(tri_symv_kernel<T>), smem);
+// The reduction: per column the three kernels, per panel the trailing update.
+static cudaError_t tridiagonalise(zd* A, int n, int lda, const TriScratch& t, cudaStream_t s) {
+  cudaError_t err = dense_eig_prepare();
   if (err != cudaSuccess) return err;
-  tri_symv_kernel<T><<<ntiles, 4 * T, smem, s>>>(A, n, lda, j, v, tau, P); ++g_launch_count;
-  tri_x_kernel<<<nd, 8 * kXRows, 0, s>>>(P, nT, m, tau, j, v, x, dots); ++g_launch_count;
-  tri_her2l_kernel<T><<<ntiles, 4 * T, 0, s>>>(A, n, lda, j, tau, v, x, dots, nd); ++g_launch_count;
-  return cudaSuccess;
+  const int nT = tiles_of(n);
+  int ndots = 0;
+  auto update = [&](int j1, int kb) {
+    const unsigned tiles = (unsigned)lower_tiles(nT - j1 / kT);
+    tri_update_kernel<<<tiles, 512, kUpdateSmem, s>>>(A, n, lda, j1, kb, t.tau, t.W, t.xw, t.dots, ndots, t.Aq, t.Aex);
+    ++g_launch_count;
+  };
+  auto column = [&](int j, int i) {
+    const int nc = (n - j + kRows - 1) / kRows;
+    tri_col_kernel<<<nc, 256, 0, s>>>(A, n, lda, j, i, t.tau, t.W, t.xw, t.dots, ndots, t.norms);
+    ++g_launch_count;
+    return nc;
+  };
+  update(0, 0);
+  int i = 0;
+  for (int j = 0; j + 1 < n; ++j) {
+    const int nn = column(j, i);
+    const unsigned tiles = (unsigned)lower_tiles(nT - (j + 1) / kT);
+    tri_symv_kernel<<<tiles + 1 + i, 256, kSymvSmem, s>>>(A, n, lda, j, i, t.W, t.norms, nn, t.Aq, t.Aex,
+                                                          t.col, t.tau, t.e, t.g, t.P);
+    ++g_launch_count;
+    ndots = (n - j - 1 + kRows - 1) / kRows;
+    tri_x_kernel<<<ndots, 256, 0, s>>>(A, n, lda, j, i, t.W, t.P, t.col, t.g, t.xw, t.dots);
+    ++g_launch_count;
+    if (++i == kNB) {
+      update(j + 1, kNB);
+      i = 0;
+    }
+  }
+  column(n - 1, i);  // the last diagonal entry
+  return cudaGetLastError();
 }
 
 static int invit_batch(int n) {
@@ -606,35 +902,19 @@ cudaError_t launch_dense_eig(zd* A, int n, int lda, bool upper_only, double* W, 
                              void* scratch, void* vscratch, cudaStream_t s) {
   if (Z && !vscratch) return cudaErrorInvalidValue;
   if (n < 1 || lda < n) return cudaErrorInvalidValue;
-  const size_t ndmax = (size_t)(n + kXRows - 1) / kXRows;
-  zd* v = reinterpret_cast<zd*>(scratch);
-  zd* x = v + n;
-  zd* tau = x + n;
-  zd* dots = tau + n;
-  zd* P = dots + ndmax;
-  double* e = reinterpret_cast<double*>(P + p_capacity(n));
-  double* d = e + n;
-  double* e2 = d + n;
-  double* bounds = e2 + n;
+  const TriScratch t(n, scratch);
+  zd* tau = t.tau;
+  double *e = t.e, *d = t.d, *ds = t.ds, *e2 = t.e2, *bounds = t.bounds;
   if (upper_only) {
     mirror_upper_kernel<<<(unsigned)(((long)n * n + 255) / 256), 256, 0, s>>>(A, n, lda); ++g_launch_count;
   }
-  for (int j = 0; j + 1 < n; ++j) {
-    const int m = n - j - 1;
-    tri_reflector_kernel<<<1, 256, 0, s>>>(A, n, lda, j, v, tau, e); ++g_launch_count;
-    const int T = pick_tile(m);
-    const cudaError_t err = T == 64 ? tri_step<64>(A, n, lda, j, v, tau, P, x, dots, s)
-                            : T == 32 ? tri_step<32>(A, n, lda, j, v, tau, P, x, dots, s)
-                                      : tri_step<16>(A, n, lda, j, v, tau, P, x, dots, s);
-    if (err != cudaSuccess) return err;
-  }
+  const cudaError_t err = tridiagonalise(A, n, lda, t, s);
+  if (err != cudaSuccess) return err;
   tri_finish_kernel<<<1, 1024, 0, s>>>(A, n, lda, d, e, bounds); ++g_launch_count;
-  if (n > 1) {
-    e2_kernel<<<(n + 255) / 256, 256, 0, s>>>(e, n, e2); ++g_launch_count;
-  }
+  tri_scale_kernel<<<(n + 255) / 256, 256, 0, s>>>(d, e, n, bounds, ds, e2); ++g_launch_count;
   int L = 1;  // about two warps per SM
   while (L < 32 && (long)n * L < 152L * 64) L *= 2;
-  tri_multisect_kernel<<<(unsigned)(((long)n * L + 127) / 128), 128, 0, s>>>(d, e2, n, bounds, W, L); ++g_launch_count;
+  tri_multisect_kernel<<<(unsigned)(((long)n * L + 127) / 128), 128, 0, s>>>(ds, e2, n, bounds, W, L); ++g_launch_count;
   if (Z) {
     double* Zt = reinterpret_cast<double*>(vscratch);
     double* work = Zt + (size_t)n * n;
