@@ -1398,6 +1398,7 @@ int wtb_bsesolvertemp(wtb_ctx* c, const wtb_bse_params* p, const wtb_temp_params
   zd* Z = c->ws.get<zd>("T_Z", (size_t)dim * dim, &err);
   double* W = c->ws.get<double>("deig_W", dim, &err);
   double* dacts = c->ws.get<double>("T_acts", (size_t)8 * dim, &err);
+  double* part = c->ws.get<double>("T_part", temp_acts_scratch((int)dim), &err);
   void* scratch = c->ws.get<zd>("deig_scratch", (dense_eig_scratch((int)dim) + sizeof(zd) - 1) / sizeof(zd), &err);
   void* vscratch = c->ws.get<double>("deig_vscratch", dense_eigvec_scratch((int)dim) / sizeof(double), &err);
   CKC(err);
@@ -1410,7 +1411,8 @@ int wtb_bsesolvertemp(wtb_ctx* c, const wtb_bse_params* p, const wtb_temp_params
   CKC(dense_eig_prepare());
   // H is row-major, i.e. conj(H) column-major: its eigenvectors are conjugated back
   CKC(launch_dense_eig(H, (int)dim, (int)dim, false, W, Z, true, scratch, vscratch, c->s));
-  CKC(launch_temp_acts(Z, (int)dim, c->ws.get<zd>("hrvel", 0, &err), f, tp->dtfull, tp->cpol, dacts, c->s));
+  CKC(launch_temp_acts(Z, (int)dim, c->ws.get<zd>("hrvel", 0, &err), f, tp->dtfull, tp->cpol, part,
+                       dacts, c->s));
   if (Ws) CKC(cudaMemcpyAsync(Ws, W, sizeof(double) * dim, cudaMemcpyDeviceToHost, c->s));
   if (acts) CKC(cudaMemcpyAsync(acts, dacts, sizeof(double) * 8 * dim, cudaMemcpyDeviceToHost, c->s));
   if (fdeh) CKC(cudaMemcpyAsync(fdeh, f, sizeof(double) * dim, cudaMemcpyDeviceToHost, c->s));

@@ -417,8 +417,9 @@ cudaError_t launch_fermi_weights(const double* eig_win, int nk, int nv, int nc, 
 // triangle of matrizelbsetemp / matrizelbsekqtemp; dE the transition energies of H's diagonal.
 cudaError_t launch_temp_weight(zd* H, long dim, const double* f, const double* dE, cudaStream_t s);
 // dielbseptemp's eight activities acts(dim, 8) of the eigenvectors Z (row-major) and hr[5][dim].
-cudaError_t launch_temp_acts(const zd* Z, int dim, const zd* hr, const double* f, int dtfull, int cpol, double* acts,
-                             cudaStream_t s);
+size_t temp_acts_scratch(int dim);  // doubles of part
+cudaError_t launch_temp_acts(const zd* Z, int dim, const zd* hr, const double* f, int dtfull, int cpol, double* part,
+                             double* acts, cudaStream_t s);
 
 // ----------------------------------------------------------------------------- dense Hermitian eigenvalues
 // All eigenvalues (ascending) of the n x n Hermitian A (column-major, leading dimension lda; destroyed: its
