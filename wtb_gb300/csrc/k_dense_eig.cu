@@ -642,6 +642,9 @@ __global__ void __launch_bounds__(128) tri_multisect_kernel(const double* __rest
 // then spans its eigenspace).  Outside clusters the vectors are orthogonal to eps ||T|| / gap <= 2e-9.
 // One thread per cluster start; its scratch (6 arrays of n) is interleaved across the batch's threads so the
 // row loops are coalesced.  Zt(i, k) = Zt[i * n + k] (row-major real).
+// A thread's rows are one chain, so its latency is the time: the elimination carries its row in registers, the solves
+// load eight rows of their operands before they use the first, one division a row (the pivot's reciprocal), and a CTA
+// is one warp, so that the warps spread over the SMs.  n = 1,520: 11.2 -> 3.7 ms.
 constexpr int kInvIters = 3;
 
 // deterministic start entries in [-1, 1): splitmix64 of (k, i)
@@ -653,10 +656,11 @@ __device__ __forceinline__ double start_entry(unsigned long long k, unsigned lon
   return (double)(z >> 11) * (2.0 / 9007199254740992.0) - 1.0;
 }
 
-__global__ void __launch_bounds__(128) tri_invit_kernel(const double* __restrict__ d, const double* __restrict__ e,
-                                                        int n, const double* __restrict__ W,
-                                                        const double* __restrict__ bounds, int k0, int nb,
-                                                        double* __restrict__ work, double* __restrict__ Zt) {
+__global__ void __launch_bounds__(32) tri_invit_kernel(const double* __restrict__ d, const double* __restrict__ e,
+                                                       int n, const double* __restrict__ W,
+                                                       const double* __restrict__ bounds, int k0, int nb,
+                                                       double* __restrict__ work, double* __restrict__ Zt) {
+  constexpr int U = 8;  // rows whose operands are loaded together
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int k = k0 + t;
   if (t >= nb || k >= n) return;
@@ -666,12 +670,12 @@ __global__ void __launch_bounds__(128) tri_invit_kernel(const double* __restrict
   int kend = k + 1;
   while (kend < n && W[kend] - W[kend - 1] < ortol) ++kend;
   const size_t st = (size_t)nb;
-  double* a = work + t;             // diagonal of U
-  double* b = a + (size_t)n * st;   // first superdiagonal of U
-  double* dd = b + (size_t)n * st;  // second superdiagonal of U
-  double* c = dd + (size_t)n * st;  // multipliers
-  double* pv = c + (size_t)n * st;  // 1 where rows i, i+1 were swapped
-  double* y = pv + (size_t)n * st;  // iterate
+  double* ra = work + t;             // reciprocal of the diagonal of U
+  double* b = ra + (size_t)n * st;   // first superdiagonal of U
+  double* dd = b + (size_t)n * st;   // second superdiagonal of U
+  double* c = dd + (size_t)n * st;   // multipliers
+  double* pv = c + (size_t)n * st;   // 1 where rows i, i+1 were swapped
+  double* y = pv + (size_t)n * st;   // iterate
 #define AT(arr, i) arr[(size_t)(i) * st]
   const double tiny = DBL_EPSILON * tnorm;
   double lam_prev = 0.0;
@@ -679,123 +683,268 @@ __global__ void __launch_bounds__(128) tri_invit_kernel(const double* __restrict
     double lam = W[q];
     if (q > k && lam - lam_prev < 10.0 * DBL_EPSILON * tnorm) lam = lam_prev + 10.0 * DBL_EPSILON * tnorm;
     lam_prev = lam;
-    // T - lam I = P L U
+    // T - lam I = P L U, row i in (ai, bi)
+    double ai = d[0] - lam, bi = n > 1 ? e[0] : 0.0;
     for (int i = 0; i < n; ++i) {
-      AT(a, i) = d[i] - lam;
-      AT(b, i) = i < n - 1 ? e[i] : 0.0;
+      const bool more = i + 1 < n;
+      const double sub = more ? e[i] : 0.0;
+      const double a1 = more ? d[i + 1] - lam : 0.0, b1 = i + 2 < n ? e[i + 1] : 0.0;
+      const bool keep = fabs(ai) >= fabs(sub);
+      double piv = keep ? ai : sub;
+      if (fabs(piv) < tiny) piv = piv < 0.0 ? -tiny : tiny;
+      const double rp = 1.0 / piv, m = (keep ? sub : ai) * rp;
+      AT(ra, i) = rp;
+      AT(c, i) = m;
+      AT(pv, i) = keep ? 0.0 : 1.0;
+      AT(b, i) = keep ? bi : a1;
+      AT(dd, i) = keep ? 0.0 : b1;
+      AT(y, i) = start_entry((unsigned long long)q, (unsigned long long)i);
+      const double an = keep ? a1 - m * bi : bi - m * a1;
+      bi = keep ? b1 : -m * b1;
+      ai = an;
     }
-    for (int i = 0; i + 1 < n; ++i) {
-      const double sub = e[i], ai = AT(a, i);
-      if (fabs(ai) >= fabs(sub)) {
-        const double m = ai == 0.0 ? 0.0 : sub / ai;
-        AT(c, i) = m;
-        AT(pv, i) = 0.0;
-        AT(dd, i) = 0.0;
-        AT(a, i + 1) = AT(a, i + 1) - m * AT(b, i);
-      } else {
-        const double m = ai / sub;
-        const double a1 = AT(a, i + 1), bi = AT(b, i), b1 = i + 2 < n ? AT(b, i + 1) : 0.0;
-        AT(a, i) = sub;
-        AT(b, i) = a1;
-        AT(dd, i) = b1;
-        AT(a, i + 1) = bi - m * a1;
-        if (i + 2 < n) AT(b, i + 1) = -m * b1;
-        AT(c, i) = m;
-        AT(pv, i) = 1.0;
-      }
-    }
-    for (int i = 0; i < n; ++i)
-      if (fabs(AT(a, i)) < tiny) AT(a, i) = AT(a, i) < 0.0 ? -tiny : tiny;
-    for (int i = 0; i < n; ++i) AT(y, i) = start_entry((unsigned long long)q, (unsigned long long)i);
     for (int it = 0; it < kInvIters; ++it) {
-      for (int i = 0; i + 1 < n; ++i) {
-        if (AT(pv, i) != 0.0) {
-          const double tmp = AT(y, i);
-          AT(y, i) = AT(y, i + 1);
-          AT(y, i + 1) = tmp;
+      double cur = AT(y, 0);
+      for (int i0 = 0; i0 + 1 < n; i0 += U) {
+        double cc[U], pp[U], yy[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int i = min(i0 + u, n - 2);
+          cc[u] = AT(c, i);
+          pp[u] = AT(pv, i);
+          yy[u] = AT(y, i + 1);
         }
-        AT(y, i + 1) = AT(y, i + 1) - AT(c, i) * AT(y, i);
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i0 + u + 1 < n) {
+            const double first = pp[u] != 0.0 ? yy[u] : cur, second = pp[u] != 0.0 ? cur : yy[u];
+            AT(y, i0 + u) = first;
+            cur = second - cc[u] * first;
+          }
       }
-      for (int i = n - 1; i >= 0; --i) {
-        double r = AT(y, i);
-        if (i + 1 < n) r -= AT(b, i) * AT(y, i + 1);
-        if (i + 2 < n) r -= AT(dd, i) * AT(y, i + 2);
-        AT(y, i) = r / AT(a, i);
+      AT(y, n - 1) = cur;
+      double y1 = 0.0, y2 = 0.0, mx = 0.0;  // rows i + 1 and i + 2
+      for (int i0 = n - 1; i0 >= 0; i0 -= U) {
+        double aa[U], bb[U], ee[U], yy[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int i = max(i0 - u, 0);
+          aa[u] = AT(ra, i);
+          bb[u] = AT(b, i);
+          ee[u] = AT(dd, i);
+          yy[u] = AT(y, i);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i0 - u >= 0) {
+            const double x = (yy[u] - bb[u] * y1 - ee[u] * y2) * aa[u];
+            AT(y, i0 - u) = x;
+            mx = fmax(mx, fabs(x));
+            y2 = y1;
+            y1 = x;
+          }
       }
-      // against the cluster's earlier members, then to unit length
-      for (int p = k; p < q; ++p) {
-        double dot = 0.0;
-        for (int i = 0; i < n; ++i) dot += AT(y, i) * Zt[(size_t)i * n + p];
-        for (int i = 0; i < n; ++i) AT(y, i) -= dot * Zt[(size_t)i * n + p];
+      if (q > k) {
+        // against the cluster's earlier members
+        for (int p = k; p < q; ++p) {
+          double dot = 0.0;
+          for (int i = 0; i < n; ++i) dot += AT(y, i) * Zt[(size_t)i * n + p];
+          for (int i = 0; i < n; ++i) AT(y, i) -= dot * Zt[(size_t)i * n + p];
+        }
+        mx = 0.0;
+        for (int i = 0; i < n; ++i) mx = fmax(mx, fabs(AT(y, i)));
       }
-      double mx = 0.0;
-      for (int i = 0; i < n; ++i) mx = fmax(mx, fabs(AT(y, i)));
+      // to unit length
       const double sc = mx > 0.0 ? 1.0 / mx : 1.0;
       double nrm2 = 0.0;
+#pragma unroll 8
       for (int i = 0; i < n; ++i) {
         const double v = AT(y, i) * sc;
-        AT(y, i) = v;
-        nrm2 += v * v;
+        nrm2 = fma(v, v, nrm2);
       }
-      const double inv = 1.0 / sqrt(nrm2);
-      for (int i = 0; i < n; ++i) AT(y, i) *= inv;
+      const double f = sc / sqrt(nrm2);
+      double* out = it + 1 < kInvIters ? y : Zt + q;
+      const size_t so = it + 1 < kInvIters ? st : (size_t)n;
+      for (int i0 = 0; i0 < n; i0 += U) {
+        double yy[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) yy[u] = AT(y, min(i0 + u, n - 1));
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (i0 + u < n) out[(size_t)(i0 + u) * so] = yy[u] * f;
+      }
     }
-    for (int i = 0; i < n; ++i) Zt[(size_t)i * n + q] = AT(y, i);
   }
 #undef AT
 }
 
-constexpr int kBtCols = 8;  // eigenvector columns per CTA of the back-transformation
+// The reflectors quantised in place for the back-transformation: v_j(1:) (rows j + 2 ..) of column j as int4 with the
+// exponent exv[j]; v_j(0) = 1 is implied.  One CTA per column.
+__global__ void __launch_bounds__(256) tri_quantise_kernel(zd* __restrict__ A, int n, int lda, int* __restrict__ exv) {
+  __shared__ int s_f;
+  const int j = blockIdx.x, tid = threadIdx.x;
+  zd* v = A + (size_t)j * lda;
+  if (tid == 0) s_f = 0;
+  __syncthreads();
+  int f = 0;
+  for (int r = j + 2 + tid; r < n; r += 256) f = max(f, max(exponent_of(v[r].re), exponent_of(v[r].im)));
+  f = __reduce_max_sync(0xffffffffu, f);
+  if ((tid & 31) == 0) atomicMax(&s_f, f);
+  __syncthreads();
+  const int ex = group_ex(s_f);
+  if (tid == 0) exv[j] = ex;
+  int4* q = reinterpret_cast<int4*>(v);
+  for (int r = j + 2 + tid; r < n; r += 256) q[r] = quantise(v[r], ex);
+}
 
-// Z = Q Zt with Q = H_0 H_1 ... H_{n-2}, H_j = I - tau_j v_j v_j^H (v_j in A(j+1:n, j), v_j(0) = 1): the
-// reflectors applied from j = n-2 down to 0 to every column.  A CTA owns 8 columns and 32 row slices (row i in
-// slice i % 32) for the whole sweep, so the columns need no synchronisation between CTAs; per reflector a
-// two-barrier reduction of v^H z.  Z(i, k) = Z[i * n + k] (row-major), conjugated at the end when the solver
-// worked on conj(H).
-__global__ void __launch_bounds__(256) tri_backtransform_kernel(const zd* __restrict__ A, int n, int lda,
-                                                                const zd* __restrict__ tau,
-                                                                const double* __restrict__ Zt, zd* __restrict__ Z,
-                                                                int conj_out) {
-  __shared__ zd red[8][kBtCols];
-  __shared__ zd dots[kBtCols];
-  const int c = threadIdx.x % kBtCols, sl = threadIdx.x / kBtCols;
-  const int k = blockIdx.x * kBtCols + c;
-  const bool kv = k < n;
-  for (int i = sl; i < n; i += 32)
-    if (kv) Z[(size_t)i * n + k] = mk<double>(Zt[(size_t)i * n + k], 0.0);
+// Z = Q Zt with Q = H_0 H_1 ... H_{n-2}, H_j = I - tau_j v_j v_j^H: the reflectors applied from j = n-2 down to 0 to
+// every column.  A CTA owns kc columns for the whole sweep, so the columns need no synchronisation between CTAs.  The
+// columns are held in fixed point, 64-bit integers in units of 2^-60 (they have unit length throughout), in shared
+// memory where they fit, else in Z itself; a thread owns the same rows of its column for every reflector.  v^H z and
+// v f run as exact integer sums (kQ above; the two 32-bit halves of z are its limbs, the lower one shortened to 28
+// bits; f quantised with an exponent of its own), f = tau v^H z itself in FP64.  Rounding: 2^-61 an update and entry, where FP64 has 2^-53 of the entry; v^H z
+// to 2^-56 of its terms.  Bound by the integer multiply-adds (24 an entry and reflector; the FP64 form 8 on a pipe
+// a twelfth as fast).  n = 1,520: 38.9 -> 16.1 ms.
+// Z(i, k) = Z[i * n + k] (row-major), conjugated at the end when the solver worked on conj(H).
+constexpr int kBtThreads = 256;
+__global__ void __launch_bounds__(kBtThreads) tri_backtransform_kernel(const zd* __restrict__ A, int n, int lda,
+                                                                       const zd* __restrict__ tau,
+                                                                       const int* __restrict__ exv,
+                                                                       const double* __restrict__ Zt,
+                                                                       zd* __restrict__ Z, int conj_out, int kc,
+                                                                       int in_smem) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ long long red[2][kBtThreads];
+  __shared__ int4 fq[32];
+  __shared__ int exf[32], bad[32];
+  const int tid = threadIdx.x, nsl = kBtThreads / kc, c = tid % kc, sl = tid / kc;
+  const int k0 = blockIdx.x * kc, k = k0 + c;
+  const bool on = sl < nsl && k < n;
+  longlong2* z = in_smem ? reinterpret_cast<longlong2*>(smem_raw) + c : reinterpret_cast<longlong2*>(Z) + k;
+  const size_t ldz = in_smem ? kc : n;
+  if (tid < 32) bad[tid] = 0;
+  __syncthreads();
+  if (on)
+    for (int i = sl; i < n; i += nsl) {
+      const double x = Zt[(size_t)i * n + k];
+      if (!(fabs(x) <= 2.0)) bad[c] = 1;
+      longlong2 zi;
+      zi.x = __double2ll_rn(x * 1152921504606846976.0);  // 2^60
+      zi.y = 0;
+      z[i * ldz] = zi;
+    }
   for (int j = n - 2; j >= 0; --j) {
     const zd tj = tau[j];
-    if (tj.re == 0.0 && tj.im == 0.0) continue;
-    const zd* v = A + (size_t)j * lda + j + 1;  // v(i - j - 1) for rows i > j
-    const int i0 = j + 1 + (((sl - (j + 1)) % 32) + 32) % 32;
-    zd p = mk<double>(0.0, 0.0);
-    if (kv)
-      for (int i = i0; i < n; i += 32) cfmac(p, v[i - j - 1], Z[(size_t)i * n + k]);
-    for (int o = kBtCols; o < 32; o <<= 1) {
-      p.re += __shfl_xor_sync(0xffffffffu, p.re, o);
-      p.im += __shfl_xor_sync(0xffffffffu, p.im, o);
-    }
-    if ((threadIdx.x & 31) < kBtCols) red[threadIdx.x >> 5][c] = p;
-    __syncthreads();
-    if (threadIdx.x < kBtCols) {
-      zd t = red[0][threadIdx.x];
-      for (int w = 1; w < 8; ++w) t = cadd(t, red[w][threadIdx.x]);
-      dots[threadIdx.x] = cmul(tj, t);
-    }
-    __syncthreads();
-    const zd f = dots[c];
-    if (kv)
-      for (int i = i0; i < n; i += 32) {
-        zd z = Z[(size_t)i * n + k];
-        const zd vi = v[i - j - 1];
-        // z -= vi * f
-        z.re = fma(-vi.re, f.re, fma(vi.im, f.im, z.re));
-        z.im = fma(-vi.re, f.im, fma(-vi.im, f.re, z.im));
-        Z[(size_t)i * n + k] = z;
+    if (tj.re == 0.0 && tj.im == 0.0) continue;  // uniform
+    const int4* v = reinterpret_cast<const int4*>(A + (size_t)j * lda);
+    const int ex = exv[j];
+    const int i0 = j + 2 + ((sl - (j + 2)) % nsl + nsl) % nsl;  // this thread's first row from j + 2 on
+    const bool head = on && (j + 1) % nsl == sl;                // it owns row j + 1
+    long long rh = 0, rc = 0, ih = 0, ic = 0;
+    if (on)
+      for (int i = i0; i < n; i += nsl) {  // conj(v) z
+        const int4 a = v[i];
+        const longlong2 zi = z[i * ldz];
+        const int xl = (int)zi.x, yl = (int)zi.y;
+        const int xh = (int)(zi.x >> 32) + (xl < 0), yh = (int)(zi.y >> 32) + (yl < 0);
+        const int xs = xl >> 4, ys = yl >> 4;
+        mac(rh, rc, a.x, a.y, xh, xs);
+        mac(rh, rc, a.z, a.w, yh, ys);
+        mac(ih, ic, a.x, a.y, yh, ys);
+        mac(ih, ic, -a.z, -a.w, xh, xs);
       }
+    red[0][tid] = rh + ((rc + (1ll << 27)) >> 28);
+    red[1][tid] = ih + ((ic + (1ll << 27)) >> 28);
+    __syncthreads();
+    // the sums of a column's slices, eight lanes each, then f
+    if (tid < 8 * kc) {
+      const int cc = tid >> 3, l = tid & 7;
+      long long sr = 0, si = 0;
+      for (int q = l; q < nsl; q += 8) {
+        sr += red[0][q * kc + cc];
+        si += red[1][q * kc + cc];
+      }
+      const unsigned m = __activemask();
+      for (int o = 4; o > 0; o >>= 1) {
+        sr += __shfl_xor_sync(m, sr, o);
+        si += __shfl_xor_sync(m, si, o);
+      }
+      if (l == 0 && k0 + cc < n) {
+        const longlong2 z0 = (in_smem ? reinterpret_cast<longlong2*>(smem_raw) + cc
+                                      : reinterpret_cast<longlong2*>(Z) + k0 + cc)[(size_t)(j + 1) * ldz];
+        constexpr double u60 = 1.0 / 1152921504606846976.0;
+        const double sv = pow2(ex - kQ);
+        const zd p = mk<double>(fma((double)sr, sv, (double)z0.x * u60), fma((double)si, sv, (double)z0.y * u60));
+        const zd f = cmul(tj, p);
+        const bool ok = fabs(f.re) < 4.0 && fabs(f.im) < 4.0;
+        if (!ok) bad[cc] = 1;
+        const int ef = ok ? group_ex(max(exponent_of(f.re), exponent_of(f.im))) : kExpZero;
+        exf[cc] = ef;
+        fq[cc] = quantise(f, ef);
+      }
+    }
+    __syncthreads();
+    if (on) {
+      const int4 f = fq[c];
+      const int eh = exf[c] + 5;  // f's unit, and (below) the high sums' one, in units of z: 2^eh, 2^sh
+      if (head && eh > -62) {  // z -= f
+        longlong2 zi = z[(size_t)(j + 1) * ldz];
+        const long long fx = ((long long)f.x << 28) + f.y, fy = ((long long)f.z << 28) + f.w;
+        zi.x -= eh >= 0 ? fx << eh : (fx + (1ll << (-eh - 1))) >> -eh;
+        zi.y -= eh >= 0 ? fy << eh : (fy + (1ll << (-eh - 1))) >> -eh;
+        z[(size_t)(j + 1) * ldz] = zi;
+      }
+      const int sh = ex + eh + 1;
+      for (int i = i0; i < n; i += nsl) {  // z -= v f
+        const int4 a = v[i];
+        longlong2 zi = z[i * ldz];
+        long long xh = 0, xc = 0, yh = 0, yc = 0;
+        mac(xh, xc, a.x, a.y, f.x, f.y);
+        mac(xh, xc, -a.z, -a.w, f.z, f.w);
+        mac(yh, yc, a.x, a.y, f.z, f.w);
+        mac(yh, yc, a.z, a.w, f.x, f.y);
+        if (sh >= 0) {
+          zi.x -= (xh << sh) + ((xc + (1ll << (27 - sh))) >> (28 - sh));
+          zi.y -= (yh << sh) + ((yc + (1ll << (27 - sh))) >> (28 - sh));
+        } else if (sh > -62) {
+          const long long half = 1ll << (-sh - 1);
+          zi.x -= (xh + (xc >> 28) + half) >> -sh;
+          zi.y -= (yh + (yc >> 28) + half) >> -sh;
+        }
+        z[i * ldz] = zi;
+      }
+    }
   }
-  if (conj_out && kv)
-    for (int i = sl; i < n; i += 32) Z[(size_t)i * n + k].im = -Z[(size_t)i * n + k].im;
+  __syncthreads();
+  if (on) {
+    constexpr double u60 = 1.0 / 1152921504606846976.0;
+    const double nan = bad[c] ? __longlong_as_double(0x7ff8000000000000ll) : 0.0;
+    for (int i = sl; i < n; i += nsl) {
+      const longlong2 zi = z[i * ldz];
+      const double re = (double)zi.x * u60 + nan, im = (double)zi.y * u60 + nan;
+      Z[(size_t)i * n + k] = mk<double>(re, conj_out ? -im : im);
+    }
+  }
+}
+
+// Columns a CTA of the back-transformation: the fewest rounds of CTAs times columns, with the ~2,500 clocks of a
+// reflector's reduction hidden where several CTAs share an SM.  0: the columns do not fit shared memory.
+inline int bt_columns(int n, size_t* smem) {
+  int best = 0;
+  double cost = 0.0;
+  for (int kc = 1; kc <= 16; ++kc) {
+    const size_t b = (size_t)n * kc * sizeof(longlong2);
+    if (b > 200 * 1024) break;
+    const int res = (int)std::min<size_t>(4, (220 * 1024) / (b + 6 * 1024));
+    const long ctas = (n + kc - 1) / kc, rounds = (ctas + 152L * res - 1) / (152L * res);
+    const double work = 0.5 * n * kc * 24.0 / 21.0, t = rounds * std::max(res * work, work + 2500.0);
+    if (!best || t < cost) {
+      best = kc;
+      cost = t;
+      *smem = b;
+    }
+  }
+  return best;
 }
 
 }  // namespace
@@ -805,7 +954,7 @@ struct TriScratch {
   zd *xw, *tau, *dots, *g, *W, *P;
   double *norms, *e, *d, *ds, *e2, *bounds;
   TriCol* col;
-  int* Aex;
+  int *Aex, *exv;
   int4* Aq;
   size_t bytes;
   TriScratch(int n, void* base) {
@@ -832,6 +981,7 @@ struct TriScratch {
     e2 = reinterpret_cast<double*>(take(n * sizeof(double)));
     bounds = reinterpret_cast<double*>(take(4 * sizeof(double)));
     Aex = reinterpret_cast<int*>(take(nt * sizeof(int)));
+    exv = reinterpret_cast<int*>(take(n * sizeof(int)));
     bytes = (size_t)(p - reinterpret_cast<unsigned char*>(base));
   }
 };
@@ -920,9 +1070,18 @@ cudaError_t launch_dense_eig(zd* A, int n, int lda, bool upper_only, double* W, 
     double* work = Zt + (size_t)n * n;
     const int nb = invit_batch(n);
     for (int k0 = 0; k0 < n; k0 += nb) {
-      tri_invit_kernel<<<(nb + 127) / 128, 128, 0, s>>>(d, e, n, W, bounds, k0, nb, work, Zt); ++g_launch_count;
+      tri_invit_kernel<<<(nb + 31) / 32, 32, 0, s>>>(d, e, n, W, bounds, k0, nb, work, Zt); ++g_launch_count;
     }
-    tri_backtransform_kernel<<<(n + kBtCols - 1) / kBtCols, 256, 0, s>>>(A, n, lda, tau, Zt, Z, conj_vectors ? 1 : 0);
+    if (n > 1) {
+      tri_quantise_kernel<<<n - 1, 256, 0, s>>>(A, n, lda, t.exv); ++g_launch_count;
+    }
+    size_t smem = 0;
+    const int fit = bt_columns(n, &smem), kc = fit ? fit : 8;
+    if (!fit) smem = 0;
+    const cudaError_t eb = raise_smem_limit(reinterpret_cast<const void*>(tri_backtransform_kernel), smem);
+    if (eb != cudaSuccess) return eb;
+    tri_backtransform_kernel<<<(n + kc - 1) / kc, kBtThreads, smem, s>>>(A, n, lda, tau, t.exv, Zt, Z,
+                                                                         conj_vectors ? 1 : 0, kc, fit ? 1 : 0);
     ++g_launch_count;
   }
   return cudaGetLastError();
