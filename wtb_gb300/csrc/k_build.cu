@@ -199,17 +199,25 @@ cudaError_t launch_bse_build(const zd* vec_win, const double* dE, const double* 
 template <class S>
 cudaError_t launch_dense_mv(const cplx<S>* H, int dim, const cplx<S>* X, int ldx, cplx<S>* Y, int ldy, int ncol,
                             cudaStream_t s) {
-  // column tiles of 16 or 32 (no FMAs on padding columns); 32-row tiles when 64-row ones would leave SMs idle
+  // column tiles of 16 or 32 (no FMAs on padding columns); 32-row tiles when 64-row ones would leave SMs idle, and in
+  // FP64, where the pipe and not the operand loads is the bound, 16-row tiles while 32-row ones give fewer than four
+  // CTAs an SM (every output's sum is the same whatever the tile).  2,304 rows, 16 columns in FP64: 72 CTAs of 32 rows
+  // 1,395 us, 144 of 16 692 us (a floor of 640).
   const bool small = (dim + 63) / 64 < 2 * 152;
+  const bool tiny = sizeof(S) == 8 && (dim + 31) / 32 < 4 * 152;
   for (int c0 = 0; c0 < ncol; c0 += 32) {
     const int nc = ncol - c0 < 32 ? ncol - c0 : 32;
     if (nc <= 16) {
-      if (small)
+      if (tiny)
+        dense_mv_kernel<S, 16, 1><<<(dim + 15) / 16, 256, 0, s>>>(H, dim, X + c0, ldx, Y + c0, ldy, nc);
+      else if (small)
         dense_mv_kernel<S, 32, 1><<<(dim + 31) / 32, 256, 0, s>>>(H, dim, X + c0, ldx, Y + c0, ldy, nc);
       else
         dense_mv_kernel<S, 64, 1><<<(dim + 63) / 64, 256, 0, s>>>(H, dim, X + c0, ldx, Y + c0, ldy, nc);
     } else {
-      if (small)
+      if (tiny)
+        dense_mv_kernel<S, 16, 2><<<(dim + 15) / 16, 256, 0, s>>>(H, dim, X + c0, ldx, Y + c0, ldy, nc);
+      else if (small)
         dense_mv_kernel<S, 32, 2><<<(dim + 31) / 32, 256, 0, s>>>(H, dim, X + c0, ldx, Y + c0, ldy, nc);
       else
         dense_mv_kernel<S, 64, 2><<<(dim + 63) / 64, 256, 0, s>>>(H, dim, X + c0, ldx, Y + c0, ldy, nc);
