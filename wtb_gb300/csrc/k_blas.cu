@@ -969,6 +969,65 @@ __global__ void __launch_bounds__(256) heev_small_kernel(const zd* __restrict__ 
   }
 }
 
+// The same in FP64, one cluster of kClu CTAs per system (tridiag_cluster64), bitwise the results of one CTA: every CTA
+// forms T's eigenvalues and eigenvectors (all hold T) and every kClu-th eigenvector of A.
+// 48 x 48, 16 vectors: 597 -> 378 us; 78 x 78, 26 vectors: 1,628 -> 700 us; 16 x 16: 141 -> 124 us.  The serial chains
+// of FP64 roots and divisions are what is left.
+__global__ void __cluster_dims__(kClu, 1, 1) __launch_bounds__(256)
+    heev_cluster64_kernel(const zd* __restrict__ Ag, int lda, const int* __restrict__ nptr, int nmax, int nwant,
+                          double* __restrict__ evals, zd* __restrict__ evecs, int ldv, BatchMap bm, long a_stride,
+                          long e_stride, long v_stride) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int sys = blockIdx.x / kClu, rank = blockIdx.x % kClu;
+  if (bm_frozen(bm, sys)) return;  // uniform over the cluster
+  Ag += (size_t)sys * a_stride;
+  if (nptr) nptr += sys;
+  evals += (size_t)sys * e_stride;
+  evecs += (size_t)sys * v_stride;
+  const int n = nptr ? min(max(*nptr, 0), nmax) : nmax;
+  const int nw = min(nwant, n);
+  const int tid = threadIdx.x, nt = blockDim.x;
+  const int lds = n + 1;
+  zd* A = reinterpret_cast<zd*>(smem_raw);
+  zd* p = A + (size_t)nmax * (nmax + 1);
+  zd* w = p + nmax;
+  zd* tau = w + nmax;
+  double* d = reinterpret_cast<double*>(tau + nmax);
+  double* e = d + nmax;
+  double* e2 = e + nmax;
+  double* lam = e2 + nmax;
+  double* q = lam + nmax;
+  double* red = q + ((nmax + 1) & ~1);  // an even count of doubles before it, and 4 after: Dv is 16-byte aligned
+  // Z, Dv, Lv, vsc: nwant vectors of stride n + 1 each, regions rounded to an even count (U aliases Dv as complex)
+  const size_t zsz = ((size_t)(nmax + 1) * nwant + 1) & ~(size_t)1;
+  double* Z = red + 4;
+  double* Dv = Z + zsz;
+  double* Lv = Dv + zsz;
+  double* vsc = Lv + zsz;
+  int* cl = reinterpret_cast<int*>(vsc + zsz);
+  if (n > 0) {
+#pragma unroll 4
+    for (int x = tid; x < n * n; x += nt) {
+      const int r = x / n, c = x % n;
+      const zd a = Ag[(size_t)r * lda + c], b = Ag[(size_t)c * lda + r];
+      A[(size_t)r * lds + c] = mk<double>(0.5 * (a.re + b.re), r == c ? 0.0 : 0.5 * (a.im - b.im));
+    }
+    __syncthreads();
+    tridiag_cluster64(A, lds, n, d, e, tau, p, w, q);
+    zd* U = reinterpret_cast<zd*>(Dv);
+    tridiag_eigvecs_cta<double>(A, lds, n, nw, d, e, tau, e2, lam, Z, Dv, Lv, cl, U, n, red, rank, kClu, vsc);
+    for (int x = tid; x < nmax * nwant; x += nt) {
+      const int r = x / nwant, k = x % nwant;
+      if (k % kClu == rank) evecs[(size_t)r * ldv + k] = r < n && k < nw ? U[(size_t)k * n + r] : mk<double>(0.0, 0.0);
+    }
+    if (rank == 0)
+      for (int k = tid; k < nwant; k += nt) evals[k] = k < nw ? lam[k] : 1e30;
+  } else if (rank == 0) {
+    for (int x = tid; x < nmax * nwant; x += nt) evecs[(size_t)(x / nwant) * ldv + x % nwant] = mk<double>(0.0, 0.0);
+    for (int k = tid; k < nwant; k += nt) evals[k] = 1e30;
+  }
+}
+
 // Orthonormalising basis of the Gram matrix M = S^H S (n x n, complex(8)) by Cholesky in precision S, in the
 // basis's own order ([X W P]: the current block first) with deflation: with D = diag(M) and
 // Ms = D^-1/2 M D^-1/2, column k is kept when its residual diagonal (its squared distance from the span of the
@@ -1349,6 +1408,21 @@ cudaError_t launch_heev_small(const zd* A, int lda, const int* nptr, int nmax, i
                               int ldv, cudaStream_t s, const BatchMap& bm, long a_stride, long e_stride,
                               long v_stride) {
   if (nmax < 1 || nmax > 96 || nwant < 0 || nwant > nmax) return cudaErrorInvalidValue;
+  if constexpr (sizeof(S) == 8) {
+    // a cluster where its CTAs can have an SM each (with more systems the SMs are full of one-CTA problems, and
+    // what every CTA of a cluster repeats would be lost) and its layout fits (one warp of vectors, 90 columns)
+    const size_t smem = (size_t)nmax * (nmax + 1) * sizeof(zd) + (size_t)3 * nmax * sizeof(zd) +
+                        (size_t)(5 * nmax + 5) * sizeof(double) +
+                        (size_t)4 * ((nmax + 1) * nwant + 1) * sizeof(double) + (size_t)(nwant + 4) * sizeof(int) + 64;
+    if (bm.nsys * kClu <= 152 && nwant <= 32 && smem <= 224 * 1024) {
+      cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(heev_cluster64_kernel), smem);
+      if (e != cudaSuccess) return e;
+      heev_cluster64_kernel<<<bm.nsys * kClu, 256, smem, s>>>(A, lda, nptr, nmax, nwant, evals, evecs, ldv, bm,
+                                                              a_stride, e_stride, v_stride);
+      ++g_launch_count;
+      return cudaGetLastError();
+    }
+  }
   const size_t smem = (size_t)nmax * (nmax + 1) * sizeof(cplx<S>) + (size_t)2 * nmax * sizeof(cplx<S>) +
                       (size_t)(4 * nmax + 4) * sizeof(S) + (size_t)3 * ((nmax + 1) * nwant + 1) * sizeof(S) +
                       (size_t)(nwant + 4) * sizeof(int) + 64;

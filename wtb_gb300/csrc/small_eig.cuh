@@ -18,6 +18,8 @@
 // of the FP64 inverse-iteration vectors, and inside a cluster the Rayleigh-Ritz values of T on the cluster's
 // vectors (an FP64 instruction costs a warp far more than an FP32 one on this GPU).
 #pragma once
+#include <cooperative_groups.h>
+
 #include "wtb_internal.h"
 
 namespace wtb {
@@ -224,6 +226,186 @@ __device__ void tridiag_cta(cplx<S>* A, int lda, int n, S* d, S* e, cplx<S>* tau
   __syncthreads();
 }
 
+// Step 1 in FP64 on a cluster of kClu CTAs of 256 threads, bitwise the results of tridiag_cta<double>.  One SM issues an
+// FP64 warp instruction every 19 clocks and a warp one every 64, and the 32,000 of them of a 48 x 48 problem took
+// tridiag_cta 280 us on its SM.  Here row a of A belongs to CTA a mod kClu, which forms its entries of p = tau A22 v (eight
+// lanes a row: the four interleaved sums of tridiag_cta's two lanes, real and imaginary parts apart, added in its
+// order) and of v^H A22 v and sends them to every CTA; each then forms K and w = p + K v (once per row, not per
+// element) and updates its rows, and the next row's owner forms the reflector and sends it round.  Two cluster
+// barriers a step.  On return every CTA holds d, e, tau and the reflectors (row j right of the diagonal).
+// p, w: n complex, q: n doubles.
+constexpr int kClu = 8;
+// a b + c d with the first product fused: which product of a sum the compiler fuses is written out here, as
+// tridiag_cta<double> has it, so that the two give the same bits whatever surrounds them.
+__device__ __forceinline__ double ab_cd(double a, double b, double c, double d) { return fma(a, b, __dmul_rn(c, d)); }
+__device__ inline void tridiag_cluster64(zd* A, int lda, int n, double* d, double* e, zd* tau, zd* p, zd* w, double* q) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group clu = cg::this_cluster();
+  __shared__ double gsum[8];
+  __shared__ zd prow[96];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = (int)clu.block_rank();
+  const int cmp = lane & 1, c0 = ((lane >> 2) & 1) + (lane & 2);  // component, first column of the lane's sum
+  // the reflector of column 0, by every CTA from its own copy of row 0
+  if (n > 1 && warp == 0) reflector_warp<double>(A, lda, n, 0, d, e, tau);
+  if (n == 1 && tid == 0) d[0] = A[0].re;
+  __syncthreads();
+  clu.sync();  // every CTA has loaded its matrix before a peer writes into it
+  for (int j = 0; j < n - 1; ++j) {
+    const int L = n - 1 - j;
+    const zd* v = A + (size_t)j * lda + (j + 1);
+    zd* A22 = A + (size_t)(j + 1) * lda + (j + 1);
+    const zd tj = tau[j];
+    const bool reflect = !(tj.re == 0.0 && tj.im == 0.0);  // else A22 is unchanged
+    const int first = (rank - (j + 1) % kClu + kClu) % kClu;  // this CTA's rows of A22: first, first + kClu, ...
+    if (reflect) {
+      for (int r0 = first + kClu * 4 * warp; r0 < L; r0 += kClu * 32) {
+        const int r = r0 + kClu * (lane >> 3);
+        double acc = 0.0;
+        if (r < L) {
+          const zd* row = A22 + (size_t)r * lda;
+          const double* vd = reinterpret_cast<const double*>(v);
+          const int neg = cmp ? 0 : (int)0x80000000;
+#pragma unroll 4
+          for (int c = c0; c < L; c += 4) {
+            const zd a = row[c];
+            const double ai = __hiloint2double(__double2hiint(a.im) ^ neg, __double2loint(a.im));
+            acc = fma(a.re, vd[2 * c + cmp], acc);
+            acc = fma(ai, vd[2 * c + 1 - cmp], acc);
+          }
+        }
+        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+        acc += __shfl_xor_sync(0xffffffffu, acc, 4);
+        const double oth = __shfl_xor_sync(0xffffffffu, acc, 1);
+        const zd y = cmp ? mk<double>(oth, acc) : mk<double>(acc, oth);
+        if (r < L) {  // lane l of the row's eight writes to CTA l
+          const int to = lane & 7;
+          clu.map_shared_rank(p, to)[r] =
+              mk<double>(ab_cd(tj.re, y.re, -tj.im, y.im), ab_cd(tj.im, y.re, tj.re, y.im));
+          clu.map_shared_rank(q, to)[r] = ab_cd(v[r].re, y.re, v[r].im, y.im);
+        }
+      }
+      clu.sync();
+      // Re(v^H A22 v): sums of 16 rows as a tree, then in order
+      if (32 * warp < L) {
+        const int r = 32 * warp + lane;
+        double x = r < L ? q[r] : 0.0;
+        for (int o = 1; o < 16; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+        if ((lane & 15) == 0) gsum[2 * warp + (lane >> 4)] = x;
+      }
+      __syncthreads();
+      if (32 * warp < L) {
+        double qs = 0.0;
+        for (int g = 0; 16 * g < L; ++g) qs += gsum[g];
+        const double K = -0.5 * ab_cd(tj.re, tj.re, tj.im, tj.im) * qs;
+        const int r = 32 * warp + lane;
+        if (r < L) {
+          const zd vc = v[r], pc = p[r];
+          w[r] = mk<double>(pc.re + K * vc.re, pc.im + K * vc.im);
+        }
+      }
+      __syncthreads();
+    }
+    auto upd = [&](zd& a, const zd& vr, const zd& wr, const zd& vc, const zd& wc) {
+      a.re -= fma(wr.im, vc.im, fma(wr.re, vc.re, ab_cd(vr.re, wc.re, vr.im, wc.im)));
+      a.im -= fma(-wr.re, vc.im, fma(wr.im, vc.re, ab_cd(vr.im, wc.re, -vr.re, wc.im)));
+    };
+    const bool owner = first == 0;  // of row 0 of A22, the next pivot row
+    if (reflect) {
+      // the pivot row by the owner's warps 0 .. 2 (32 columns each), the other rows element by element
+      if (owner && 32 * warp < L) {
+        const int c = 32 * warp + lane;
+        if (c < L) {
+          zd a = A22[c];
+          upd(a, v[0], w[0], v[c], w[c]);
+          prow[c] = a;
+        }
+      }
+      if (owner) __syncthreads();  // uniform over the CTA
+    } else if (owner && warp == 0) {  // the next reflector from the row as it is
+      if (j + 1 < n - 1)
+        reflector_warp<double>(A, lda, n, j + 1, d, e, tau);
+      else if (lane == 0)
+        d[j + 1] = A22[0].re;
+      __syncwarp();
+      for (int to = 0; to < kClu; ++to) {
+        if (to == rank) continue;
+        for (int c = lane; c < L; c += 32) clu.map_shared_rank(A22, to)[c] = A22[c];
+        if (lane == 0) {
+          clu.map_shared_rank(d, to)[j + 1] = d[j + 1];
+          if (j + 1 < n - 1) {
+            clu.map_shared_rank(e, to)[j + 1] = e[j + 1];
+            clu.map_shared_rank(tau, to)[j + 1] = tau[j + 1];
+          }
+        }
+      }
+    }
+    if (reflect && owner && warp == 0) {
+      zd a[3];
+#pragma unroll
+      for (int h = 0; h < 3; ++h) a[h] = lane + 32 * h < L ? prow[lane + 32 * h] : mk<double>(0.0, 0.0);
+      const bool last = j + 1 >= n - 1;
+      double beta = 0.0;
+      zd t = mk<double>(0.0, 0.0), sc = t;
+      bool refl = false;
+      if (!last) {
+        double sg = 0.0;
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+          const int c = lane + 32 * h;
+          if (c >= 2 && c < L) sg += ab_cd(a[h].re, a[h].re, a[h].im, a[h].im);
+        }
+        sg = warp_allsum(sg);
+        const zd alpha =
+            mk<double>(__shfl_sync(0xffffffffu, a[0].re, 1), -__shfl_sync(0xffffffffu, a[0].im, 1));
+        refl = !(sg == 0.0 && alpha.im == 0.0);
+        if (!refl) {
+          beta = alpha.re;
+        } else {
+          const double an = sqrt(ab_cd(alpha.re, alpha.re, alpha.im, alpha.im) + sg);
+          beta = alpha.re >= 0.0 ? -an : an;
+          const double dr = alpha.re - beta, di = alpha.im, dd = ab_cd(di, di, dr, dr);
+          // both reciprocals by one division, on two lanes
+          const double inv = 1.0 / (lane & 1 ? dd : beta);
+          const double ib = __shfl_sync(0xffffffffu, inv, 0), idd = __shfl_sync(0xffffffffu, inv, 1);
+          t = mk<double>((beta - alpha.re) * ib, -alpha.im * ib);
+          sc = mk<double>(dr * idd, -di * idd);  // 1 / (alpha - beta)
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 3; ++h) {
+        const int c = lane + 32 * h;
+        if (c < L) {
+          zd o = a[h];  // c = 0: the diagonal
+          if (!last) {
+            if (c == 1) o = mk<double>(1.0, 0.0);
+            else if (c >= 2 && refl) {
+              o = mk<double>(ab_cd(a[h].re, sc.re, a[h].im, sc.im), ab_cd(a[h].re, sc.im, -a[h].im, sc.re));
+            }
+          }
+          for (int to = 0; to < kClu; ++to) clu.map_shared_rank(A22, to)[c] = o;
+        }
+      }
+      if (lane < kClu) {
+        clu.map_shared_rank(d, lane)[j + 1] = __shfl_sync((1u << kClu) - 1u, a[0].re, 0);
+        if (!last) {
+          clu.map_shared_rank(e, lane)[j + 1] = beta;
+          clu.map_shared_rank(tau, lane)[j + 1] = t;
+        }
+      }
+    } else if (reflect) {
+      // this CTA's rows but the pivot row, by its warps (the owner's first one is busy)
+      const int f0 = owner ? kClu : first, nr = f0 < L ? (L - f0 + kClu - 1) / kClu : 0, ne = nr * L;
+      const int t1 = owner ? tid - 32 : tid, nt1 = owner ? 224 : 256;
+      const float rL = 1.0f / (float)L;
+      for (int e2 = t1; e2 < ne; e2 += nt1) {
+        const int rr = qdiv(e2, rL), c = e2 - rr * L, r = f0 + kClu * rr;
+        upd(A22[(size_t)r * lda + c], v[r], w[r], v[c], w[c]);
+      }
+    }
+    clu.sync();
+  }
+}
+
 // Number of eigenvalues of T below x (Sturm count of T - x I, pivots safeguarded by pivmin).
 template <class S>
 __device__ __forceinline__ int sturm_count(const S* d, const S* e2, int n, S x, S pivmin) {
@@ -242,11 +424,13 @@ __device__ __forceinline__ int sturm_count(const S* d, const S* e2, int n, S x, 
 // of A column by column, U[k * ldu + i] (complex, shared memory, ldu >= n).  Scratch (shared): e2[n], and Z, Dv,
 // Lv of nwant * (n + 1) each (vector k at offset k * (n + 1): one thread per vector and one warp per vector
 // both read them without bank conflicts), Lv directly after Dv (U may alias Dv, both being dead by step 4),
-// cl[nwant] (ints), red[4].
+// cl[nwant] (ints), red[4].  The eigenvalues and T's eigenvectors are formed for every k, the vectors of A for
+// k = kfirst, kfirst + kstride, ... only (CTAs of a cluster that hold the same T share them out).  vsc: scratch of Z's
+// size for the split inverse iteration (FP64), or null.
 template <class S>
 __device__ void tridiag_eigvecs_cta(const cplx<S>* A, int lda, int n, int nwant, const S* d, const S* e,
                                     const cplx<S>* tau, S* e2, S* lam, S* Z, S* Dv, S* Lv, int* cl, cplx<S>* U,
-                                    int ldu, S* red) {
+                                    int ldu, S* red, int kfirst = 0, int kstride = 1, S* vsc = nullptr) {
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   const int ldz = n + 1;
   const S eps = sizeof(S) == 4 ? (S)5.96e-8 : (S)1.11e-16;
@@ -348,6 +532,89 @@ __device__ void tridiag_eigvecs_cta(const cplx<S>* A, int lda, int n, int nwant,
   }
   // FP32 shifts carry about 1e-7 of the spread of T: two passes reach FP32 accuracy, three FP64's
   constexpr int kPasses = sizeof(S) == 4 ? 2 : 3;
+  if (vsc) {
+    // the same operations with only the recurrences left to the one warp that holds the vectors (an FP64 instruction
+    // takes a warp 64 clocks whatever it does): the elementwise products by the whole CTA, comparisons on the bits
+    const S* sh = lam;
+    auto abs_bits = [](S x) { return __double_as_longlong((double)x) & 0x7fffffffffffffffll; };
+    const long long tiny_b = abs_bits(tiny), inf_b = 0x7ff0000000000000ll;
+    const bool mine = tid < nwant;  // nwant <= 32: one warp
+    S *zk = Z + (size_t)(mine ? tid : 0) * ldz, *dk = Dv + (size_t)(mine ? tid : 0) * ldz,
+      *lk = Lv + (size_t)(mine ? tid : 0) * ldz, *vk = vsc + (size_t)(mine ? tid : 0) * ldz;
+    __syncthreads();
+    for (int q = tid; q < nwant * n; q += nt) {
+      const int k = q / n, i = q - k * n;
+      unsigned h = (unsigned)(i + 1) * 2654435761u ^ (unsigned)(k + 7) * 2246822519u;
+      h ^= h >> 15;
+      h *= 0x2c1b3c6du;
+      h ^= h >> 12;
+      Z[(size_t)k * ldz + i] = (S)(h & 0xffffffu) * (S)(1.0 / 8388608.0) - (S)1;
+      Dv[(size_t)k * ldz + i] = d[i] - sh[k];
+    }
+    __syncthreads();
+    if (mine) {
+      S Dp = dk[0];
+      if (abs_bits(Dp) < tiny_b) Dp = tiny;
+      S Dr = (S)1 / Dp;
+      dk[0] = Dr;
+      for (int i = 1; i < n; ++i) {
+        const S l = e[i - 1] * Dr;
+        lk[i - 1] = l;
+        Dp = fma(-l, e[i - 1], dk[i]);
+        if (abs_bits(Dp) < tiny_b) Dp = tiny;
+        Dr = (S)1 / Dp;
+        dk[i] = Dr;
+      }
+    }
+    for (int pass = 0; pass < kPasses; ++pass) {
+      if (mine) {
+        S y = zk[0];
+        for (int i = 1; i < n; ++i) {
+          y = fma(-lk[i - 1], y, zk[i]);
+          zk[i] = y;
+        }
+      }
+      __syncthreads();
+      for (int q = tid; q < nwant * n; q += nt) {
+        const int k = q / n, i = q - k * n;
+        Z[(size_t)k * ldz + i] *= Dv[(size_t)k * ldz + i];
+      }
+      __syncthreads();
+      S imx = 0;
+      if (mine) {
+        S x = zk[n - 1];
+        long long mx = abs_bits(x);
+        if (mx > inf_b) mx = 0;  // fmax passes a NaN over
+        for (int i = n - 2; i >= 0; --i) {
+          x = fma(-lk[i], x, zk[i]);
+          zk[i] = x;
+          const long long b = abs_bits(x);
+          if (b > mx && b <= inf_b) mx = b;
+        }
+        S mv = (S)__longlong_as_double(mx);
+        if (mx == 0) mv = (S)1;
+        imx = (S)1 / mv;
+        vk[n] = imx;
+      }
+      __syncthreads();
+      for (int q = tid; q < nwant * n; q += nt) {
+        const int k = q / n, i = q - k * n;
+        vsc[(size_t)k * ldz + i] = Z[(size_t)k * ldz + i] * vsc[(size_t)k * ldz + n];
+      }
+      __syncthreads();
+      if (mine) {
+        S nrm = 0;
+        for (int i = 0; i < n; ++i) nrm = fma(vk[i], vk[i], nrm);
+        vk[n] = imx / sqrt(nrm);
+      }
+      __syncthreads();
+      for (int q = tid; q < nwant * n; q += nt) {
+        const int k = q / n, i = q - k * n;
+        Z[(size_t)k * ldz + i] *= vsc[(size_t)k * ldz + n];
+      }
+      __syncthreads();
+    }
+  } else
   for (int k = tid; k < nwant; k += nt) {
     S* zk = Z + (size_t)k * ldz;
     S* dk = Dv + (size_t)k * ldz;  // reciprocal pivots (one division per pivot; the solves multiply)
@@ -531,9 +798,12 @@ __device__ void tridiag_eigvecs_cta(const cplx<S>* A, int lda, int n, int nwant,
   {
     const int TS = n > 16 ? 16 : 8;
     const int tl = tid & (TS - 1), team = tid / TS, nteam = nt / TS;
-    const int kmax = (nwant + nteam - 1) / nteam * nteam;  // uniform trip count: every lane reaches the shuffles
-    for (int k = team; k < kmax; k += nteam) {
-      const bool on = k < nwant;
+    const int nk = nwant > kfirst ? (nwant - kfirst + kstride - 1) / kstride : 0;  // vectors of this CTA
+    const int kmax = (nk + nteam - 1) / nteam * nteam;  // uniform trip count: every lane reaches the shuffles
+    for (int kk = team; kk < kmax; kk += nteam) {
+      const bool on = kk < nk;
+      if (!__any_sync(0xffffffffu, on)) continue;  // a warp without a vector leaves the FP64 pipe to the others
+      const int k = kfirst + kk * kstride;
       cplx<S>* u = U + (size_t)(on ? k : 0) * ldu;
       if (on)
         for (int i = tl; i < n; i += TS) u[i] = mk<S>(Z[(size_t)k * ldz + i], 0);
