@@ -3,9 +3,9 @@
 //
 // 1. Householder tridiagonalisation A = Q T Q^H, lower form, blocked as LAPACK's zhetrd: within a panel of 32 columns
 //    the trailing matrix is left as it was, a column is brought up to date from the panel's v and w, and its Hermitian
-//    product is corrected by them; after the panel the trailing matrix takes all 32 rank-2 updates at once.  Three
-//    launches a column (the column and the w before it; the Hermitian product by 64 x 64 lower tiles; x) and one a
-//    panel.  8/3 n^3 multiply-adds: on the FP64 pipe 62 ms at n = 2,304, so the Hermitian product and the trailing
+//    product is corrected by them; after the panel the trailing matrix takes all 32 rank-2 updates at once.  Two
+//    launches a column (the Hermitian product by 64 x 64 lower tiles; x and the next column but for a multiple of v,
+//    which the next product's loads subtract) and one a panel.  8/3 n^3 multiply-adds: on the FP64 pipe 62 ms at n = 2,304, so the Hermitian product and the trailing
 //    update run as exact integer sums of quantised components (below), the rest in FP64.
 // 2. Eigenvalues of the real symmetric tridiagonal T by bisection on Sturm counts, as multisection with a few lanes
 //    per eigenvalue index where n alone would leave SMs idle, to the FP64 resolution of the Gershgorin interval.
@@ -105,10 +105,16 @@ __device__ __forceinline__ void lower_tile(int b, int* R, int* C) {
   *C = b - r * (r + 1) / 2;
 }
 
-// The column's reflector: what K2's first CTA leaves for K3.
+// The column's reflector, what K1's first CTA leaves for K2: om = 1 - sc x1, v = sc x + om e_1 for x = A(j+1:n, j),
+// x1 = x's first entry.
 struct TriCol {
-  zd tau, sc, om;  // om = 1 - sc alpha: v = sc x + om e_1 for x = A(j+1:n, j)
+  zd tau, sc, om, x1;
 };
+
+// Programmatic dependent launch: a kernel's CTAs start once every CTA of the one before has called launch_next, and
+// wait_previous returns once that kernel has completed.
+__device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // alpha = -(tau/2) sum_b dots[b], the sum split over one warp's lanes in a fixed order.
 __device__ __forceinline__ zd her2_alpha(const zd* __restrict__ dots, int ndots, zd tau) {
@@ -121,113 +127,124 @@ __device__ __forceinline__ zd her2_alpha(const zd* __restrict__ dots, int ndots,
   return cscale(cmul(tau, d), -0.5);
 }
 
-__device__ __forceinline__ zd half_warp_sum(zd a) {
-  for (int o = 8; o > 0; o >>= 1) {
-    a.re += __shfl_xor_sync(0xffffffffu, a.re, o);
-    a.im += __shfl_xor_sync(0xffffffffu, a.im, o);
-  }
-  return a;
+// a and b summed over each half warp, the four components' sums shared out over its lanes: 5 FP64 adds instead of 16.
+__device__ __forceinline__ void half_warp_sum2(zd& a, zd& b) {
+  const int lane = threadIdx.x & 31;
+  const bool h8 = lane & 8, h4 = lane & 4;
+  // lanes with bit 3 keep b, the others a
+  const double k0 = h8 ? b.re : a.re, k1 = h8 ? b.im : a.im;
+  const double g0 = h8 ? a.re : b.re, g1 = h8 ? a.im : b.im;
+  const double s0 = k0 + __shfl_xor_sync(0xffffffffu, g0, 8), s1 = k1 + __shfl_xor_sync(0xffffffffu, g1, 8);
+  // lanes with bit 2 keep the imaginary part
+  double t = (h4 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, h4 ? s0 : s1, 4);
+  t += __shfl_xor_sync(0xffffffffu, t, 2);
+  t += __shfl_xor_sync(0xffffffffu, t, 1);
+  const int base = lane & 16;
+  a.re = __shfl_sync(0xffffffffu, t, base);
+  a.im = __shfl_sync(0xffffffffu, t, base + 4);
+  b.re = __shfl_sync(0xffffffffu, t, base + 8);
+  b.im = __shfl_sync(0xffffffffu, t, base + 12);
 }
 
-constexpr int kRows = 16;  // rows of a CTA of the column kernels, 16 lanes each
+constexpr int kRows = 8;  // rows of a CTA of K2, 16 lanes each
 
-// K1, column j = j0 + i: w_{i-1} = x - (tau/2)(x^H v) v of the column before, then
-// A(j:n, j) -= sum_{l < i} v_l conj(w_l(j)) + w_l conj(v_l(j)), and the column's norm (rows from j + 2) by CTA.
-__global__ void __launch_bounds__(256) tri_col_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
-                                                      const zd* __restrict__ tau, zd* __restrict__ W,
-                                                      const zd* __restrict__ xw, const zd* __restrict__ dots, int ndots,
-                                                      double* __restrict__ norms) {
-  __shared__ zd vj[kNB], wj[kNB], s_alpha;
-  __shared__ double red[8];
-  const int tid = threadIdx.x, lane = tid & 15, j0 = j - i;
-  if (i > 0 && tid < 32) {
-    const zd al = her2_alpha(dots, ndots, tau[j - 1]);
-    if (tid == 0) s_alpha = al;
-  }
-  __syncthreads();
-  zd alpha = mk<double>(0.0, 0.0);
-  if (i > 0) alpha = s_alpha;
-  if (tid < i) {
-    const zd v = A[(size_t)(j0 + tid) * lda + j];
-    vj[tid] = v;
-    wj[tid] = tid == i - 1 ? cadd(xw[j], cmul(alpha, v)) : W[(size_t)tid * n + j];
-  }
-  __syncthreads();
-  const int r = j + blockIdx.x * kRows + tid / 16;
-  zd acc = mk<double>(0.0, 0.0);
-  if (r < n)
-    for (int l = lane; l < i; l += 16) {
-      const zd v = A[(size_t)(j0 + l) * lda + r];
-      zd w;
-      if (l == i - 1) {
-        w = cadd(xw[r], cmul(alpha, v));
-        W[(size_t)l * n + r] = w;
-      } else {
-        w = W[(size_t)l * n + r];
-      }
-      cfmac(acc, wj[l], v);
-      cfmac(acc, vj[l], w);
-    }
-  acc = half_warp_sum(acc);
-  double s2 = 0.0;
-  if (lane == 0 && r < n) {
-    zd a = csub(A[(size_t)j * lda + r], acc);
-    if (r == j) a.im = 0.0;
-    A[(size_t)j * lda + r] = a;
-    if (r > j + 1) s2 = fma(a.re, a.re, a.im * a.im);
-  }
-  s2 += __shfl_xor_sync(0xffffffffu, s2, 16);
-  if ((tid & 31) == 0) red[tid >> 5] = s2;
-  __syncthreads();
-  if (tid == 0) {
-    double t = red[0];
-    for (int w = 1; w < 8; ++w) t += red[w];
-    norms[blockIdx.x] = t;
-  }
-}
-
-// K2, with x = A(j+1:n, j) (no scaling of the reflector yet: A v = sc A x + om A(:, j+1)).
-//   CTA 0: the reflector's tau, beta, sc and om.  CTAs 1 .. i: v_l^H x and w_l^H x.
+// K1, column j = j0 + i.  The column brought up to date is x = A(j:n, j) for i = 0, else u - s v_{j-1}, with u and
+// the parts of s = 2 Re alpha, alpha = -(tau/2) x_w^H v, from K2 of the column before (w_{j-1} = x_w + alpha v_{j-1}
+// has w_{j-1}(j) = x_w(j) + alpha and v_{j-1}(j) = 1).  No scaling of the reflector yet: A v = sc A x + om A(:, j+1).
+//   CTA 0: x into column j, the reflector's tau, beta, sc and om.  CTAs 1 .. i: v_l^H x and w_l^H x; CTA i also w_{j-1}.
 //   The others, one per lower tile (R, C) of the trailing block: the quantised strict lower triangle's A_RC x_C to
 //   the rows of block R and A_RC^H x_R to the rows of block C, as P[other block][row] (a diagonal tile's second
 //   product as P[nT][row]), each (slot, row) written once.  A thread sums one row (or column) over a quarter of the
-//   tile.  Bound by the integer multiply-adds (24 an element, 21 lanes a clock and SM measured): 22 us at m = 2,304
-//   where the FP64 product took 55, 12.6 us averaged over the columns of n = 2,304.
-__global__ void __launch_bounds__(256) tri_symv_kernel(const zd* __restrict__ A, int n, int lda, int j, int i,
-                                                       const zd* __restrict__ W, const double* __restrict__ norms,
-                                                       int nnorms, const int4* __restrict__ Aq,
-                                                       const int* __restrict__ Aex, TriCol* __restrict__ col,
-                                                       zd* __restrict__ tau_out, double* __restrict__ e_out,
-                                                       zd* __restrict__ g, zd* __restrict__ P) {
+//   tile.  Bound by the integer multiply-adds (24 an element, 21 lanes a clock and SM measured): 24 us at m = 2,304
+//   where the FP64 product took 55, 14 us averaged over the columns of n = 2,304.  Within a panel the tiles' elements
+//   are on their way before the kernel before has finished.
+__global__ void __launch_bounds__(256) tri_symv_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
+                                                       zd* __restrict__ W, const zd* __restrict__ u,
+                                                       const zd* __restrict__ xw, const zd* __restrict__ dots,
+                                                       const double* __restrict__ sparts, int ndots,
+                                                       const int4* __restrict__ Aq, const int* __restrict__ Aex,
+                                                       TriCol* __restrict__ col, zd* __restrict__ tau_out,
+                                                       double* __restrict__ e_out, zd* __restrict__ g,
+                                                       zd* __restrict__ P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double s_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const zd* x = A + (size_t)j * lda;  // by absolute row, from j + 1
+  const zd* vp = A + (size_t)(j - 1) * lda;  // v_{j-1} by absolute row, read for i > 0 only
+  auto load_s = [&]() {
+    if (i > 0 && warp == 0) {
+      double t = 0.0;
+      for (int b = lane; b < ndots; b += 32) t += sparts[b];
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) s_s = t;
+    }
+    __syncthreads();
+    return i > 0 ? s_s : 0.0;
+  };
+  auto x_at = [&](int r, double s) {
+    if (i == 0) return A[(size_t)j * lda + r];
+    const zd ur = u[r], vr = vp[r];
+    return mk<double>(fma(-s, vr.re, ur.re), fma(-s, vr.im, ur.im));
+  };
   if ((int)blockIdx.x <= i) {
+    wait_previous();
+    launch_next();
+    const double s = load_s();
     zd* red = reinterpret_cast<zd*>(smem_raw);
     if (blockIdx.x == 0) {
-      if (warp == 0) {
-        double t = 0.0;
-        for (int b = lane; b < nnorms; b += 32) t += norms[b];
-        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (lane == 0) {
-          const Reflector R = make_reflector(x[j + 1], t);
-          tau_out[j] = R.tau;
-          e_out[j] = R.beta;
-          col->tau = R.tau;
-          col->sc = R.scale;
-          const zd sa = cmul(R.scale, x[j + 1]);
-          col->om = mk<double>(1.0 - sa.re, -sa.im);
-        }
+      double t = 0.0;
+      zd x1 = mk<double>(0.0, 0.0);
+      for (int r = j + tid; r < n; r += 256) {
+        zd x = x_at(r, s);
+        if (r == j) x.im = 0.0;
+        if (r == j + 1) x1 = x;  // thread 1 (row j + 1 is its first)
+        if (r > j + 1) t = fma(x.re, x.re, fma(x.im, x.im, t));
+        if (i > 0 || r == j) A[(size_t)j * lda + r] = x;
+      }
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      double* rd = reinterpret_cast<double*>(smem_raw);
+      if (lane == 0) rd[warp] = t;
+      __syncthreads();
+      if (tid == 1 && j + 1 < n) {
+        t = rd[0];
+        for (int w = 1; w < 8; ++w) t += rd[w];
+        const Reflector R = make_reflector(x1, t);
+        tau_out[j] = R.tau;
+        e_out[j] = R.beta;
+        col->tau = R.tau;
+        col->sc = R.scale;
+        const zd sa = cmul(R.scale, x1);
+        col->om = mk<double>(1.0 - sa.re, -sa.im);
+        col->x1 = x1;
       }
       return;
     }
     const int l = blockIdx.x - 1;
     const zd* v = A + (size_t)(j - i + l) * lda;
-    const zd* w = W + (size_t)l * n;
+    zd* w = W + (size_t)l * n;
+    const bool fresh = l == i - 1;  // w_{j-1} is still x_w + alpha v_{j-1}
+    zd alpha = mk<double>(0.0, 0.0);
+    if (fresh) {
+      if (warp == 0) {
+        const zd al = her2_alpha(dots, ndots, tau_out[j - 1]);
+        if (tid == 0) red[0] = al;
+      }
+      __syncthreads();
+      alpha = red[0];
+      __syncthreads();  // red is written again below
+    }
     zd gv = mk<double>(0.0, 0.0), gw = gv;
     for (int r = j + 1 + tid; r < n; r += 256) {
-      cfmac(gv, v[r], x[r]);
-      cfmac(gw, w[r], x[r]);
+      const zd x = x_at(r, s), vr = v[r];
+      zd wr;
+      if (fresh) {
+        wr = xw[r];
+        cfma(wr, alpha, vr);
+        w[r] = wr;
+      } else {
+        wr = w[r];
+      }
+      cfmac(gv, vr, x);
+      cfmac(gw, wr, x);
     }
     for (int o = 16; o > 0; o >>= 1) {
       gv.re += __shfl_xor_sync(0xffffffffu, gv.re, o);
@@ -259,17 +276,23 @@ __global__ void __launch_bounds__(256) tri_symv_kernel(const zd* __restrict__ A,
   C += C0;
   const size_t t = (size_t)R * (R + 1) / 2 + C;
   const int4* src = Aq + t * kT * kT;
+  // Aq was written by the panel's update: for i > 0 at least two kernels ago, complete before the one before this
+  // could start it
+  if (i == 0) wait_previous();
   for (int e = tid; e < kT * kT; e += 256)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
                      (uint32_t)__cvta_generic_to_shared(tile + (e / kT) * kPad + e % kT)),
                  "l"(src + e)
                  : "memory");
   asm volatile("cp.async.commit_group;" ::: "memory");
+  if (i > 0) wait_previous();
+  launch_next();
+  const double s = load_s();
   __shared__ int s_f[4];  // largest exponent fields of x over the halves of the two blocks
   zd z = mk<double>(0.0, 0.0);
   if (tid < 2 * kT) {
     const int r = (tid < kT ? R : C) * kT + tid % kT;
-    if (r > j && r < n) z = x[r];
+    if (r > j && r < n) z = x_at(r, s);
     const int f = __reduce_max_sync(0xffffffffu, max(exponent_of(z.re), exponent_of(z.im)));
     if (lane == 0) s_f[warp] = f;
   }
@@ -322,59 +345,93 @@ __global__ void __launch_bounds__(256) tri_symv_kernel(const zd* __restrict__ A,
   }
 }
 
-// K3: x_w = tau (A v - sum_l v_l (w_l^H v) + w_l (v_l^H v)) with A v = sc (P + diag x) + om A(:, j+1), v into column
-// j, and the dots conj(x_w) v by CTA.
-__global__ void __launch_bounds__(256) tri_x_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
-                                                    const zd* __restrict__ W, const zd* __restrict__ P,
-                                                    const TriCol* __restrict__ col, const zd* __restrict__ g,
-                                                    zd* __restrict__ xw, zd* __restrict__ dots) {
-  __shared__ zd gv[kNB], gw[kNB], red[8];
-  const int tid = threadIdx.x, lane = tid & 15, j0 = j - i;
+// K2: x_w = tau (A v - sum_l v_l (w_l^H v) + w_l (v_l^H v)) with A v = sc (P + diag x) + om A(:, j+1), v into column
+// j, the parts of conj(x_w) v and of -Re(tau conj(x_w) v) by CTA, and, unless column j ends its panel (next = 0), of
+// the next column
+//   u = A(:, j+1) - sum_{l < i} (v_l conj(w_l(j+1)) + w_l conj(v_l(j+1))) - v conj(x_w(j+1)) - x_w,
+// with x_w(j+1) formed by every CTA for itself (a ninth row).  FP64 instructions hold the pipe whatever the number of
+// lanes that take part, so the sums over lanes are shared out (half_warp_sum2) and the nine rows' remaining arithmetic
+// is done by nine lanes of one warp.  8.1 us averaged over the columns of n = 2,304; the two kernels took the place of
+// three (32 us a column) that brought the next column up to date by themselves: n = 2,304 84 -> 71 ms, 1,520 with
+// vectors 70 -> 54 ms.
+__global__ void __launch_bounds__(16 * (kRows + 2)) tri_x_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
+                                                                 int next, const zd* __restrict__ W,
+                                                                 const zd* __restrict__ P,
+                                                                 const TriCol* __restrict__ col,
+                                                                 const zd* __restrict__ g, zd* __restrict__ u,
+                                                                 zd* __restrict__ xw, zd* __restrict__ dots,
+                                                                 double* __restrict__ sparts) {
+  __shared__ zd gv[kNB], gw[kNB], vj[kNB], wj[kNB], sx[kRows + 1], su[kRows + 1];
+  const int tid = threadIdx.x, lane = tid & 15, half = tid / 16, j0 = j - i;
+  wait_previous();
+  launch_next();
   const zd tau = col->tau, sc = col->sc, om = col->om;
   if (tid < 2 * i) {
     const int l = tid >> 1;
     const zd at = (tid & 1) ? W[(size_t)l * n + j + 1] : A[(size_t)(j0 + l) * lda + j + 1];
+    ((tid & 1) ? wj : vj)[l] = at;
     zd t = cmul(sc, g[tid]);
     cfma(t, om, cconj(at));
     ((tid & 1) ? gw : gv)[l] = t;  // v_l^H v, w_l^H v
   }
-  __syncthreads();
-  const int r = j + 1 + blockIdx.x * kRows + tid / 16;
   const int nT = (n + kT - 1) / kT, C0 = (j + 1) / kT;
-  zd acc = mk<double>(0.0, 0.0);
-  if (r < n) {
-    zd y = mk<double>(0.0, 0.0);
+  auto row_of = [&](int h) { return h < kRows ? j + 1 + (int)blockIdx.x * kRows + h : h == kRows ? j + 1 : n; };
+  const int r = row_of(half);
+  zd y = mk<double>(0.0, 0.0);
+  if (r < n)
     for (int t = C0 + lane; t <= nT; t += 16) y = cadd(y, P[(size_t)t * n + r]);
+  __syncthreads();
+  zd acc = mk<double>(0.0, 0.0), un = acc;
+  if (r < n) {
     acc = cmul(sc, y);
     for (int l = lane; l < i; l += 16) {
       const zd v = A[(size_t)(j0 + l) * lda + r], w = W[(size_t)l * n + r];
       cfma(acc, mk<double>(-v.re, -v.im), gw[l]);
       cfma(acc, mk<double>(-w.re, -w.im), gv[l]);
+      if (next) {
+        cfmac(un, wj[l], v);
+        cfmac(un, vj[l], w);
+      }
     }
   }
-  acc = half_warp_sum(acc);
-  zd d = mk<double>(0.0, 0.0);
-  if (lane == 0 && r < n) {
-    const zd x = A[(size_t)j * lda + r];
-    const double dg = A[(size_t)r * lda + r].re;
-    zd a1 = A[(size_t)(j + 1) * lda + r];
-    if (r == j + 1) a1.im = 0.0;
-    const zd v = r == j + 1 ? mk<double>(1.0, 0.0) : cmul(sc, x);
+  half_warp_sum2(acc, un);
+  if (lane == 0 && half <= kRows) {
+    sx[half] = acc;
+    su[half] = un;
+  }
+  __syncthreads();
+  if (tid >= 32) return;
+  const int q = row_of(tid <= kRows ? tid : kRows + 1);
+  zd xr = mk<double>(0.0, 0.0), v = xr, a1 = xr, d = xr;
+  if (q < n) {
+    acc = sx[tid];
+    const zd x = q == j + 1 ? col->x1 : A[(size_t)j * lda + q];  // CTA 0 overwrites row j + 1
+    const double dg = A[(size_t)q * lda + q].re;
+    a1 = A[(size_t)(j + 1) * lda + q];
+    if (q == j + 1) a1.im = 0.0;
+    v = q == j + 1 ? mk<double>(1.0, 0.0) : cmul(sc, x);
     cfma(acc, sc, cscale(x, dg));
     cfma(acc, om, a1);
-    const zd xr = cmul(tau, acc);
-    xw[r] = xr;
-    A[(size_t)j * lda + r] = v;
+    xr = cmul(tau, acc);
+  }
+  const zd x1 = mk<double>(__shfl_sync(0xffffffffu, xr.re, kRows), __shfl_sync(0xffffffffu, xr.im, kRows));
+  if (q < n && tid < kRows) {
+    xw[q] = xr;
+    A[(size_t)j * lda + q] = v;
+    if (next) {
+      zd un1 = csub(csub(a1, su[tid]), xr);
+      cfma(un1, mk<double>(-v.re, -v.im), cconj(x1));
+      u[q] = un1;
+    }
     d = cmulc(xr, v);
   }
-  d.re += __shfl_xor_sync(0xffffffffu, d.re, 16);
-  d.im += __shfl_xor_sync(0xffffffffu, d.im, 16);
-  if ((tid & 31) == 0) red[tid >> 5] = d;
-  __syncthreads();
+  for (int o = kRows / 2; o > 0; o >>= 1) {
+    d.re += __shfl_xor_sync(0xffffffffu, d.re, o);
+    d.im += __shfl_xor_sync(0xffffffffu, d.im, o);
+  }
   if (tid == 0) {
-    zd t = red[0];
-    for (int w = 1; w < 8; ++w) t = cadd(t, red[w]);
-    dots[blockIdx.x] = t;
+    dots[blockIdx.x] = d;
+    sparts[blockIdx.x] = -cmul(tau, d).re;
   }
 }
 
@@ -951,8 +1008,8 @@ inline int bt_columns(int n, size_t* smem) {
 
 // The reduction's buffers in one scratch block.
 struct TriScratch {
-  zd *xw, *tau, *dots, *g, *W, *P;
-  double *norms, *e, *d, *ds, *e2, *bounds;
+  zd *xw, *u, *tau, *dots, *g, *W, *P;
+  double *sparts, *e, *d, *ds, *e2, *bounds;
   TriCol* col;
   int *Aex, *exv;
   int4* Aq;
@@ -970,11 +1027,12 @@ struct TriScratch {
     P = reinterpret_cast<zd*>(take((size_t)(nT + 1) * n * sizeof(zd)));
     W = reinterpret_cast<zd*>(take((size_t)kNB * n * sizeof(zd)));
     xw = reinterpret_cast<zd*>(take(n * sizeof(zd)));
+    u = reinterpret_cast<zd*>(take(n * sizeof(zd)));
     tau = reinterpret_cast<zd*>(take(n * sizeof(zd)));
     dots = reinterpret_cast<zd*>(take(nd * sizeof(zd)));
     g = reinterpret_cast<zd*>(take(2 * kNB * sizeof(zd)));
     col = reinterpret_cast<TriCol*>(take(sizeof(TriCol)));
-    norms = reinterpret_cast<double*>(take(nd * sizeof(double)));
+    sparts = reinterpret_cast<double*>(take(nd * sizeof(double)));
     e = reinterpret_cast<double*>(take(n * sizeof(double)));
     d = reinterpret_cast<double*>(take(n * sizeof(double)));
     ds = reinterpret_cast<double*>(take(n * sizeof(double)));
@@ -997,7 +1055,7 @@ cudaError_t dense_eig_prepare() {
   return err;
 }
 
-// The reduction: per column the three kernels, per panel the trailing update.
+// The reduction: per column the two kernels, per panel the trailing update.
 static cudaError_t tridiagonalise(zd* A, int n, int lda, const TriScratch& t, cudaStream_t s) {
   cudaError_t err = dense_eig_prepare();
   if (err != cudaSuccess) return err;
@@ -1008,30 +1066,38 @@ static cudaError_t tridiagonalise(zd* A, int n, int lda, const TriScratch& t, cu
     tri_update_kernel<<<tiles, 512, kUpdateSmem, s>>>(A, n, lda, j1, kb, t.tau, t.W, t.xw, t.dots, ndots, t.Aq, t.Aex);
     ++g_launch_count;
   };
-  auto column = [&](int j, int i) {
-    const int nc = (n - j + kRows - 1) / kRows;
-    tri_col_kernel<<<nc, 256, 0, s>>>(A, n, lda, j, i, t.tau, t.W, t.xw, t.dots, ndots, t.norms);
+  cudaLaunchAttribute early = {};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  auto launch = [&](auto kernel, unsigned grid, unsigned threads, size_t smem, auto... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
     ++g_launch_count;
-    return nc;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
   };
   update(0, 0);
   int i = 0;
-  for (int j = 0; j + 1 < n; ++j) {
-    const int nn = column(j, i);
-    const unsigned tiles = (unsigned)lower_tiles(nT - (j + 1) / kT);
-    tri_symv_kernel<<<tiles + 1 + i, 256, kSymvSmem, s>>>(A, n, lda, j, i, t.W, t.norms, nn, t.Aq, t.Aex,
-                                                          t.col, t.tau, t.e, t.g, t.P);
-    ++g_launch_count;
+  for (int j = 0; j < n; ++j) {
+    const bool last = j + 1 == n;  // the last column has a diagonal entry only
+    const unsigned tiles = last ? 0 : (unsigned)lower_tiles(nT - (j + 1) / kT);
+    err = launch(tri_symv_kernel, tiles + 1 + (last ? 0 : i), 256, kSymvSmem, A, n, lda, j, i, t.W, t.u, t.xw, t.dots,
+                 t.sparts, ndots, t.Aq, t.Aex, t.col, t.tau, t.e, t.g, t.P);
+    if (err != cudaSuccess || last) break;
     ndots = (n - j - 1 + kRows - 1) / kRows;
-    tri_x_kernel<<<ndots, 256, 0, s>>>(A, n, lda, j, i, t.W, t.P, t.col, t.g, t.xw, t.dots);
-    ++g_launch_count;
+    err = launch(tri_x_kernel, (unsigned)ndots, 16 * (kRows + 2), 0, A, n, lda, j, i, i + 1 < kNB ? 1 : 0, t.W, t.P,
+                 t.col, t.g, t.u, t.xw, t.dots, t.sparts);
+    if (err != cudaSuccess) break;
     if (++i == kNB) {
       update(j + 1, kNB);
       i = 0;
     }
   }
-  column(n - 1, i);  // the last diagonal entry
-  return cudaGetLastError();
+  return err == cudaSuccess ? cudaGetLastError() : err;
 }
 
 static int invit_batch(int n) {
