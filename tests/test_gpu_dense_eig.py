@@ -53,3 +53,11 @@ def test_eigenpairs(ctx, n, kind):
     assert np.linalg.norm(A @ Z - Z * W) <= 8.0 * np.sqrt(n) * EPS * nrm
     # eigenvectors of values closer than 1e-7 ||A|| are orthogonalised, the others by their gaps (eps / 1e-7)
     assert np.abs(Z.conj().T @ Z - np.eye(n)).max() <= 1e-8
+
+
+@pytest.mark.parametrize("scale", [1e-150, 1e-100, 1e150])
+@pytest.mark.parametrize("n", [33, 130])
+def test_scaled_eigenvalues(ctx, n, scale):
+    A = matrix(n, "random") * scale
+    W, ref = ctx.zheev(A), np.linalg.eigvalsh(A)
+    assert np.abs(W - ref).max() <= n * EPS * np.abs(ref).max()

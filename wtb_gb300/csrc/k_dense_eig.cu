@@ -62,8 +62,9 @@ __device__ __forceinline__ double pow2(int e) {
   return scalbn(1.0, e);
 }
 // an exact sum of products hh 2^56 + cr 2^28 of groups with exponents adding to e, as a double
-__device__ __forceinline__ double from_sums(long long hh, long long cr, double s56, double s28) {
-  return fma((double)hh, s56, (double)cr * s28);
+// (2^28 alone may lie below the range of doubles where 2^56 does not)
+__device__ __forceinline__ double from_sums(long long hh, long long cr, double s56) {
+  return fma((double)cr, 0x1p-28, (double)hh) * s56;
 }
 __device__ __forceinline__ void mac(long long& hh, long long& cr, int ah, int al, int bh, int bl) {
   hh += (long long)ah * bh;
@@ -333,13 +334,13 @@ __global__ void __launch_bounds__(256) tri_symv_kernel(zd* __restrict__ A, int n
     const int out = (second ? C : R) * kT + row;
     if (tid < kT && out < n) {
       const int e_all = Aex[t] + (second ? exR : exC) - 2 * kQ;
-      const double s56 = pow2(e_all + 56), s28 = pow2(e_all + 28);
+      const double s56 = pow2(e_all + 56);
       long long s[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) s[c] = (sums[c * kT + row] + sums[(4 + c) * kT + row]) +
                                          (sums[(8 + c) * kT + row] + sums[(12 + c) * kT + row]);
       const int slot = second ? (R == C ? nT : R) : C;
-      P[(size_t)slot * n + out] = mk<double>(from_sums(s[0], s[1], s56, s28), from_sums(s[2], s[3], s56, s28));
+      P[(size_t)slot * n + out] = mk<double>(from_sums(s[0], s[1], s56), from_sums(s[2], s[3], s56));
     }
     __syncthreads();
   }
