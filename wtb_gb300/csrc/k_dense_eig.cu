@@ -10,6 +10,8 @@
 // 2. Eigenvalues of the real symmetric tridiagonal T by bisection on Sturm counts, as multisection with a few lanes
 //    per eigenvalue index where n alone would leave SMs idle, to the FP64 resolution of the Gershgorin interval.
 //    Backward stable: |lambda - lambda_exact| <~ n eps ||A||.
+#include <cooperative_groups.h>
+
 #include <cfloat>
 
 #include "wtb_internal.h"
@@ -72,13 +74,14 @@ __device__ __forceinline__ void mac(long long& hh, long long& cr, int ah, int al
   cr += (long long)al * bh;
 }
 
-// zlarfg for x = A(j+1:n, j): returns tau, beta and the scale 1/(alpha - beta) applied to x(2:m).
+// zlarfg for x = A(j+1:n, j): returns tau, beta and the scale 1/(alpha - beta) applied to x(2:m).  By one warp, the four
+// quotients on four lanes (a division is a chain of 460 clocks).
 struct Reflector {
   zd tau, scale;
   double beta;
 };
 
-__device__ Reflector make_reflector(zd alpha, double xnorm2) {
+__device__ __forceinline__ Reflector make_reflector(zd alpha, double xnorm2) {
   Reflector r;
   if (xnorm2 == 0.0 && alpha.im == 0.0) {
     r.tau = mk<double>(0.0, 0.0);
@@ -86,14 +89,16 @@ __device__ Reflector make_reflector(zd alpha, double xnorm2) {
     r.beta = alpha.re;
     return r;
   }
+  const int lane = threadIdx.x & 31;
   const double nrm = sqrt(alpha.re * alpha.re + alpha.im * alpha.im + xnorm2);
   const double beta = alpha.re >= 0.0 ? -nrm : nrm;
   r.beta = beta;
-  r.tau = mk<double>((beta - alpha.re) / beta, -alpha.im / beta);
-  // 1 / (alpha - beta)
   const double dr = alpha.re - beta, di = alpha.im;
   const double den = dr * dr + di * di;
-  r.scale = mk<double>(dr / den, -di / den);
+  // tau = (beta - alpha) / beta, 1 / (alpha - beta) = conj(alpha - beta) / den
+  const double q = (lane & 1 ? -di : lane & 2 ? dr : -dr) / (lane & 2 ? den : beta);
+  r.tau = mk<double>(__shfl_sync(0xffffffffu, q, 0), __shfl_sync(0xffffffffu, q, 1));
+  r.scale = mk<double>(__shfl_sync(0xffffffffu, q, 2), __shfl_sync(0xffffffffu, q, 3));
   return r;
 }
 
@@ -128,45 +133,42 @@ __device__ __forceinline__ zd her2_alpha(const zd* __restrict__ dots, int ndots,
   return cscale(cmul(tau, d), -0.5);
 }
 
-// a and b summed over each half warp, the four components' sums shared out over its lanes: 5 FP64 adds instead of 16.
-__device__ __forceinline__ void half_warp_sum2(zd& a, zd& b) {
+// a summed over each half warp, the two components' sums shared out over its lanes: 4 FP64 adds instead of 8.
+__device__ __forceinline__ zd half_warp_sum(zd a) {
   const int lane = threadIdx.x & 31;
-  const bool h8 = lane & 8, h4 = lane & 4;
-  // lanes with bit 3 keep b, the others a
-  const double k0 = h8 ? b.re : a.re, k1 = h8 ? b.im : a.im;
-  const double g0 = h8 ? a.re : b.re, g1 = h8 ? a.im : b.im;
-  const double s0 = k0 + __shfl_xor_sync(0xffffffffu, g0, 8), s1 = k1 + __shfl_xor_sync(0xffffffffu, g1, 8);
-  // lanes with bit 2 keep the imaginary part
-  double t = (h4 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, h4 ? s0 : s1, 4);
-  t += __shfl_xor_sync(0xffffffffu, t, 2);
-  t += __shfl_xor_sync(0xffffffffu, t, 1);
+  const bool im = lane & 8;
+  double t = (im ? a.im : a.re) + __shfl_xor_sync(0xffffffffu, im ? a.re : a.im, 8);
+  for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   const int base = lane & 16;
-  a.re = __shfl_sync(0xffffffffu, t, base);
-  a.im = __shfl_sync(0xffffffffu, t, base + 4);
-  b.re = __shfl_sync(0xffffffffu, t, base + 8);
-  b.im = __shfl_sync(0xffffffffu, t, base + 12);
+  return mk<double>(__shfl_sync(0xffffffffu, t, base), __shfl_sync(0xffffffffu, t, base + 8));
 }
 
-constexpr int kRows = 8;  // rows of a CTA of K2, 16 lanes each
+constexpr int kRows = 8;     // rows of a CTA of K2, 16 lanes each
+constexpr int kDotRows = 512;  // rows of x whose products with one v and w take one CTA of K1
+constexpr int kNextRows = 16;  // rows of the next column of a CTA of K1
 
 // K1, column j = j0 + i.  The column brought up to date is x = A(j:n, j) for i = 0, else u - s v_{j-1}, with u and
 // the parts of s = 2 Re alpha, alpha = -(tau/2) x_w^H v, from K2 of the column before (w_{j-1} = x_w + alpha v_{j-1}
 // has w_{j-1}(j) = x_w(j) + alpha and v_{j-1}(j) = 1).  No scaling of the reflector yet: A v = sc A x + om A(:, j+1).
-//   CTA 0: x into column j, the reflector's tau, beta, sc and om.  CTAs 1 .. i: v_l^H x and w_l^H x; CTA i also w_{j-1}.
+//   CTA 0: x into column j, the reflector's tau, beta, sc and om.  The next i nch: v_l^H x and w_l^H x over 512 rows
+//   each (an SM issues an FP64 instruction every 19 clocks: over all 2,304 rows they outlasted the tiles), the last
+//   l's also w_{j-1}.  The next nnext: next(r) = A(r, j+1) - sum_{l < i} (v_l(r) conj(w_l(j+1)) + w_l(r) conj(v_l(j+1)))
+//   over 16 rows each, for K2 (FP64 work beside the tiles' integer work; in K2 it took 2 to 3 us).
 //   The others, one per lower tile (R, C) of the trailing block: the quantised strict lower triangle's A_RC x_C to
 //   the rows of block R and A_RC^H x_R to the rows of block C, as P[other block][row] (a diagonal tile's second
 //   product as P[nT][row]), each (slot, row) written once.  A thread sums one row (or column) over a quarter of the
-//   tile.  Bound by the integer multiply-adds (24 an element, 21 lanes a clock and SM measured): 24 us at m = 2,304
-//   where the FP64 product took 55, 14 us averaged over the columns of n = 2,304.  Within a panel the tiles' elements
-//   are on their way before the kernel before has finished.
-__global__ void __launch_bounds__(256) tri_symv_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
+//   tile.  Large trailing blocks are bound by the integer multiply-adds (18 an element) and the tiles' way from L2: 17 us
+//   at m = 2,304 where the FP64 product took 55; small ones by the chain of waits and FP64 sums, 7 to 9 us; 11.9 us
+//   averaged over the columns of n = 2,304 (14.1 with four real products, two CTAs an SM and one CTA per v and w).
+//   Within a panel the tiles' elements are on their way before the kernel before has finished.
+__global__ void __launch_bounds__(256, 3) tri_symv_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
                                                        zd* __restrict__ W, const zd* __restrict__ u,
                                                        const zd* __restrict__ xw, const zd* __restrict__ dots,
                                                        const double* __restrict__ sparts, int ndots,
                                                        const int4* __restrict__ Aq, const int* __restrict__ Aex,
                                                        TriCol* __restrict__ col, zd* __restrict__ tau_out,
-                                                       double* __restrict__ e_out, zd* __restrict__ g,
-                                                       zd* __restrict__ P) {
+                                                       double* __restrict__ e_out, zd* __restrict__ g, int nch,
+                                                       zd* __restrict__ next, int nnext, zd* __restrict__ P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -186,18 +188,63 @@ __global__ void __launch_bounds__(256) tri_symv_kernel(zd* __restrict__ A, int n
     const zd ur = u[r], vr = vp[r];
     return mk<double>(fma(-s, vr.re, ur.re), fma(-s, vr.im, ur.im));
   };
-  if ((int)blockIdx.x <= i) {
+  const int ndot = i * nch;
+  if ((int)blockIdx.x > ndot && (int)blockIdx.x <= ndot + nnext) {
+    __shared__ zd s_al, vj[kNB], wj[kNB];
+    const int l16 = tid & 15, r = j + 1 + ((int)blockIdx.x - ndot - 1) * kNextRows + tid / 16, j0 = j - i;
+    wait_previous();
+    launch_next();
+    if (warp == 0 && i > 0) {
+      const zd al = her2_alpha(dots, ndots, tau_out[j - 1]);
+      if (tid == 0) s_al = al;
+    }
+    zd v[2], w[2], a = mk<double>(0.0, 0.0);
+    if (r < n) a = A[(size_t)(j + 1) * lda + r];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int l = l16 + 16 * h;
+      v[h] = w[h] = mk<double>(0.0, 0.0);
+      if (r < n && l < i) {
+        v[h] = A[(size_t)(j0 + l) * lda + r];
+        w[h] = l < i - 1 ? W[(size_t)l * n + r] : xw[r];
+      }
+    }
+    __syncthreads();
+    if (tid < i) {
+      const zd v1 = A[(size_t)(j0 + tid) * lda + j + 1];
+      zd w1 = tid < i - 1 ? W[(size_t)tid * n + j + 1] : xw[j + 1];
+      if (tid == i - 1) cfma(w1, s_al, v1);
+      vj[tid] = v1;
+      wj[tid] = w1;
+    }
+    __syncthreads();
+    zd t = mk<double>(0.0, 0.0);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      if (16 * h < i) {  // uniform
+        const int l = l16 + 16 * h;
+        if (l == i - 1) cfma(w[h], s_al, v[h]);
+        if (l < i) {
+          cfmac(t, wj[l], v[h]);
+          cfmac(t, vj[l], w[h]);
+        }
+      }
+    t = half_warp_sum(t);
+    if (l16 == 0 && r < n) next[r] = mk<double>(a.re - t.re, r == j + 1 ? 0.0 : a.im - t.im);
+    return;
+  }
+  if ((int)blockIdx.x <= ndot) {
     wait_previous();
     launch_next();
     const double s = load_s();
     zd* red = reinterpret_cast<zd*>(smem_raw);
     if (blockIdx.x == 0) {
       double t = 0.0;
-      zd x1 = mk<double>(0.0, 0.0);
+      __shared__ zd s_x1;
       for (int r = j + tid; r < n; r += 256) {
         zd x = x_at(r, s);
         if (r == j) x.im = 0.0;
-        if (r == j + 1) x1 = x;  // thread 1 (row j + 1 is its first)
+        if (r == j + 1) s_x1 = x;
         if (r > j + 1) t = fma(x.re, x.re, fma(x.im, x.im, t));
         if (i > 0 || r == j) A[(size_t)j * lda + r] = x;
       }
@@ -205,21 +252,24 @@ __global__ void __launch_bounds__(256) tri_symv_kernel(zd* __restrict__ A, int n
       double* rd = reinterpret_cast<double*>(smem_raw);
       if (lane == 0) rd[warp] = t;
       __syncthreads();
-      if (tid == 1 && j + 1 < n) {
-        t = rd[0];
-        for (int w = 1; w < 8; ++w) t += rd[w];
+      if (warp == 0 && j + 1 < n) {
+        t = rd[lane & 7];
+        for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        const zd x1 = s_x1;
         const Reflector R = make_reflector(x1, t);
-        tau_out[j] = R.tau;
-        e_out[j] = R.beta;
-        col->tau = R.tau;
-        col->sc = R.scale;
-        const zd sa = cmul(R.scale, x1);
-        col->om = mk<double>(1.0 - sa.re, -sa.im);
-        col->x1 = x1;
+        if (lane == 0) {
+          tau_out[j] = R.tau;
+          e_out[j] = R.beta;
+          col->tau = R.tau;
+          col->sc = R.scale;
+          const zd sa = cmul(R.scale, x1);
+          col->om = mk<double>(1.0 - sa.re, -sa.im);
+          col->x1 = x1;
+        }
       }
       return;
     }
-    const int l = blockIdx.x - 1;
+    const int ch = (blockIdx.x - 1) % nch, l = (blockIdx.x - 1) / nch;
     const zd* v = A + (size_t)(j - i + l) * lda;
     zd* w = W + (size_t)l * n;
     const bool fresh = l == i - 1;  // w_{j-1} is still x_w + alpha v_{j-1}
@@ -234,7 +284,7 @@ __global__ void __launch_bounds__(256) tri_symv_kernel(zd* __restrict__ A, int n
       __syncthreads();  // red is written again below
     }
     zd gv = mk<double>(0.0, 0.0), gw = gv;
-    for (int r = j + 1 + tid; r < n; r += 256) {
+    for (int r = j + 1 + ch * kDotRows + tid; r < min(n, j + 1 + (ch + 1) * kDotRows); r += 256) {
       const zd x = x_at(r, s), vr = v[r];
       zd wr;
       if (fresh) {
@@ -261,18 +311,18 @@ __global__ void __launch_bounds__(256) tri_symv_kernel(zd* __restrict__ A, int n
     if (tid < 2) {
       zd t = red[tid];
       for (int q = 1; q < 8; ++q) t = cadd(t, red[2 * q + tid]);
-      g[2 * l + tid] = t;
+      g[ch * 2 * kNB + 2 * l + tid] = t;
     }
     return;
   }
   constexpr int kPad = kT + 1;                       // conflict-free columns and rows
   int4* tile = reinterpret_cast<int4*>(smem_raw);    // [column][row]
-  int4* xR = tile + kT * kPad;
-  int4* xC = xR + kT;
-  long long* sums = reinterpret_cast<long long*>(xC + kT);  // [4 quarters][4][kT]
+  int4* xa = tile + kT * kPad;                       // rows' 64 entries of x, then the columns': re, im - re
+  int2* xb = reinterpret_cast<int2*>(xa + 2 * kT);   // re + im
+  long long* sums = reinterpret_cast<long long*>(smem_raw);  // [2][4 quarters][4][kT], over the tile once it is used
   const int nT = (n + kT - 1) / kT, C0 = (j + 1) / kT;
   int R, C;
-  lower_tile(blockIdx.x - i - 1, &R, &C);
+  lower_tile(blockIdx.x - ndot - nnext - 1, &R, &C);
   R += C0;
   C += C0;
   const size_t t = (size_t)R * (R + 1) / 2 + C;
@@ -288,81 +338,100 @@ __global__ void __launch_bounds__(256) tri_symv_kernel(zd* __restrict__ A, int n
   asm volatile("cp.async.commit_group;" ::: "memory");
   if (i > 0) wait_previous();
   launch_next();
-  const double s = load_s();
   __shared__ int s_f[4];  // largest exponent fields of x over the halves of the two blocks
-  zd z = mk<double>(0.0, 0.0);
+  zd z = mk<double>(0.0, 0.0), zv = z;
   if (tid < 2 * kT) {
     const int r = (tid < kT ? R : C) * kT + tid % kT;
-    if (r > j && r < n) z = x_at(r, s);
+    if (r > j && r < n) {
+      z = i == 0 ? A[(size_t)j * lda + r] : u[r];
+      if (i > 0) zv = vp[r];
+    }
+  }
+  const double s = load_s();
+  if (tid < 2 * kT) {
+    if (i > 0) z = mk<double>(fma(-s, zv.re, z.re), fma(-s, zv.im, z.im));
     const int f = __reduce_max_sync(0xffffffffu, max(exponent_of(z.re), exponent_of(z.im)));
     if (lane == 0) s_f[warp] = f;
   }
   __syncthreads();
   const int exR = group_ex(max(s_f[0], s_f[1])), exC = group_ex(max(s_f[2], s_f[3]));
-  if (tid < 2 * kT) (tid < kT ? xR : xC)[tid % kT] = quantise(z, tid < kT ? exR : exC);
+  if (tid < 2 * kT) {
+    const int4 q = quantise(z, tid < kT ? exR : exC);
+    xa[tid] = make_int4(q.x, q.y, q.z - q.x, q.w - q.y);
+    xb[tid] = make_int2(q.x + q.z, q.y + q.w);
+  }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   const int row = tid % kT, q0 = (tid / kT) * (kT / 4);
-#pragma unroll 1
+  // a complex product by three real ones (all exact, so the sums are those of four): with s = b.re (a.re + a.im),
+  // a b = s - a.im (b.re + b.im) + i (s + a.re (b.im - b.re)), and conj(a) b the same with -a.im
+  long long o[2][4];
+#pragma unroll
   for (int second = 0; second < 2; ++second) {
-    long long rh = 0, rc = 0, ih = 0, ic = 0;
+    long long sh = 0, sl = 0, ph = 0, pl = 0, mh = 0, ml = 0;
     if (!second) {
 #pragma unroll 4
-      for (int c = q0; c < q0 + kT / 4; ++c) {  // a x
-        const int4 a = tile[c * kPad + row], b = xC[c];
-        mac(rh, rc, a.x, a.y, b.x, b.y);
-        mac(rh, rc, -a.z, -a.w, b.z, b.w);
-        mac(ih, ic, a.x, a.y, b.z, b.w);
-        mac(ih, ic, a.z, a.w, b.x, b.y);
+      for (int c = q0; c < q0 + kT / 4; ++c) {
+        const int4 a = tile[c * kPad + row], b = xa[kT + c];
+        const int2 p = xb[kT + c];
+        mac(sh, sl, a.x + a.z, a.y + a.w, b.x, b.y);
+        mac(ph, pl, a.z, a.w, p.x, p.y);
+        mac(mh, ml, a.x, a.y, b.z, b.w);
       }
+      ph = -ph;
+      pl = -pl;
     } else {
 #pragma unroll 4
-      for (int r = q0; r < q0 + kT / 4; ++r) {  // conj(a) x
-        const int4 a = tile[row * kPad + r], b = xR[r];
-        mac(rh, rc, a.x, a.y, b.x, b.y);
-        mac(rh, rc, a.z, a.w, b.z, b.w);
-        mac(ih, ic, a.x, a.y, b.z, b.w);
-        mac(ih, ic, -a.z, -a.w, b.x, b.y);
+      for (int r = q0; r < q0 + kT / 4; ++r) {
+        const int4 a = tile[row * kPad + r], b = xa[r];
+        const int2 p = xb[r];
+        mac(sh, sl, a.x - a.z, a.y - a.w, b.x, b.y);
+        mac(ph, pl, a.z, a.w, p.x, p.y);
+        mac(mh, ml, a.x, a.y, b.z, b.w);
       }
     }
-    long long* o = sums + (tid / kT) * 4 * kT + row;
-    o[0] = rh;
-    o[kT] = rc;
-    o[2 * kT] = ih;
-    o[3 * kT] = ic;
-    __syncthreads();
-    const int out = (second ? C : R) * kT + row;
-    if (tid < kT && out < n) {
-      const int e_all = Aex[t] + (second ? exR : exC) - 2 * kQ;
-      const double s56 = pow2(e_all + 56);
-      long long s[4];
+    o[second][0] = sh + ph;
+    o[second][1] = sl + pl;
+    o[second][2] = sh + mh;
+    o[second][3] = sl + ml;
+  }
+  __syncthreads();
 #pragma unroll
-      for (int c = 0; c < 4; ++c) s[c] = (sums[c * kT + row] + sums[(4 + c) * kT + row]) +
-                                         (sums[(8 + c) * kT + row] + sums[(12 + c) * kT + row]);
-      const int slot = second ? (R == C ? nT : R) : C;
-      P[(size_t)slot * n + out] = mk<double>(from_sums(s[0], s[1], s56), from_sums(s[2], s[3], s56));
-    }
-    __syncthreads();
+  for (int second = 0; second < 2; ++second)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) sums[((second * 4 + tid / kT) * 4 + c) * kT + row] = o[second][c];
+  __syncthreads();
+  const int second = tid / kT, out = (second ? C : R) * kT + row;
+  if (tid < 2 * kT && out < n) {
+    const double s56 = pow2(Aex[t] + (second ? exR : exC) - 2 * kQ + 56);
+    const long long* q = sums + second * 16 * kT + row;
+    long long v[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[c] = (q[c * kT] + q[(4 + c) * kT]) + (q[(8 + c) * kT] + q[(12 + c) * kT]);
+    const int slot = second ? (R == C ? nT : R) : C;
+    P[(size_t)slot * n + out] = mk<double>(from_sums(v[0], v[1], s56), from_sums(v[2], v[3], s56));
   }
 }
 
 // K2: x_w = tau (A v - sum_l v_l (w_l^H v) + w_l (v_l^H v)) with A v = sc (P + diag x) + om A(:, j+1), v into column
-// j, the parts of conj(x_w) v and of -Re(tau conj(x_w) v) by CTA, and, unless column j ends its panel (next = 0), of
+// j, the parts of conj(x_w) v and of -Re(tau conj(x_w) v) by CTA, and, unless column j ends its panel (next null), of
 // the next column
-//   u = A(:, j+1) - sum_{l < i} (v_l conj(w_l(j+1)) + w_l conj(v_l(j+1))) - v conj(x_w(j+1)) - x_w,
+//   u = next - v conj(x_w(j+1)) - x_w,
 // with x_w(j+1) formed by every CTA for itself (a ninth row).  FP64 instructions hold the pipe whatever the number of
-// lanes that take part, so the sums over lanes are shared out (half_warp_sum2) and the nine rows' remaining arithmetic
-// is done by nine lanes of one warp.  8.1 us averaged over the columns of n = 2,304; the two kernels took the place of
-// three (32 us a column) that brought the next column up to date by themselves: n = 2,304 84 -> 71 ms, 1,520 with
-// vectors 70 -> 54 ms.
+// lanes that take part, so the sums over lanes are shared out (half_warp_sum) and the nine rows' remaining arithmetic
+// is done by nine lanes of one warp.  7.1 us averaged over the columns of n = 2,304 (8.1 with the sums of next formed
+// here); the two kernels took the place of three (32 us a column) that brought the next column up to date by
+// themselves: n = 2,304 84 -> 71 ms, and 65 with both as they are.
 __global__ void __launch_bounds__(16 * (kRows + 2)) tri_x_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
-                                                                 int next, const zd* __restrict__ W,
+                                                                 const zd* __restrict__ next,
+                                                                 const zd* __restrict__ W,
                                                                  const zd* __restrict__ P,
                                                                  const TriCol* __restrict__ col,
-                                                                 const zd* __restrict__ g, zd* __restrict__ u,
+                                                                 const zd* __restrict__ g, int nch,
+                                                                 zd* __restrict__ u,
                                                                  zd* __restrict__ xw, zd* __restrict__ dots,
                                                                  double* __restrict__ sparts) {
-  __shared__ zd gv[kNB], gw[kNB], vj[kNB], wj[kNB], sx[kRows + 1], su[kRows + 1];
+  __shared__ zd gv[kNB], gw[kNB], sx[kRows + 1];
   const int tid = threadIdx.x, lane = tid & 15, half = tid / 16, j0 = j - i;
   wait_previous();
   launch_next();
@@ -370,45 +439,43 @@ __global__ void __launch_bounds__(16 * (kRows + 2)) tri_x_kernel(zd* __restrict_
   if (tid < 2 * i) {
     const int l = tid >> 1;
     const zd at = (tid & 1) ? W[(size_t)l * n + j + 1] : A[(size_t)(j0 + l) * lda + j + 1];
-    ((tid & 1) ? wj : vj)[l] = at;
-    zd t = cmul(sc, g[tid]);
+    zd gs = g[tid];
+    for (int c = 1; c < nch; ++c) gs = cadd(gs, g[c * 2 * kNB + tid]);
+    zd t = cmul(sc, gs);
     cfma(t, om, cconj(at));
     ((tid & 1) ? gw : gv)[l] = t;  // v_l^H v, w_l^H v
   }
   const int nT = (n + kT - 1) / kT, C0 = (j + 1) / kT;
   auto row_of = [&](int h) { return h < kRows ? j + 1 + (int)blockIdx.x * kRows + h : h == kRows ? j + 1 : n; };
-  const int r = row_of(half);
+  const int r = row_of(half), q = row_of(tid <= kRows ? tid : kRows + 1);
+  zd x = mk<double>(0.0, 0.0), a1 = x, un = x;
+  double dg = 0.0;
+  if (q < n) {  // for the last part, on their way meanwhile
+    x = q == j + 1 ? col->x1 : A[(size_t)j * lda + q];  // CTA 0 overwrites row j + 1
+    dg = A[(size_t)q * lda + q].re;
+    a1 = A[(size_t)(j + 1) * lda + q];
+    if (next) un = next[q];
+  }
   zd y = mk<double>(0.0, 0.0);
   if (r < n)
     for (int t = C0 + lane; t <= nT; t += 16) y = cadd(y, P[(size_t)t * n + r]);
   __syncthreads();
-  zd acc = mk<double>(0.0, 0.0), un = acc;
+  zd acc = mk<double>(0.0, 0.0);
   if (r < n) {
     acc = cmul(sc, y);
     for (int l = lane; l < i; l += 16) {
       const zd v = A[(size_t)(j0 + l) * lda + r], w = W[(size_t)l * n + r];
       cfma(acc, mk<double>(-v.re, -v.im), gw[l]);
       cfma(acc, mk<double>(-w.re, -w.im), gv[l]);
-      if (next) {
-        cfmac(un, wj[l], v);
-        cfmac(un, vj[l], w);
-      }
     }
   }
-  half_warp_sum2(acc, un);
-  if (lane == 0 && half <= kRows) {
-    sx[half] = acc;
-    su[half] = un;
-  }
+  acc = half_warp_sum(acc);
+  if (lane == 0 && half <= kRows) sx[half] = acc;
   __syncthreads();
   if (tid >= 32) return;
-  const int q = row_of(tid <= kRows ? tid : kRows + 1);
-  zd xr = mk<double>(0.0, 0.0), v = xr, a1 = xr, d = xr;
+  zd xr = mk<double>(0.0, 0.0), v = xr, d = xr;
   if (q < n) {
     acc = sx[tid];
-    const zd x = q == j + 1 ? col->x1 : A[(size_t)j * lda + q];  // CTA 0 overwrites row j + 1
-    const double dg = A[(size_t)q * lda + q].re;
-    a1 = A[(size_t)(j + 1) * lda + q];
     if (q == j + 1) a1.im = 0.0;
     v = q == j + 1 ? mk<double>(1.0, 0.0) : cmul(sc, x);
     cfma(acc, sc, cscale(x, dg));
@@ -420,7 +487,7 @@ __global__ void __launch_bounds__(16 * (kRows + 2)) tri_x_kernel(zd* __restrict_
     xw[q] = xr;
     A[(size_t)j * lda + q] = v;
     if (next) {
-      zd un1 = csub(csub(a1, su[tid]), xr);
+      zd un1 = csub(un, xr);
       cfma(un1, mk<double>(-v.re, -v.im), cconj(x1));
       u[q] = un1;
     }
@@ -436,54 +503,66 @@ __global__ void __launch_bounds__(16 * (kRows + 2)) tri_x_kernel(zd* __restrict_
   }
 }
 
-// After a panel of kb reflectors (columns j1 - kb .. j1 - 1): A(r, c) -= sum_l v_l(r) conj(w_l(c)) + w_l(r) conj(v_l(c))
-// for r >= c >= j1, one CTA per 64 x 64 tile, the products quantised, then the tile's own quantised form (strict lower
-// triangle) for the next panel's Hermitian products.  kb = 0: only that.  512 threads, 4 x 2 entries each.  Bound by
-// the integer multiply-adds (768 an entry): 404 us at m = 2,304, where 32 FP64 rank-2 updates took 1.6 ms; all panels of
-// n = 2,304 13 ms against 55.
-__global__ void __launch_bounds__(512, 1) tri_update_kernel(zd* __restrict__ A, int n, int lda, int j1, int kb,
-                                                            const zd* __restrict__ tau, const zd* __restrict__ W,
-                                                            const zd* __restrict__ xw, const zd* __restrict__ dots,
-                                                            int ndots, int4* __restrict__ Aq, int* __restrict__ Aex) {
+// After a panel (columns j1 - 32 .. j1 - 1): A(r, c) -= sum_l v_l(r) conj(w_l(c)) + w_l(r) conj(v_l(c))
+// for r >= c >= j1, one cluster of two CTAs per 64 x 64 tile (32 columns each: one CTA's time is 80 us for the last
+// tiles), the products quantised, then the tile's own quantised form (strict lower triangle) for the next panel's
+// Hermitian products, on the larger exponent of the two.  reflectors = 0: only that.  512 threads, 4 entries each.  A complex
+// product a conj(b) takes three real ones: with s = b.re (a.re + a.im), it is s - a.im (b.re - b.im)
+// + i (s - a.re (b.re + b.im)), all exact.  Bound by the integer multiply-adds (576 an entry), 9 of a
+// CTA's 39 us its loads and the quantising: 350 us at m = 2,240, where four real products on whole tiles took 399 and 32
+// FP64 rank-2 updates 1.6 ms; averaged over the panels of n = 2,304 176 -> 148 us.
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(512, 1)
+    tri_update_kernel(zd* __restrict__ A, int n, int lda, int j1, int reflectors, const zd* __restrict__ tau,
+                      const zd* __restrict__ W, const zd* __restrict__ xw, const zd* __restrict__ dots, int ndots,
+                      int4* __restrict__ Aq, int* __restrict__ Aex) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group clu = cg::this_cluster();
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int kH = kT / 2;
   int4* vR = reinterpret_cast<int4*>(smem_raw);  // [kNB][kT] each
   int4* wR = vR + kNB * kT;
-  int4* vC = wR + kNB * kT;
-  int4* wC = vC + kNB * kT;
+  int4* vC = wR + kNB * kT;  // [kNB][kH] each
+  int4* wC = vC + kNB * kH;
   __shared__ zd s_alpha;
   __shared__ int s_exv, s_exw, s_ext;
-  const int tid = threadIdx.x, C0 = j1 / kT;
+  const int tid = threadIdx.x, C0 = j1 / kT, c0 = (blockIdx.x & 1) * kH;
   int R, C;
-  lower_tile(blockIdx.x, &R, &C);
+  lower_tile(blockIdx.x / 2, &R, &C);
   R += C0;
   C += C0;
   if (tid == 0) s_exv = s_exw = s_ext = 0;
-  if (kb > 0 && tid < 32) {
+  if (reflectors && tid < 32) {
     const zd al = her2_alpha(dots, ndots, tau[j1 - 1]);
     if (tid == 0) s_alpha = al;
   }
   __syncthreads();
   const int tr = tid % 16, tc = tid / 16;
-  long long rh[8], rc[8], ih[8], ic[8];
+  long long rh[4], rc[4], ih[4], ic[4];
 #pragma unroll
-  for (int e = 0; e < 8; ++e) rh[e] = rc[e] = ih[e] = ic[e] = 0;
+  for (int e = 0; e < 4; ++e) rh[e] = rc[e] = ih[e] = ic[e] = 0;
   double scale = 0.0;
-  if (kb > 0) {
-    const zd alpha = s_alpha;
-    auto w_at = [&](int l, int r) {  // the last column's w is still x - (tau/2)(x^H v) v
-      if (r < j1 || r >= n) return mk<double>(0.0, 0.0);
-      if (l < kb - 1) return W[(size_t)l * n + r];
-      return cadd(xw[r], cmul(alpha, A[(size_t)(j1 - 1) * lda + r]));
-    };
-    auto v_at = [&](int l, int r) {
-      return r >= j1 && r < n ? A[(size_t)(j1 - kb + l) * lda + r] : mk<double>(0.0, 0.0);
-    };
+  if (reflectors) {
+    // v and w of the tile's rows, then of its columns: all loads in flight at once, quantised once the largest exponent
+    // is known
+    constexpr int kG = kT + kH, kE = kG * kNB / 512;
+    auto at = [&](int rr) { return rr < kT ? R * kT + rr : C * kT + c0 + rr - kT; };
+    zd v[kE], w[kE];
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+      const int e = tid + 512 * q, l = e / kG, r = at(e % kG);
+      v[q] = w[q] = mk<double>(0.0, 0.0);
+      if (r >= j1 && r < n) {
+        v[q] = A[(size_t)(j1 - kNB + l) * lda + r];
+        w[q] = l < kNB - 1 ? W[(size_t)l * n + r] : xw[r];
+      }
+    }
     int fv = 0, fw = 0;
-    for (int e = tid; e < 2 * kb * kT; e += 512) {
-      const int l = e / (2 * kT), rr = e % (2 * kT), r = (rr < kT ? R : C) * kT + rr % kT;
-      const zd v = v_at(l, r), w = w_at(l, r);
-      fv = max(fv, max(exponent_of(v.re), exponent_of(v.im)));
-      fw = max(fw, max(exponent_of(w.re), exponent_of(w.im)));
+    const zd alpha = s_alpha;
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+      if ((tid + 512 * q) / kG == kNB - 1) cfma(w[q], alpha, v[q]);  // still x - (tau/2)(x^H v) v
+      fv = max(fv, max(exponent_of(v[q].re), exponent_of(v[q].im)));
+      fw = max(fw, max(exponent_of(w[q].re), exponent_of(w[q].im)));
     }
     fv = __reduce_max_sync(0xffffffffu, fv);
     fw = __reduce_max_sync(0xffffffffu, fw);
@@ -493,49 +572,54 @@ __global__ void __launch_bounds__(512, 1) tri_update_kernel(zd* __restrict__ A, 
     }
     __syncthreads();
     const int exv = group_ex(s_exv), exw = group_ex(s_exw);
-    for (int e = tid; e < 2 * kb * kT; e += 512) {
-      const int l = e / (2 * kT), rr = e % (2 * kT), r = (rr < kT ? R : C) * kT + rr % kT;
-      (rr < kT ? wR : wC)[l * kT + rr % kT] = quantise(w_at(l, r), exw);
-      (rr < kT ? vR : vC)[l * kT + rr % kT] = quantise(v_at(l, r), exv);
+#pragma unroll
+    for (int q = 0; q < kE; ++q) {
+      const int e = tid + 512 * q, l = e / kG, rr = e % kG;
+      *(rr < kT ? wR + l * kT + rr : wC + l * kH + rr - kT) = quantise(w[q], exw);
+      *(rr < kT ? vR + l * kT + rr : vC + l * kH + rr - kT) = quantise(v[q], exv);
     }
     __syncthreads();
-    for (int l = 0; l < kb; ++l) {
-      int4 v2[2], w2[2];
+    long long sh[4], sl[4];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        v2[c] = vC[l * kT + tc + 32 * c];
-        w2[c] = wC[l * kT + tc + 32 * c];
+    for (int e = 0; e < 4; ++e) sh[e] = sl[e] = 0;
+    auto product = [&](int e, const int4& a, const int2& as, const int4& b, const int2& bd, const int2& bs) {
+      mac(sh[e], sl[e], as.x, as.y, b.x, b.y);
+      mac(rh[e], rc[e], a.z, a.w, bd.x, bd.y);
+      mac(ih[e], ic[e], a.x, a.y, bs.x, bs.y);
+    };
+    auto sum = [](const int4& a) { return make_int2(a.x + a.z, a.y + a.w); };
+    auto dif = [](const int4& a) { return make_int2(a.x - a.z, a.y - a.w); };
+    for (int l = 0; l < kNB; ++l) {
+      const int4 v2 = vC[l * kH + tc], w2 = wC[l * kH + tc];
+      const int2 vs = sum(v2), vd = dif(v2), ws = sum(w2), wd = dif(w2);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int4 v = vR[l * kT + tr + 16 * e], w = wR[l * kT + tr + 16 * e];
+        product(e, v, sum(v), w2, wd, ws);
+        product(e, w, sum(w), v2, vd, vs);
       }
+    }
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int4 v = vR[l * kT + tr + 16 * q], w = wR[l * kT + tr + 16 * q];
-#pragma unroll
-        for (int c = 0; c < 2; ++c) {
-          const int e = q * 2 + c;
-          mac(rh[e], rc[e], v.x, v.y, w2[c].x, w2[c].y);
-          mac(rh[e], rc[e], v.z, v.w, w2[c].z, w2[c].w);
-          mac(rh[e], rc[e], w.x, w.y, v2[c].x, v2[c].y);
-          mac(rh[e], rc[e], w.z, w.w, v2[c].z, v2[c].w);
-          mac(ih[e], ic[e], v.z, v.w, w2[c].x, w2[c].y);
-          mac(ih[e], ic[e], -v.x, -v.y, w2[c].z, w2[c].w);
-          mac(ih[e], ic[e], w.z, w.w, v2[c].x, v2[c].y);
-          mac(ih[e], ic[e], -w.x, -w.y, v2[c].z, v2[c].w);
-        }
-      }
+    for (int e = 0; e < 4; ++e) {
+      rh[e] = sh[e] - rh[e];
+      rc[e] = sl[e] - rc[e];
+      ih[e] = sh[e] - ih[e];
+      ic[e] = sl[e] - ic[e];
     }
     scale = pow2(exw + exv - 2 * kQ + 56);
   }
   // the new entries, and the tile's largest exponent off the diagonal
-  zd a[8];
+  zd a[4];
   int f = 0;
+  const int c = C * kT + c0 + tc;
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int r = R * kT + tr + 16 * (e >> 1), c = C * kT + tc + 32 * (e & 1);
+  for (int e = 0; e < 4; ++e) {
+    const int r = R * kT + tr + 16 * e;
     a[e] = mk<double>(0.0, 0.0);
     if (r < n && c >= j1 && r >= c) {
       zd* p = A + (size_t)c * lda + r;
       a[e] = *p;
-      if (kb > 0) {  // the low sums carried into the high ones, rounded at 2^-54 of the largest product
+      if (reflectors) {  // the low sums carried into the high ones, rounded at 2^-54 of the largest product
         const long long hr = rh[e] + ((rc[e] + (1ll << 27)) >> 28), hi = ih[e] + ((ic[e] + (1ll << 27)) >> 28);
         a[e].re = fma(-(double)hr, scale, a[e].re);
         a[e].im = r == c ? 0.0 : fma(-(double)hi, scale, a[e].im);
@@ -549,13 +633,13 @@ __global__ void __launch_bounds__(512, 1) tri_update_kernel(zd* __restrict__ A, 
   }
   f = __reduce_max_sync(0xffffffffu, f);
   if ((tid & 31) == 0) atomicMax(&s_ext, f);
-  __syncthreads();
-  const int ex = group_ex(s_ext);
+  clu.sync();
+  const int ex = group_ex(max(s_ext, *clu.map_shared_rank(&s_ext, clu.block_rank() ^ 1)));
   const size_t t = (size_t)R * (R + 1) / 2 + C;
-  if (tid == 0) Aex[t] = ex;
+  if (tid == 0 && c0 == 0) Aex[t] = ex;
 #pragma unroll
-  for (int e = 0; e < 8; ++e)
-    Aq[t * kT * kT + (tc + 32 * (e & 1)) * kT + tr + 16 * (e >> 1)] = quantise(a[e], ex);
+  for (int e = 0; e < 4; ++e) Aq[t * kT * kT + (c0 + tc) * kT + tr + 16 * e] = quantise(a[e], ex);
+  clu.sync();  // the peer has read s_ext
 }
 
 // A(j,i) = conj(A(i,j)) for i < j (the upper triangle is the input, as ZHEEV 'U' reads it); real diagonal.
@@ -1009,7 +1093,7 @@ inline int bt_columns(int n, size_t* smem) {
 
 // The reduction's buffers in one scratch block.
 struct TriScratch {
-  zd *xw, *u, *tau, *dots, *g, *W, *P;
+  zd *xw, *u, *next, *tau, *dots, *g, *W, *P;
   double *sparts, *e, *d, *ds, *e2, *bounds;
   TriCol* col;
   int *Aex, *exv;
@@ -1029,9 +1113,10 @@ struct TriScratch {
     W = reinterpret_cast<zd*>(take((size_t)kNB * n * sizeof(zd)));
     xw = reinterpret_cast<zd*>(take(n * sizeof(zd)));
     u = reinterpret_cast<zd*>(take(n * sizeof(zd)));
+    next = reinterpret_cast<zd*>(take(n * sizeof(zd)));
     tau = reinterpret_cast<zd*>(take(n * sizeof(zd)));
     dots = reinterpret_cast<zd*>(take(nd * sizeof(zd)));
-    g = reinterpret_cast<zd*>(take(2 * kNB * sizeof(zd)));
+    g = reinterpret_cast<zd*>(take((size_t)(n + kDotRows - 1) / kDotRows * 2 * kNB * sizeof(zd)));
     col = reinterpret_cast<TriCol*>(take(sizeof(TriCol)));
     sparts = reinterpret_cast<double*>(take(nd * sizeof(double)));
     e = reinterpret_cast<double*>(take(n * sizeof(double)));
@@ -1047,8 +1132,8 @@ struct TriScratch {
 
 size_t dense_eig_scratch(int n) { return TriScratch(n, nullptr).bytes; }
 
-constexpr size_t kSymvSmem = sizeof(int4) * (kT * (kT + 1) + 2 * kT) + sizeof(long long) * 16 * kT;
-constexpr size_t kUpdateSmem = sizeof(int4) * 4 * kNB * kT;
+constexpr size_t kSymvSmem = sizeof(int4) * (kT * (kT + 1) + 2 * kT) + sizeof(int2) * 2 * kT;
+constexpr size_t kUpdateSmem = sizeof(int4) * 3 * kNB * kT;
 
 cudaError_t dense_eig_prepare() {
   cudaError_t err = raise_smem_limit(reinterpret_cast<const void*>(tri_symv_kernel), kSymvSmem);
@@ -1062,9 +1147,10 @@ static cudaError_t tridiagonalise(zd* A, int n, int lda, const TriScratch& t, cu
   if (err != cudaSuccess) return err;
   const int nT = tiles_of(n);
   int ndots = 0;
-  auto update = [&](int j1, int kb) {
-    const unsigned tiles = (unsigned)lower_tiles(nT - j1 / kT);
-    tri_update_kernel<<<tiles, 512, kUpdateSmem, s>>>(A, n, lda, j1, kb, t.tau, t.W, t.xw, t.dots, ndots, t.Aq, t.Aex);
+  auto update = [&](int j1, int reflectors) {
+    const unsigned ctas = 2 * (unsigned)lower_tiles(nT - j1 / kT);
+    tri_update_kernel<<<ctas, 512, kUpdateSmem, s>>>(A, n, lda, j1, reflectors, t.tau, t.W, t.xw, t.dots, ndots, t.Aq,
+                                                     t.Aex);
     ++g_launch_count;
   };
   cudaLaunchAttribute early = {};
@@ -1086,15 +1172,17 @@ static cudaError_t tridiagonalise(zd* A, int n, int lda, const TriScratch& t, cu
   for (int j = 0; j < n; ++j) {
     const bool last = j + 1 == n;  // the last column has a diagonal entry only
     const unsigned tiles = last ? 0 : (unsigned)lower_tiles(nT - (j + 1) / kT);
-    err = launch(tri_symv_kernel, tiles + 1 + (last ? 0 : i), 256, kSymvSmem, A, n, lda, j, i, t.W, t.u, t.xw, t.dots,
-                 t.sparts, ndots, t.Aq, t.Aex, t.col, t.tau, t.e, t.g, t.P);
+    const int nch = (n - j - 1 + kDotRows - 1) / kDotRows;
+    const int nnext = i + 1 < kNB ? (n - j - 1 + kNextRows - 1) / kNextRows : 0;  // a panel's last column has no next
+    err = launch(tri_symv_kernel, tiles + 1 + (unsigned)(i * nch + nnext), 256, kSymvSmem, A, n, lda, j, i, t.W, t.u, t.xw, t.dots,
+                 t.sparts, ndots, t.Aq, t.Aex, t.col, t.tau, t.e, t.g, nch, t.next, nnext, t.P);
     if (err != cudaSuccess || last) break;
     ndots = (n - j - 1 + kRows - 1) / kRows;
-    err = launch(tri_x_kernel, (unsigned)ndots, 16 * (kRows + 2), 0, A, n, lda, j, i, i + 1 < kNB ? 1 : 0, t.W, t.P,
-                 t.col, t.g, t.u, t.xw, t.dots, t.sparts);
+    err = launch(tri_x_kernel, (unsigned)ndots, 16 * (kRows + 2), 0, A, n, lda, j, i, nnext ? t.next : (const zd*)nullptr, t.W, t.P,
+                 t.col, t.g, nch, t.u, t.xw, t.dots, t.sparts);
     if (err != cudaSuccess) break;
     if (++i == kNB) {
-      update(j + 1, kNB);
+      update(j + 1, 1);
       i = 0;
     }
   }
