@@ -42,3 +42,11 @@ def test_operator_matches_the_oracle(built, ngrid, fft):
     # the transforms' rounding is a few log2(P) ulp of the column's norm, the bands 1e-13 relative
     assert np.linalg.norm(Y - ref) <= 1e-12 * np.linalg.norm(ref)
     ctx.close()
+
+
+# every pruned first factor (2, 4, 8, 10, 16), with coprime second factors and with twiddles, on meshes of half the length
+# and shorter, and twiddles without pruning
+@pytest.mark.parametrize("ngrid", [(5, 1, 1), (18, 3, 1), (15, 4, 1), (20, 6, 1), (5, 5, 5), (4, 4, 10), (3, 50, 1),
+                                   (3, 49, 1), (100, 2, 1), (64, 5, 1), (13, 4, 3)])
+def test_pruned_and_twiddled_factors(built, ngrid):
+    test_operator_matches_the_oracle(built, ngrid, True)

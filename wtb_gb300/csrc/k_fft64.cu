@@ -9,10 +9,12 @@
 // design counts FP64 instructions and nothing else; index arithmetic, shared memory and barriers are cheap beside
 // them.  Each length P = R1 R2 with coprime R1, R2 <= 16 runs as a Good-Thomas (prime-factor) transform: element
 // (R2 a + R1 b) mod P is slot (a, b), an R1-point DFT over a and an R2-point DFT over b give X[k] with k = k1 mod R1,
-// k2 mod R2 in slot (k1, k2), with no twiddle factors at all.  The frequencies stay in that order; the spectrum is
-// stored in it.  The lengths come from the table in plan_length (15 x 8 = 120 for 60 points: 17.8 FP64 instructions a
-// point against 21 for the radix-2 128).  At 60 x 60 a column takes about 0.83 M FP64 instructions where the product
-// takes 26 M.
+// k2 mod R2 in slot (k1, k2), with no twiddle factors at all; other factors run with twiddles between them (96 = 8 x 12
+// for 48 points).  The frequencies stay in that order; the spectrum is stored in it.  Half of a transform's input is
+// zero and half of its output unused: where the first factor is 2, 4, 8, 10 or 16 and the mesh at most P / 2 long, of
+// the two elements that its first radix-2 stage would add, one is always zero, whatever the second factor's index, so
+// that stage takes sign changes only (and its inverse one addition of two).  At 60 x 60 a column takes about 0.78 M
+// FP64 instructions where the product takes 26 M.
 //
 // One CTA per complex column.  The mesh is taken as m1 x m2 x m3 with unit dimensions dropped (2D: m2 = 1):
 //   A. rows: DFT over the innermost dimension, m1 m2 rows of P3 slots in shared memory;
@@ -20,12 +22,14 @@
 //      times S, inverse over dimension 1, over dimension 2; the m1 x m2 results on the mesh go back to the rows;
 //   C. inverse rows; the m3 results on the mesh go to T.
 // The second factor of dimension 1, the product with S and the inverse's first factor stay in registers.
-// Measured per 16-column application: 3.04 ms at 48 x 45, w = 12 (2,304 columns of 0.61 M FP64 instructions: 73 % of
-// the FP64 pipe's issue rate; the product 37.3 ms), 4.48 ms at 11^3, w = 16 (the product 24.5 ms), 0.40 ms at 30 x 30,
-// w = 8 (3.9 ms).
+// Measured per 16-column application: 2.45 ms at 48 x 45, w = 12 (2,304 columns of 0.49 M FP64 instructions: 93 % of
+// the FP64 pipe's issue rate; without the pruned stages and 96 points 3.04 ms of 0.61 M; the product 37.3 ms), 4.20 ms
+// at 11^3, w = 16 (4.48 and 24.5 ms).
 #include "wtb_internal.h"
 
 #include <algorithm>
+#include <numeric>
+#include <vector>
 
 namespace wtb {
 namespace {
@@ -235,6 +239,136 @@ __device__ __forceinline__ void any_dft(int R, const L& load, const St& store) {
   }
 }
 
+__device__ __forceinline__ d2 neg_if(d2 a, bool neg) {  // on the sign bits: no FP64 instruction
+  const int f = neg ? (int)0x80000000 : 0;
+  return D(__hiloint2double(__double2hiint(a.x) ^ f, __double2loint(a.x)),
+           __hiloint2double(__double2hiint(a.y) ^ f, __double2loint(a.y)));
+}
+
+// times exp(-2 pi i a / R), R = 4, 8, 16
+template <int R>
+__device__ __forceinline__ d2 tw_const(d2 x, int a) {
+  constexpr double C = 0.92387953251128675613, S = 0.38268343236508977173, Q = 0.70710678118654752440;
+  switch (a * (16 / R)) {  // compile-time
+    case 0: return x;
+    case 1: return tw(x, C, S);
+    case 2: return D(Q * (x.x + x.y), Q * (x.y - x.x));
+    case 3: return tw(x, S, C);
+    case 4: return mi(x);
+    case 5: return tw(x, -S, C);
+    case 6: return D(Q * (x.y - x.x), -Q * (x.x + x.y));
+    default: return tw(x, -C, S);
+  }
+}
+
+// The first factor R = 2 H of a transform of which only one element of every pair (a, a + H) is on the mesh (the pair is
+// P / 2 apart, the mesh at most P / 2 long): the first radix-2 stage takes no additions.  from(a, &neg): the pair's
+// element on the mesh, neg if it is the second.  to(m, X[m]).
+template <int R, class L, class St>
+__device__ __forceinline__ void half_in(const L& from, const St& to) {
+  constexpr int H = R / 2;
+  d2 e[H], o[H];
+#pragma unroll
+  for (int t = 0; t < H; ++t) {
+    // R = 10 = 2 * 5 by the prime-factor map (e, o over t of the elements 2 t mod 10), else by twiddles
+    const int a = R == 10 ? 2 * t % H : t;
+    bool neg;
+    e[t] = from(a, &neg);
+    o[t] = neg_if(e[t], R == 10 ? neg != (2 * t >= H) : neg);
+    if constexpr (R != 10) o[t] = tw_const<R>(o[t], t);
+  }
+  if constexpr (H > 1) {
+    dft<H>(e);
+    dft<H>(o);
+  }
+#pragma unroll
+  for (int k = 0; k < H; ++k) {
+    if constexpr (R == 10) {  // X[k], k = 0 or 1 mod 2 and k = t mod 5
+      to(k % 2 ? k + 5 : k, e[k]);
+      to(k % 2 ? k : k + 5, o[k]);
+    } else {
+      to(2 * k, e[k]);
+      to(2 * k + 1, o[k]);
+    }
+  }
+}
+// Its inverse: from(m) = X[m], of every pair the element on the mesh.  to(a, &, value, value if it is the second).
+template <int R, class L, class St>
+__device__ __forceinline__ void half_out(const L& from, const St& to) {
+  constexpr int H = R / 2;
+  d2 e[H], o[H];
+#pragma unroll
+  for (int k = 0; k < H; ++k) {
+    e[k] = swp(from(R == 10 ? (k % 2 ? k + 5 : k) : 2 * k));
+    o[k] = swp(from(R == 10 ? (k % 2 ? k : k + 5) : 2 * k + 1));
+  }
+  if constexpr (H > 1) {
+    dft<H>(e);
+    dft<H>(o);
+  }
+#pragma unroll
+  for (int t = 0; t < H; ++t) {
+    const int a = R == 10 ? 2 * t % H : t;
+    if constexpr (R != 10) o[t] = tw_const<R>(o[t], t);
+    to(a, [&](bool neg) { return swp(add(e[t], neg_if(o[t], R == 10 ? neg != (2 * t >= H) : neg))); });
+  }
+}
+
+// The first factor of a forward transform from the mesh, put(a, X): element a is at l = idx(a) < P, of which l < n are
+// on the mesh (get(l)), the others zero.
+template <class I, class L, class St>
+__device__ __forceinline__ void mesh_in(int R, bool half, int P, int n, const I& idx, const L& get, const St& put) {
+  if (!half) {
+    any_dft<false>(
+        R,
+        [&](int a) {
+          const int l = idx(a);
+          return l < n ? get(l) : D(0.0, 0.0);
+        },
+        put);
+    return;
+  }
+  const int Q = P / 2;
+  auto from = [&](int a, bool* neg) {
+    int l = idx(a);
+    *neg = l >= Q;
+    l -= *neg ? Q : 0;
+    return l < n ? get(l) : D(0.0, 0.0);
+  };
+  switch (R) {
+    case 2: half_in<2>(from, put); break;
+    case 4: half_in<4>(from, put); break;
+    case 8: half_in<8>(from, put); break;
+    case 10: half_in<10>(from, put); break;
+    default: half_in<16>(from, put); break;
+  }
+}
+// The first factor of an inverse transform, last to run: get(a), put(l, x) for the elements on the mesh.
+template <class I, class L, class St>
+__device__ __forceinline__ void mesh_out(int R, bool half, int P, int n, const I& idx, const L& get, const St& put) {
+  if (!half) {
+    any_dft<true>(R, get, [&](int a, d2 v) {
+      const int l = idx(a);
+      if (l < n) put(l, v);
+    });
+    return;
+  }
+  const int Q = P / 2;
+  auto to = [&](int a, const auto& value) {
+    int l = idx(a);
+    const bool neg = l >= Q;
+    l -= neg ? Q : 0;
+    if (l < n) put(l, value(neg));
+  };
+  switch (R) {
+    case 2: half_out<2>(get, to); break;
+    case 4: half_out<4>(get, to); break;
+    case 8: half_out<8>(get, to); break;
+    case 10: half_out<10>(get, to); break;
+    default: half_out<16>(get, to); break;
+  }
+}
+
 // R-point DFT, product with the spectrum values sp(m), inverse R-point DFT
 template <int R, class L, class Sp, class St>
 __device__ __forceinline__ void one_mul(const L& load, const Sp& sp, const St& store) {
@@ -269,8 +403,9 @@ __device__ __forceinline__ void any_mul(int R, const L& load, const Sp& sp, cons
   }
 }
 
-__device__ __forceinline__ int slot_of(int a, int b, int R1, int R2, int P) {
-  const int t = R2 * a + R1 * b;
+// slot (a, b) of a transform with the strides sa, sb of its factors
+__device__ __forceinline__ int slot_of(int a, int b, int sa, int sb, int P) {
+  const int t = sa * a + sb * b;
   return t < P ? t : t - P;
 }
 
@@ -280,24 +415,44 @@ __global__ void __launch_bounds__(256) fft64_conv_kernel(Fft64Plan pl, const dou
   const int m1 = pl.m[0], m2 = pl.m[1], m3 = pl.m[2], nrow = m1 * m2;
   const int P1 = pl.P[0], P2 = pl.P[1], P3 = pl.P[2];
   const int A1 = pl.R1[0], B1 = pl.R2[0], A2 = pl.R1[1], B2 = pl.R2[1], A3 = pl.R1[2], B3 = pl.R2[2];
+  const int C1 = pl.ct[0] ? 1 : A1, C2 = pl.ct[1] ? 1 : A2, C3 = pl.ct[2] ? 1 : A3;  // the second factors' strides
   d2* Sb = reinterpret_cast<d2*>(smem_raw);  // [nrow][P3]
   d2* G = Sb + nrow * P3;                    // [batch][P1][P2]
+  d2* tw1 = G + pl.batch * P1 * P2;          // the twiddle tables of the dimensions that have one
+  d2* tw2 = tw1 + (pl.ct[0] ? P1 : 0);
+  d2* tw3 = tw2 + (pl.ct[1] ? P2 : 0);
   const int tid = threadIdx.x, nt = blockDim.x, q = blockIdx.x;
+  {
+    const d2* table = spec + (size_t)P1 * P2 * P3;
+    if (pl.ct[0])
+      for (int i = tid; i < P1; i += nt) tw1[i] = table[i];
+    if (pl.ct[1])
+      for (int i = tid; i < P2; i += nt) tw2[i] = table[P1 + i];
+    if (pl.ct[2])
+      for (int i = tid; i < P3; i += nt) tw3[i] = table[P1 + P2 + i];
+    if (pl.ct[0] || pl.ct[1] || pl.ct[2]) __syncthreads();
+  }
+  auto fwd = [](const d2* t, bool ct, int i, d2 v) {
+    if (!ct) return v;
+    const d2 w = t[i];
+    return tw(v, w.x, w.y);
+  };
+  auto inv = [](const d2* t, bool ct, int i, d2 v) {
+    if (!ct) return v;
+    const d2 w = t[i];
+    return D(fma(-w.y, v.y, w.x * v.x), fma(w.y, v.x, w.x * v.y));
+  };
   const double* zre = Z + (size_t)(2 * q) * ldz;
   const double* zim = zre + ldz;
-  const d2 zero = D(0.0, 0.0);
   // A. rows: over a (from global memory), then over b
   for (int it = tid; it < nrow * B3; it += nt) {
     const int b = it % B3, r = it / B3;
     d2* row = Sb + r * P3;
     const double *pr = zre + r * m3, *pi = zim + r * m3;
-    any_dft<false>(
-        A3,
-        [&](int a) {
-          const int l = slot_of(a, b, A3, B3, P3);
-          return l < m3 ? D(pr[l], pi[l]) : zero;
-        },
-        [&](int a, d2 v) { row[slot_of(a, b, A3, B3, P3)] = v; });
+    mesh_in(
+        A3, pl.half[2], P3, m3, [&](int a) { return slot_of(a, b, B3, C3, P3); },
+        [&](int l) { return D(pr[l], pi[l]); },
+        [&](int a, d2 v) { row[slot_of(a, b, B3, C3, P3)] = fwd(tw3, pl.ct[2], a * b, v); });
   }
   __syncthreads();
   if (B3 > 1) {
@@ -305,8 +460,8 @@ __global__ void __launch_bounds__(256) fft64_conv_kernel(Fft64Plan pl, const dou
       const int a = it % A3;
       d2* row = Sb + (it / A3) * P3;
       any_dft<false>(
-          B3, [&](int b) { return row[slot_of(a, b, A3, B3, P3)]; },
-          [&](int b, d2 v) { row[slot_of(a, b, A3, B3, P3)] = v; });
+          B3, [&](int b) { return row[slot_of(a, b, B3, C3, P3)]; },
+          [&](int b, d2 v) { row[slot_of(a, b, B3, C3, P3)] = v; });
     }
     __syncthreads();
   }
@@ -318,13 +473,10 @@ __global__ void __launch_bounds__(256) fft64_conv_kernel(Fft64Plan pl, const dou
       for (int it = tid; it < np * m1 * B2; it += nt) {
         const int p = it % np, t = it / np, b = t % B2, i = t / B2;
         d2* row = G + p * PP + i * P2;
-        any_dft<false>(
-            A2,
-            [&](int a) {
-              const int j = slot_of(a, b, A2, B2, P2);
-              return j < m2 ? Sb[(i * m2 + j) * P3 + w0 + p] : zero;
-            },
-            [&](int a, d2 v) { row[slot_of(a, b, A2, B2, P2)] = v; });
+        mesh_in(
+            A2, pl.half[1], P2, m2, [&](int a) { return slot_of(a, b, B2, C2, P2); },
+            [&](int j) { return Sb[(i * m2 + j) * P3 + w0 + p]; },
+            [&](int a, d2 v) { row[slot_of(a, b, B2, C2, P2)] = fwd(tw2, pl.ct[1], a * b, v); });
       }
       __syncthreads();
       if (B2 > 1) {
@@ -332,25 +484,23 @@ __global__ void __launch_bounds__(256) fft64_conv_kernel(Fft64Plan pl, const dou
           const int p = it % np, t = it / np, a = t % A2, i = t / A2;
           d2* row = G + p * PP + i * P2;
           any_dft<false>(
-              B2, [&](int b) { return row[slot_of(a, b, A2, B2, P2)]; },
-              [&](int b, d2 v) { row[slot_of(a, b, A2, B2, P2)] = v; });
+              B2, [&](int b) { return row[slot_of(a, b, B2, C2, P2)]; },
+              [&](int b, d2 v) { row[slot_of(a, b, B2, C2, P2)] = v; });
         }
         __syncthreads();
       }
     }
     const bool two = P2 > 1;
     if (B1 > 1) {
-      // columns: over a, from the mesh rows (the others are zero)
+      // columns: over a, from the mesh rows (the others are zero).  With P2 > 1 the mesh elements of an item are among
+      // its own slots in G (of a pair's two, both are slots of the same b)
       for (int it = tid; it < np * P2 * B1; it += nt) {
         const int p = it % np, t = it / np, v = t % P2, b = t / P2;
         d2* col = G + p * PP + v;
-        any_dft<false>(
-            A1,
-            [&](int a) {
-              const int i = slot_of(a, b, A1, B1, P1);
-              return i < m1 ? (two ? col[i * P2] : Sb[i * P3 + w0 + p]) : zero;
-            },
-            [&](int a, d2 x) { col[slot_of(a, b, A1, B1, P1) * P2] = x; });
+        mesh_in(
+            A1, pl.half[0], P1, m1, [&](int a) { return slot_of(a, b, B1, C1, P1); },
+            [&](int i) { return two ? col[i * P2] : Sb[i * P3 + w0 + p]; },
+            [&](int a, d2 x) { col[slot_of(a, b, B1, C1, P1) * P2] = fwd(tw1, pl.ct[0], a * b, x); });
       }
       __syncthreads();
       // over b, times the spectrum, inverse over b
@@ -359,25 +509,23 @@ __global__ void __launch_bounds__(256) fft64_conv_kernel(Fft64Plan pl, const dou
         d2* col = G + p * PP + v;
         const d2* sp = spec + (size_t)v * P3 + w0 + p;
         any_mul(
-            B1, [&](int b) { return col[slot_of(a, b, A1, B1, P1) * P2]; },
-            [&](int b) { return sp[(size_t)slot_of(a, b, A1, B1, P1) * P2 * P3]; },
-            [&](int b, d2 x) { col[slot_of(a, b, A1, B1, P1) * P2] = x; });
+            B1, [&](int b) { return col[slot_of(a, b, B1, C1, P1) * P2]; },
+            [&](int b) { return sp[(size_t)slot_of(a, b, B1, C1, P1) * P2 * P3]; },
+            [&](int b, d2 x) { col[slot_of(a, b, B1, C1, P1) * P2] = x; });
       }
       __syncthreads();
       // inverse over a; the mesh rows stay
       for (int it = tid; it < np * P2 * B1; it += nt) {
         const int p = it % np, t = it / np, v = t % P2, b = t / P2;
         d2* col = G + p * PP + v;
-        any_dft<true>(
-            A1, [&](int a) { return col[slot_of(a, b, A1, B1, P1) * P2]; },
-            [&](int a, d2 x) {
-              const int i = slot_of(a, b, A1, B1, P1);
-              if (i < m1) {
-                if (two)
-                  col[i * P2] = x;
-                else
-                  Sb[i * P3 + w0 + p] = x;
-              }
+        mesh_out(
+            A1, pl.half[0], P1, m1, [&](int a) { return slot_of(a, b, B1, C1, P1); },
+            [&](int a) { return inv(tw1, pl.ct[0], a * b, col[slot_of(a, b, B1, C1, P1) * P2]); },
+            [&](int i, d2 x) {
+              if (two)
+                col[i * P2] = x;
+              else
+                Sb[i * P3 + w0 + p] = x;
             });
       }
       __syncthreads();
@@ -387,7 +535,7 @@ __global__ void __launch_bounds__(256) fft64_conv_kernel(Fft64Plan pl, const dou
         d2* col = G + p * PP + v;
         const d2* sp = spec + (size_t)v * P3 + w0 + p;
         any_mul(
-            A1, [&](int i) { return i < m1 ? (two ? col[i * P2] : Sb[i * P3 + w0 + p]) : zero; },
+            A1, [&](int i) { return i < m1 ? (two ? col[i * P2] : Sb[i * P3 + w0 + p]) : D(0.0, 0.0); },
             [&](int i) { return sp[(size_t)i * P2 * P3]; },
             [&](int i, d2 x) {
               if (i < m1) {
@@ -406,20 +554,18 @@ __global__ void __launch_bounds__(256) fft64_conv_kernel(Fft64Plan pl, const dou
           const int p = it % np, t = it / np, a = t % A2, i = t / A2;
           d2* row = G + p * PP + i * P2;
           any_dft<true>(
-              B2, [&](int b) { return row[slot_of(a, b, A2, B2, P2)]; },
-              [&](int b, d2 v) { row[slot_of(a, b, A2, B2, P2)] = v; });
+              B2, [&](int b) { return row[slot_of(a, b, B2, C2, P2)]; },
+              [&](int b, d2 v) { row[slot_of(a, b, B2, C2, P2)] = v; });
         }
         __syncthreads();
       }
       for (int it = tid; it < np * m1 * B2; it += nt) {
         const int p = it % np, t = it / np, b = t % B2, i = t / B2;
         const d2* row = G + p * PP + i * P2;
-        any_dft<true>(
-            A2, [&](int a) { return row[slot_of(a, b, A2, B2, P2)]; },
-            [&](int a, d2 v) {
-              const int j = slot_of(a, b, A2, B2, P2);
-              if (j < m2) Sb[(i * m2 + j) * P3 + w0 + p] = v;
-            });
+        mesh_out(
+            A2, pl.half[1], P2, m2, [&](int a) { return slot_of(a, b, B2, C2, P2); },
+            [&](int a) { return inv(tw2, pl.ct[1], a * b, row[slot_of(a, b, B2, C2, P2)]); },
+            [&](int j, d2 v) { Sb[(i * m2 + j) * P3 + w0 + p] = v; });
       }
       __syncthreads();
     }
@@ -430,8 +576,8 @@ __global__ void __launch_bounds__(256) fft64_conv_kernel(Fft64Plan pl, const dou
       const int a = it % A3;
       d2* row = Sb + (it / A3) * P3;
       any_dft<true>(
-          B3, [&](int b) { return row[slot_of(a, b, A3, B3, P3)]; },
-          [&](int b, d2 v) { row[slot_of(a, b, A3, B3, P3)] = v; });
+          B3, [&](int b) { return row[slot_of(a, b, B3, C3, P3)]; },
+          [&](int b, d2 v) { row[slot_of(a, b, B3, C3, P3)] = v; });
     }
     __syncthreads();
   }
@@ -439,35 +585,36 @@ __global__ void __launch_bounds__(256) fft64_conv_kernel(Fft64Plan pl, const dou
     const int b = it % B3, r = it / B3;
     const d2* row = Sb + r * P3;
     double* out = T + (size_t)r * m3 * ldt + 2 * q;
-    any_dft<true>(
-        A3, [&](int a) { return row[slot_of(a, b, A3, B3, P3)]; },
-        [&](int a, d2 v) {
-          const int l = slot_of(a, b, A3, B3, P3);
-          if (l < m3) *reinterpret_cast<d2*>(out + (size_t)l * ldt) = v;
-        });
+    mesh_out(
+        A3, pl.half[2], P3, m3, [&](int a) { return slot_of(a, b, B3, C3, P3); },
+        [&](int a) { return inv(tw3, pl.ct[2], a * b, row[slot_of(a, b, B3, C3, P3)]); },
+        [&](int l, d2 v) { *reinterpret_cast<d2*>(out + (size_t)l * ldt) = v; });
   }
 }
 
 // out[o][slot][i] = scale sum_l in[o][l][i] W_P^(f(slot) (l - (n - 1))), l < 2 n - 1, f(slot) the frequency in the
-// slot (k1 mod R1, k2 mod R2): one dimension of the spectrum, W_P^m from a shared table.  first: in is the real stencil.
+// slot: one dimension of the spectrum, W_P^m from a shared table, which also goes to table (the twiddle factors of a
+// transform with ct).  first: in is the real stencil.
 __global__ void __launch_bounds__(128) fft64_spec_kernel(const double* __restrict__ in, int first, int outer, int inner,
-                                                         int n, int P, int R1, int R2, double scale,
-                                                         d2* __restrict__ out) {
+                                                         int n, int P, int R1, int R2, int ct, double scale,
+                                                         d2* __restrict__ out, d2* __restrict__ table) {
   __shared__ double wr[256], wi[256];
   for (int m = threadIdx.x; m < P; m += blockDim.x) {
     double sn, cs;
     sincospi(2.0 * m / P, &sn, &cs);
     wr[m] = cs;
     wi[m] = -sn;
+    if (blockIdx.x == 0) table[m] = D(cs, sn);
   }
   __syncthreads();
   const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= (long)outer * P * inner) return;
   const int i = (int)(e % inner), slot = (int)((e / inner) % P);
   const long o = e / ((long)inner * P);
-  // the frequency k with slot = (R2 k1 + R1 k2) mod P, k1 = k mod R1, k2 = k mod R2: the inverse of k -> slot
-  int f = 0;
-  for (int k = 0; k < P; ++k)
+  // slot = (R2 k1 + R1 k2) mod P of the frequency k, k1 = k mod R1, k2 = k mod R2 (inverted by search), or with ct
+  // R2 k1 + k2 of k = k1 + R1 k2
+  int f = ct ? slot / R2 + R1 * (slot % R2) : 0;
+  for (int k = 0; k < P && !ct; ++k)
     if ((R2 * (k % R1) + R1 * (k % R2)) % P == slot) f = k;
   const int L = 2 * n - 1;
   double re = 0.0, im = 0.0;
@@ -507,76 +654,149 @@ int dft_cost(int R) {
   }
 }
 
-// The cheapest P = R1 R2 >= 2 n - 1 with coprime factors (an R of one factor only: R2 = 1)
-bool plan_length(int n, int* P, int* R1, int* R2, long* cost) {
-  static const int kR[] = {1, 2, 3, 4, 5, 7, 8, 9, 10, 12, 15, 16};
-  auto gcd = [](int a, int b) {
-    while (b) {
-      const int t = a % b;
-      a = b;
-      b = t;
-    }
-    return a;
-  };
-  if (n == 1) {
-    *P = *R1 = *R2 = 1;
-    *cost = 0;
-    return true;
+// The time of a plan in FP64 instructions at the pipe's rate: 0.556 of its instructions and this for every R-point DFT.
+// Fitted (root mean square error 4.5 %) to the measured times of 717 plans of ten meshes, 7^3 to 48 x 45: large powers
+// of two keep the pipe busiest, 3, 5, 10 and 15 points least.
+double dft_time(int R) {
+  switch (R) {
+    case 1: return 0.0;
+    case 2: return 4.5;
+    case 3: return 11.4;
+    case 4: return 11.9;
+    case 5: return 25.4;
+    case 7: return 40.8;
+    case 8: return 29.6;
+    case 9: return 54.2;
+    case 10: return 62.2;
+    case 12: return 56.6;
+    case 15: return 121.8;
+    default: return 93.0;
   }
-  long best = -1;
+}
+constexpr double kInstrTime = 0.556;
+
+// A transform of one dimension: its length P = R1 R2, the kinds of its factors, and the FP64 instructions and the time
+// of a forward and an inverse.
+struct Length {
+  int P = 0, R1 = 1, R2 = 1, half = 0, ct = 0;
+  double cost = 0.0, time = 0.0;
+};
+
+// Lengths P >= 2 n - 1 for n mesh points, none of them both longer and slower than another.  Coprime factors need no
+// twiddles; others (ct) do, P complex products each way.  half: the mesh takes at most half of P and R1 has a half
+// form.
+std::vector<Length> lengths(int n) {
+  static const int kR[] = {16, 15, 12, 10, 9, 8, 7, 5, 4, 3, 2, 1};  // the larger factor first where two plans tie
+  std::vector<Length> best;
+  if (n == 1) {
+    best.resize(1);
+    best[0].P = 1;
+    return best;
+  }
+  Length by_p[257];  // the cheapest of each length
   for (int a : kR)
     for (int b : kR) {
-      if (b > a || a * b < 2 * n - 1 || gcd(a, b) != 1) continue;
-      const long c = (long)b * dft_cost(a) + (long)a * dft_cost(b);
-      if (best < 0 || c < best || (c == best && a * b < *P)) {
-        best = c;
-        *P = a * b;
-        *R1 = a;
-        *R2 = b;
+      const int P = a * b;
+      // one factor alone makes one item a row: up to 5 points only (16 alone on an 8 x 8 mesh cost
+      // its full run 4.25 instead of 4.03 ms)
+      if (a == 1 || (b == 1 && a > 5) || P < 2 * n - 1) continue;
+      const bool ct = b > 1 && std::gcd(a, b) != 1;
+      long in = dft_cost(a), out = in;
+      const bool half = b > 1 && 2 * n <= P && (a == 2 || a == 4 || a == 8 || a == 10 || a == 16);
+      if (half) {  // two DFTs of R / 2, the twiddles between, and one addition of two per pair on the way out
+        static const int kTw[] = {0, 0, 0, 0, 0, 0, 0, 0, 8, 0, 0, 0, 0, 0, 0, 0, 24};
+        in = 2 * dft_cost(a / 2) + kTw[a];
+        out = in + a;
       }
+      Length x;
+      x.P = P;
+      x.R1 = a;
+      x.R2 = b;
+      x.half = half ? 1 : 0;
+      x.ct = ct ? 1 : 0;
+      x.cost = (double)b * (in + out) + 2.0 * a * dft_cost(b) + (ct ? 8.0 * P : 0.0);
+      x.time = kInstrTime * x.cost + 2.0 * b * dft_time(a) + 2.0 * a * dft_time(b);
+      if (by_p[P].P == 0 || x.time < by_p[P].time) by_p[P] = x;
     }
-  *cost = best;
-  return best >= 0;
+  for (const Length& x : by_p)
+    if (x.P && (best.empty() || x.time < best.back().time)) best.push_back(x);
+  return best;
 }
 
-constexpr size_t kFft64Smem = 220 * 1024;  // dynamic shared memory of one CTA at most
+constexpr size_t kFft64Smem = 220 * 1024;   // dynamic shared memory of one CTA at most
+constexpr size_t kFft64Smem2 = 110 * 1024;  // of one of two CTAs an SM
+constexpr int kFft64Mesh = 120;             // mesh points of a dimension at most
 
-}  // namespace
-
-// The plan of an n1 x n2 x n3 mesh, or false where the transforms do not fit one CTA (the caller then multiplies by
-// the table).  *per_column: FP64 instructions of one complex column.
-bool fft64_plan(int n1, int n2, int n3, Fft64Plan* pl, double* per_column) {
-  const int n[3] = {n1, n2, n3};
-  int d[3], nd = 0;
-  for (int i = 0; i < 3; ++i) {
-    if (n[i] < 1) return false;
-    if (n[i] > 1) d[nd++] = n[i];
-  }
-  pl->m[0] = nd >= 2 ? d[0] : 1;
-  pl->m[1] = nd == 3 ? d[1] : 1;
-  pl->m[2] = nd >= 1 ? d[nd - 1] : 1;
-  long c[3];
+// Batches of planes and shared memory for the lengths in pl; false where they do not fit.
+bool fft64_batches(Fft64Plan* pl) {
+  size_t rows = sizeof(double2) * pl->m[0] * pl->m[1] * pl->P[2];
+  const size_t plane = sizeof(double2) * pl->P[0] * pl->P[1];
   for (int i = 0; i < 3; ++i)
-    if (!plan_length(pl->m[i], &pl->P[i], &pl->R1[i], &pl->R2[i], &c[i])) return false;
-  const size_t rows = sizeof(double2) * pl->m[0] * pl->m[1] * pl->P[2], plane = sizeof(double2) * pl->P[0] * pl->P[1];
+    if (pl->ct[i]) rows += sizeof(double2) * pl->P[i];
   // planes a batch: enough items for the CTA's 256 threads in the pass with the fewest (P1 P2 / 16 a plane), and no
   // more shared memory than leaves room for a second CTA where the rows alone do
   int batch = (int)std::max<long>(1, (256L * 16 + pl->P[0] * pl->P[1] - 1) / (pl->P[0] * pl->P[1]));
   batch = std::min(batch, pl->P[2]);
-  const size_t room = rows + plane <= 110 * 1024 ? 110 * 1024 : kFft64Smem;
+  const size_t room = rows + plane <= kFft64Smem2 ? kFft64Smem2 : kFft64Smem;
   while (batch > 1 && rows + batch * plane > room) --batch;
   if (rows + batch * plane > kFft64Smem) return false;
   // equal batches
   const int nb = (pl->P[2] + batch - 1) / batch;
   pl->batch = (pl->P[2] + nb - 1) / nb;
   pl->smem = rows + pl->batch * plane;
-  if (per_column)
-    *per_column = 2.0 * pl->m[0] * pl->m[1] * c[2] + pl->P[2] * (2.0 * pl->m[0] * c[1] + 2.0 * pl->P[1] * c[0]) +
-                  4.0 * pl->P[0] * pl->P[1] * pl->P[2];
   return true;
 }
 
-size_t fft64_spec_size(const Fft64Plan& pl) { return (size_t)pl.P[0] * pl.P[1] * pl.P[2]; }
+}  // namespace
+
+// The plan of an n1 x n2 x n3 mesh, or false where the transforms do not fit one CTA (the caller then multiplies by
+// the table).  *per_column: FP64 instructions of one complex column.  The lengths of the three dimensions are chosen
+// together (a longer one adds transforms to the others): the least time, plans that leave an SM one CTA counted half
+// as much again (its FP64 pipe idles between the passes).
+bool fft64_plan(int n1, int n2, int n3, Fft64Plan* pl, double* per_column) {
+  const int n[3] = {n1, n2, n3};
+  int d[3], nd = 0;
+  for (int i = 0; i < 3; ++i) {
+    if (n[i] < 1 || n[i] > kFft64Mesh) return false;
+    if (n[i] > 1) d[nd++] = n[i];
+  }
+  Fft64Plan t;
+  t.m[0] = nd >= 2 ? d[0] : 1;
+  t.m[1] = nd == 3 ? d[1] : 1;
+  t.m[2] = nd >= 1 ? d[nd - 1] : 1;
+  const std::vector<Length> L[3] = {lengths(t.m[0]), lengths(t.m[1]), lengths(t.m[2])};
+  double best = 0.0;
+  for (const Length& x : L[0])
+    for (const Length& y : L[1])
+      for (const Length& z : L[2]) {
+        const Length* l[3] = {&x, &y, &z};
+        for (int i = 0; i < 3; ++i) {
+          t.P[i] = l[i]->P;
+          t.R1[i] = l[i]->R1;
+          t.R2[i] = l[i]->R2;
+          t.half[i] = l[i]->half;
+          t.ct[i] = l[i]->ct;
+        }
+        auto column = [&](double Length::*what, double product) {
+          return (double)t.m[0] * t.m[1] * (z.*what) + z.P * ((double)t.m[0] * (y.*what) + (double)y.P * (x.*what)) +
+                 product * x.P * y.P * z.P;
+        };
+        double time = column(&Length::time, 4.0 * kInstrTime);
+        if ((best > 0.0 && time >= best) || !fft64_batches(&t)) continue;
+        if (t.smem > kFft64Smem2) time *= 1.5;
+        if (best == 0.0 || time < best) {
+          best = time;
+          *pl = t;
+          if (per_column) *per_column = column(&Length::cost, 4.0);
+        }
+      }
+  return best > 0.0;
+}
+
+// the spectrum, then the dimensions' twiddle tables
+size_t fft64_spec_size(const Fft64Plan& pl) {
+  return (size_t)pl.P[0] * pl.P[1] * pl.P[2] + pl.P[0] + pl.P[1] + pl.P[2];
+}
 
 size_t fft64_work_size(const Fft64Plan& pl) {
   return (size_t)(2 * pl.m[0] - 1) * (2 * pl.m[1] - 1 + pl.P[1]) * pl.P[2];
@@ -587,17 +807,20 @@ cudaError_t launch_fft64_spectrum(const Fft64Plan& pl, const double* stencil, zd
   d2* sp = reinterpret_cast<d2*>(spec);
   d2* wk = reinterpret_cast<d2*>(work);
   d2* wk2 = wk + (size_t)L1 * L2 * pl.P[2];
+  d2* table = sp + (size_t)pl.P[0] * pl.P[1] * pl.P[2];
   auto grid = [](long n) { return (unsigned)((n + 127) / 128); };
   // stencil [L1][L2][L3] -> [L1][L2][P3] -> [L1][P2][P3] -> spec [P1][P2][P3]
   fft64_spec_kernel<<<grid((long)L1 * L2 * pl.P[2]), 128, 0, s>>>(stencil, 1, L1 * L2, 1, pl.m[2], pl.P[2], pl.R1[2],
-                                                                  pl.R2[2], 1.0, wk);
+                                                                  pl.R2[2], pl.ct[2], 1.0, wk,
+                                                                  table + pl.P[0] + pl.P[1]);
   ++g_launch_count;
   fft64_spec_kernel<<<grid((long)L1 * pl.P[1] * pl.P[2]), 128, 0, s>>>(
-      reinterpret_cast<const double*>(wk), 0, L1, pl.P[2], pl.m[1], pl.P[1], pl.R1[1], pl.R2[1], 1.0, wk2);
+      reinterpret_cast<const double*>(wk), 0, L1, pl.P[2], pl.m[1], pl.P[1], pl.R1[1], pl.R2[1],
+      pl.ct[1], 1.0, wk2, table + pl.P[0]);
   ++g_launch_count;
   fft64_spec_kernel<<<grid((long)pl.P[0] * pl.P[1] * pl.P[2]), 128, 0, s>>>(
       reinterpret_cast<const double*>(wk2), 0, 1, pl.P[1] * pl.P[2], pl.m[0], pl.P[0], pl.R1[0], pl.R2[0],
-      1.0 / ((double)pl.P[0] * pl.P[1] * pl.P[2]), sp);
+      pl.ct[0], 1.0 / ((double)pl.P[0] * pl.P[1] * pl.P[2]), sp, table);
   ++g_launch_count;
   return cudaGetLastError();
 }

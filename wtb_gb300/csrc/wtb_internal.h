@@ -150,6 +150,7 @@ cudaError_t launch_fft_conv(const float* Z, int ldz, int npairs, int n1, int n2,
 // T[k][2q + (0, 1)] (row k at T + k ldt).
 struct Fft64Plan {
   int m[3] = {1, 1, 1}, P[3] = {1, 1, 1}, R1[3] = {1, 1, 1}, R2[3] = {1, 1, 1};
+  int half[3] = {0, 0, 0}, ct[3] = {0, 0, 0};  // pruned first factor; factors with twiddles
   int batch = 1;
   size_t smem = 0;
 };
