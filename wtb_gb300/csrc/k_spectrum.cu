@@ -95,30 +95,56 @@ __global__ void __launch_bounds__(256) osc_final_kernel(const double* __restrict
 // smef = CSHIFT + 10 * (sum_{i>=1} (E_i - E_{i-1})) / nrows  (fixed-order tree reduction)
 // Also records in smef[1] the end of the last row with a nonzero activity in any component: rows past it add
 // exactly zero to every Lorentzian sum (bsesolver leaves the rows past nev at zero).
-__global__ void __launch_bounds__(1024) avgsme_kernel(const double* __restrict__ Ws, int nrows, double sme,
-                                                      const double* __restrict__ f, int ncomp,
-                                                      double* __restrict__ smef) {
-  __shared__ double red[1024];
-  __shared__ int s_last;
-  if (threadIdx.x == 0) s_last = 0;
-  double acc = 0.0;
-  const int chunk = (nrows + blockDim.x - 1) / blockDim.x;
-  const int i0 = threadIdx.x * chunk;
-  int last = 0;
-  for (int i = max(i0, 1); i < min(nrows, i0 + chunk); ++i) acc = acc + Ws[i] - Ws[i - 1];
-  for (int i = i0; i < min(nrows, i0 + chunk); ++i)
-    for (int c = 0; c < ncomp; ++c)
-      if (f[(size_t)c * nrows + i] != 0.0) last = i + 1;
-  red[threadIdx.x] = acc;
+// Two kernels, since one CTA takes 0.2 ms to read 57,600 rows of six components: rows by CTA into
+// stats[block] = {sum, last}, then their sum.
+constexpr int kStatRows = 2048;
+__device__ __forceinline__ void block_sum_max(double* acc, int* last, double* red, int* s_last) {
+  if (threadIdx.x == 0) *s_last = 0;
+  red[threadIdx.x] = *acc;
   __syncthreads();
-  if (last) atomicMax(&s_last, last);
+  if (*last) atomicMax(s_last, *last);
   for (int off = blockDim.x / 2; off > 0; off >>= 1) {
     if (threadIdx.x < off) red[threadIdx.x] += red[threadIdx.x + off];
     __syncthreads();
   }
+  *acc = red[0];
+  *last = *s_last;
+}
+
+__global__ void __launch_bounds__(256) row_stats_kernel(const double* __restrict__ Ws, int nrows, int per,
+                                                        const double* __restrict__ f, int ncomp,
+                                                        double* __restrict__ stats) {
+  __shared__ double red[256];
+  __shared__ int s_last;
+  const int i0 = blockIdx.x * per, i1 = min(nrows, i0 + per);
+  double acc = 0.0;
+  int last = 0;
+  for (int i = i0 + threadIdx.x; i < i1; i += 256) {
+    if (i > 0) acc += Ws[i] - Ws[i - 1];
+    for (int c = 0; c < ncomp; ++c)
+      if (f[(size_t)c * nrows + i] != 0.0) last = i + 1;
+  }
+  block_sum_max(&acc, &last, red, &s_last);
   if (threadIdx.x == 0) {
-    smef[0] = 10.0 * (red[0] / (double)nrows) + sme;
-    smef[1] = (double)s_last;
+    stats[2 * blockIdx.x] = acc;
+    stats[2 * blockIdx.x + 1] = (double)last;
+  }
+}
+
+__global__ void __launch_bounds__(256) avgsme_kernel(const double* __restrict__ stats, int nblk, int nrows, double sme,
+                                                     double* __restrict__ smef) {
+  __shared__ double red[256];
+  __shared__ int s_last;
+  double acc = 0.0;
+  int last = 0;
+  for (int b = threadIdx.x; b < nblk; b += 256) {
+    acc += stats[2 * b];
+    last = max(last, (int)stats[2 * b + 1]);
+  }
+  block_sum_max(&acc, &last, red, &s_last);
+  if (threadIdx.x == 0) {
+    smef[0] = 10.0 * (acc / (double)nrows) + sme;
+    smef[1] = (double)last;
   }
 }
 
@@ -129,10 +155,22 @@ __device__ __forceinline__ double omega_of(double e0, double ef, int nesp, int j
   return e0 + ((ef - e0) * (double)j) / ((double)nesp - 1.0);
 }
 
+// 1 / x for finite x > 0 away from the ends of the range, within an ulp: the hardware's 20-bit approximation r and one
+// third-order Newton-Schulz (Chebyshev) step r (1 + e + e^2), e = 1 - x r, three FP64 instructions; a division takes
+// a dozen.  Elsewhere (zero, subnormal, infinity, NaN) the division.
+__device__ __forceinline__ double reciprocal(double x) {
+  if ((unsigned)__double2hiint(x) - 0x01000000u >= 0x7e000000u - 0x01000000u) return 1.0 / x;
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
+}
+
 // Partial Lorentzian sums of optdiel over one chunk of the rows, all NC components at once: the two
 // quotients (E - omega) / eaux and gamma / eaux do not depend on the component, so each (row, omega) pair
-// costs one FP64 division (1/eaux) instead of two per component, and the products f_c * quotient are the
-// reference's own.  A thread owns one photon energy; the chunk's rows pass through shared memory.
+// costs one reciprocal of eaux, and gamma multiplies the finished sums.  The FP64 pipe bounds the kernel: 18
+// instructions a pair of six components (27 with a division and the quotients formed apart): 57,600 rows x 1,000
+// energies 2.2 -> 1.76 ms.  A thread owns one photon energy; the chunk's rows pass through shared memory.
 // part[chunk][c][0: real, 1: imaginary][nesp].
 template <int NC>
 __global__ void __launch_bounds__(kLorOmega) lorentz_partial_kernel(const double* __restrict__ Ws, int nrows,
@@ -166,16 +204,13 @@ __global__ void __launch_bounds__(kLorOmega) lorentz_partial_kernel(const double
     if (j < nesp)
       for (int r = 0; r < nt; ++r) {
         const double ex = sW[r];
-        const double eaux = ((elux - ex) * (elux - ex)) + (smef * smef);
-        // one FP64 division per pair (the FP64 pipe bounds this kernel): the quotients as products with 1/eaux,
-        // within an ulp of the reference's two divisions
-        const double ie = 1.0 / eaux;
-        const double q1 = (ex - elux) * ie;
-        const double q2 = smef * ie;
+        const double d = ex - elux;
+        const double ie = reciprocal(d * d + smef * smef);
+        const double q1 = d * ie;
 #pragma unroll
         for (int c = 0; c < NC; ++c) {
           rp[c] += sf[c][r] * q1;
-          ip[c] += sf[c][r] * q2;
+          ip[c] += sf[c][r] * ie;
         }
       }
   }
@@ -184,7 +219,7 @@ __global__ void __launch_bounds__(kLorOmega) lorentz_partial_kernel(const double
   for (int c = 0; c < NC; ++c) {
     double* o = part + ((size_t)ch * NC + c) * 2 * nesp + j;
     o[0] = rp[c];
-    o[nesp] = ip[c];
+    o[nesp] = smef * ip[c];
   }
 }
 
@@ -318,35 +353,57 @@ __global__ void sp_records_kernel(const double* __restrict__ kpt, const int* __r
 }
 
 constexpr int kRankThreads = 256;
+constexpr int kRankRows = 2 * kRankThreads;  // rows a CTA, two a thread
 constexpr int kRankTile = 2048;
 
 // Bubblem (src/module_math.F90:287-308) is a bubble sort that swaps adjacent rows only when the upper key is
 // strictly greater: a stable ascending sort.  Row i therefore lands at
 //   rank(i) = #{j : key_j < key_i} + #{j < i : key_j == key_i}
 // (float comparisons, so -0 and +0 tie as in the reference).  Every count is exact whatever the order of
-// the additions; the keys pass through shared memory in tiles and blockIdx.y splits the j range.
+// the additions; the keys pass through shared memory in tiles and blockIdx.y splits the j range.  Rows j before all of
+// the CTA's count by <=, rows after by <, so that only the CTA's own need both and the order of i and j: 57,600 rows
+// 0.69 -> 0.37 ms.
 __global__ void __launch_bounds__(kRankThreads) stable_rank_kernel(const float* __restrict__ key, int n,
                                                                    int* __restrict__ rank) {
-  __shared__ float sk[kRankTile];
-  const int i = blockIdx.x * kRankThreads + threadIdx.x;
-  const float ki = i < n ? key[i] : 0.0f;
+  __shared__ __align__(16) float sk[kRankTile];
+  const int i0 = blockIdx.x * kRankRows, ia = i0 + threadIdx.x, ib = ia + kRankThreads;
+  const float ka = ia < n ? key[ia] : 0.0f, kb = ib < n ? key[ib] : 0.0f;
   const int per = (n + gridDim.y - 1) / gridDim.y;
   const int j0 = min(n, (int)blockIdx.y * per), j1 = min(n, j0 + per);
-  int cnt = 0;
-  for (int t0 = j0; t0 < j1; t0 += kRankTile) {
-    const int nt = min(kRankTile, j1 - t0);
-    __syncthreads();
-    for (int e = threadIdx.x; e < nt; e += kRankThreads) sk[e] = key[t0 + e];
-    __syncthreads();
-    if (i < n) {
-      const int lim = i - t0;  // tile rows below this bound come before row i
-      for (int r = 0; r < nt; ++r) {
-        const float kj = sk[r];
-        cnt += (kj < ki) | ((kj == ki) & (r < lim));
+  int ca = 0, cb = 0;
+  // counts(kj, j) over the rows from .. to - 1
+  auto scan = [&](int from, int to, auto counts) {
+    for (int t0 = from; t0 < to; t0 += kRankTile) {
+      const int nt = min(kRankTile, to - t0), n4 = nt & ~3;
+      __syncthreads();
+      for (int e = threadIdx.x; e < nt; e += kRankThreads) sk[e] = key[t0 + e];
+      __syncthreads();
+      int r = 0;
+#pragma unroll 4
+      for (; r < n4; r += 4) {
+        const float4 k = *reinterpret_cast<const float4*>(sk + r);
+        counts(k.x, t0 + r);
+        counts(k.y, t0 + r + 1);
+        counts(k.z, t0 + r + 2);
+        counts(k.w, t0 + r + 3);
       }
+      for (; r < nt; ++r) counts(sk[r], t0 + r);
     }
-  }
-  if (i < n && cnt) atomicAdd(&rank[i], cnt);
+  };
+  scan(j0, min(j1, i0), [&](float k, int) {
+    ca += k <= ka;
+    cb += k <= kb;
+  });
+  scan(max(j0, i0), min(j1, i0 + kRankRows), [&](float k, int j) {
+    ca += (k < ka) | ((k == ka) & (j < ia));
+    cb += (k < kb) | ((k == kb) & (j < ib));
+  });
+  scan(max(j0, i0 + kRankRows), j1, [&](float k, int) {
+    ca += k < ka;
+    cb += k < kb;
+  });
+  if (ia < n && ca) atomicAdd(&rank[ia], ca);
+  if (ib < n && cb) atomicAdd(&rank[ib], cb);
 }
 
 __global__ void permute_rows_kernel(const float* __restrict__ in, const int* __restrict__ rank, int n, int ncol,
@@ -432,7 +489,11 @@ cudaError_t launch_spectrum(const double* Ws, int nrows, const double* f, int nc
   if ((ncomp != 5 && ncomp != 6) || nrows < 1 || nesp < 2) return cudaErrorInvalidValue;
   if (partial_len < spectrum_partial_len(nrows, nesp, ncomp)) return cudaErrorInvalidValue;
   const int nchunk = lorentz_chunks(nrows, nesp);
-  avgsme_kernel<<<1, 1024, 0, s>>>(Ws, nrows, sme, f, ncomp, partial); ++g_launch_count;
+  // the statistics by block pass through the partial sums' room (at least 20 values)
+  const int room = (int)std::min<size_t>(1 << 20, (partial_len - 2) / 2);
+  const int nblk = std::min((nrows + kStatRows - 1) / kStatRows, room), per = (nrows + nblk - 1) / nblk;
+  row_stats_kernel<<<nblk, 256, 0, s>>>(Ws, nrows, per, f, ncomp, partial + 2); ++g_launch_count;
+  avgsme_kernel<<<1, 256, 0, s>>>(partial + 2, nblk, nrows, sme, partial); ++g_launch_count;
   const dim3 grid((nesp + kLorOmega - 1) / kLorOmega, nchunk);
   if (ncomp == 5)
     lorentz_partial_kernel<5><<<grid, kLorOmega, 0, s>>>(Ws, nrows, f, partial, e0, ef, nesp, partial + 2);
@@ -461,9 +522,10 @@ cudaError_t launch_sp_records(const double* kpt, const int* nocp, const double* 
   sp_records_kernel<<<(n + 255) / 256, 256, 0, s>>>(kpt, nocp, eig_win, hr, nk, nv, nc, f, rec, key); ++g_launch_count;
   cudaError_t e = cudaMemsetAsync(rank, 0, sizeof(int) * n, s);
   if (e != cudaSuccess) return e;
-  const int gx = (n + kRankThreads - 1) / kRankThreads;
-  // split the compared range so that a small sort still fills the GPU (at least one key tile per split)
-  const int gy = std::max(1, std::min((2 * 152 + gx - 1) / gx, (n + kRankTile - 1) / kRankTile));
+  const int gx = (n + kRankRows - 1) / kRankRows;
+  // split the compared range so that a small sort still fills the GPU (at least one key tile per split), and into
+  // CTAs enough, eight an SM, that the SMs finish together
+  const int gy = std::max(1, std::min((8 * 152 + gx - 1) / gx, (n + kRankTile - 1) / kRankTile));
   stable_rank_kernel<<<dim3(gx, gy), kRankThreads, 0, s>>>(key, n, rank); ++g_launch_count;
   e = cudaMemsetAsync(sorted, 0, sizeof(float) * 15 * n, s);
   if (e != cudaSuccess) return e;
