@@ -22,8 +22,8 @@
 //      times S, inverse over dimension 1, over dimension 2; the m1 x m2 results on the mesh go back to the rows;
 //   C. inverse rows; the m3 results on the mesh go to T.
 // The second factor of dimension 1, the product with S and the inverse's first factor stay in registers.
-// Measured per 16-column application: 2.45 ms at 48 x 45, w = 12 (2,304 columns of 0.49 M FP64 instructions: 93 % of
-// the FP64 pipe's issue rate; without the pruned stages and 96 points 3.04 ms of 0.61 M; the product 37.3 ms), 4.20 ms
+// Measured per 16-column application: 2.45 ms at 48 x 45, w = 12 (2,304 columns of 0.49 M FP64 instructions; the FP64
+// pipe busy 79 % of the cycles; without the pruned stages and 96 points 3.04 ms of 0.61 M; the product 37.3 ms), 4.20 ms
 // at 11^3, w = 16 (4.48 and 24.5 ms).
 #include "wtb_internal.h"
 
