@@ -692,8 +692,8 @@ __global__ void __launch_bounds__(1024) tri_finish_kernel(const zd* __restrict__
 // Number of eigenvalues of the scaled T below x: the sign changes of p_0 = 1, p_{i+1} = (d_i - x) p_i - e_{i-1}^2 p_{i-1}
 // (the leading minors; Givens' recurrence, each p_i the exact one of a T whose entries differ by a few ulp).  One
 // multiply-add of latency and three FP64 instructions a row, against a division's chain of 460 clocks and eleven
-// instructions for the ratios q_i = p_{i+1} / p_i (all eigenvalues at n = 2,304: 20 -> 6.9 ms).  T is scaled to entries of at most 1, so that the pair (p_i, p_{i-1})
-// can lose at most 53 bits a row and gain two: every eighth row rescales it by a power of two.  A zero counts as
+// instructions for the ratios q_i = p_{i+1} / p_i (all eigenvalues at n = 2,304: 20 -> 6.9 ms).  T is scaled to entries of at
+// most 1, so that the pair (p_i, p_{i-1}) can lose at most 53 bits a row and gain two: every eighth row rescales it by a power of two.  A zero counts as
 // of the other sign than its predecessor (a zero pivot replaced by a small negative one).
 __device__ __forceinline__ int sturm_count(const double* __restrict__ d, const double* __restrict__ e2, int n,
                                            double x) {
@@ -721,16 +721,44 @@ __device__ __forceinline__ int sturm_count(const double* __restrict__ d, const d
   return cnt;
 }
 
-// ds, e2: T scaled by the power of two that brings its Gershgorin interval to at most 1 in magnitude (bounds[2])
+// The same in FP32, rescaled every fourth row (24 bits a row).
+__device__ __forceinline__ int sturm_count(const float* __restrict__ d, const float* __restrict__ e2, int n, float x) {
+  auto nonzero = [](float p, float before) {
+    return p == 0.0f ? __int_as_float((__float_as_int(before) & 0x80000000) ^ (int)0xab800000) : p;  // -+ 2^-40
+  };
+  float p0 = 1.0f, p1 = nonzero(d[0] - x, 1.0f);
+  int cnt = (unsigned)__float_as_int(p1) >> 31;
+  for (int i0 = 1; i0 < n; i0 += 4) {
+    const int e = max((__float_as_int(p0) >> 23) & 0xff, (__float_as_int(p1) >> 23) & 0xff);
+    const float sc = __int_as_float(max(254 - e, 1) << 23);
+    p0 *= sc;
+    p1 *= sc;
+    const int i1 = min(i0 + 4, n);
+#pragma unroll 4
+    for (int i = i0; i < i1; ++i) {
+      const float p = nonzero(fmaf(d[i] - x, p1, -(e2[i - 1] * p0)), p1);
+      cnt += (unsigned)(__float_as_int(p) ^ __float_as_int(p1)) >> 31;
+      p0 = p1;
+      p1 = p;
+    }
+  }
+  return cnt;
+}
+
+// ds, e2: T scaled by the power of two that brings its Gershgorin interval to at most 1 in magnitude (bounds[2]), and
+// both rounded to FP32
 __global__ void tri_scale_kernel(const double* __restrict__ d, const double* __restrict__ e, int n,
-                                 const double* __restrict__ bounds, double* __restrict__ ds, double* __restrict__ e2) {
+                                 const double* __restrict__ bounds, double* __restrict__ ds, double* __restrict__ e2,
+                                 float* __restrict__ dsf, float* __restrict__ e2f) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double s = bounds[2];
   ds[i] = d[i] * s;
+  dsf[i] = (float)ds[i];
   if (i < n - 1) {
     const double es = e[i] * s;
     e2[i] = es * es;
+    e2f[i] = (float)e2[i];
   }
 }
 
@@ -738,10 +766,16 @@ __global__ void tri_scale_kernel(const double* __restrict__ d, const double* __r
 // lanes evaluate the Sturm count at L interior points of the bracket, which shrinks (L+1)-fold per pass, to the
 // resolution 2 eps max|bound|.  The count is non-decreasing in x, so the points with count <= k form a prefix
 // of the group and the new bracket is read off the ballot.  L = 1 is plain bisection (the fewest counts); the
-// launcher raises L only until the GPU's SMs all have work, since a Sturm count (one FP64 division per row)
-// queues on the SM's FP64 pipe.  Groups that have converged idle until their whole warp has.
+// launcher raises L only until the GPU's SMs all have work, since a Sturm count queues on the SM's FP64 pipe.  Groups
+// that have converged idle until their whole warp has.
+// The first 20 bits come from FP32 counts of the rounded T (an FP32 instruction costs a sixtieth): their bracket,
+// widened by 2^-18 for the rounding (entries of at most 1, each off by a few 2^-24), is only where the first FP64
+// points lie, from its one end to the other inside the Gershgorin interval; the FP64 counts decide.  n = 1,520:
+// 4.6 -> 3.6 ms.
 __global__ void __launch_bounds__(128) tri_multisect_kernel(const double* __restrict__ d,
                                                             const double* __restrict__ e2, int n,
+                                                            const float* __restrict__ df,
+                                                            const float* __restrict__ e2f,
                                                             const double* __restrict__ bounds,
                                                             double* __restrict__ W, int L) {
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -752,11 +786,32 @@ __global__ void __launch_bounds__(128) tri_multisect_kernel(const double* __rest
   double lo = bounds[0] * sc, hi = bounds[1] * sc;
   const double tol = 2.0 * DBL_EPSILON * fmax(fabs(lo), fabs(hi));
   bool done = k >= n;
+  float lof = (float)lo, hif = (float)hi;
+  for (int it = 0; it < 24; ++it) {
+    const bool narrow = done || !(hif - lof > 0x1p-19f);
+    if (__all_sync(0xffffffffu, narrow)) break;
+    const float xf = lof + (hif - lof) / (float)(L + 1) * (float)(g + 1);
+    const int cnt = narrow ? 0 : sturm_count(df, e2f, n, xf);
+    const unsigned bal = __ballot_sync(0xffffffffu, !narrow && cnt <= k);
+    const int nlo = __popc(bal & gmask);
+    const float xlo = __shfl_sync(0xffffffffu, xf, base + max(nlo - 1, 0));
+    const float xhi = __shfl_sync(0xffffffffu, xf, base + min(nlo, L - 1));
+    if (!narrow) {
+      lof = nlo > 0 ? xlo : lof;
+      hif = nlo < L ? xhi : hif;
+    }
+  }
+  const double first = (double)lof - 0x1p-18, last = (double)hif + 0x1p-18;
+  const int nfirst = L > 1 ? 1 : 2;  // passes over the FP32 bracket
   for (int it = 0; it < 256; ++it) {
     if (!done && !(hi - lo > tol)) done = true;
     if (__all_sync(0xffffffffu, done)) break;
     const double h = (hi - lo) / (double)(L + 1);
-    const double x = lo + h * (double)(g + 1);
+    double x = lo + h * (double)(g + 1);
+    if (it < nfirst) {
+      x = L > 1 ? first + (last - first) / (double)(L - 1) * (double)g : it == 0 ? first : last;
+      x = fmin(fmax(x, lo), hi);
+    }
     const int cnt = done ? 0 : sturm_count(d, e2, n, x);
     const unsigned bal = __ballot_sync(0xffffffffu, !done && cnt <= k);
     const int nlo = __popc(bal & gmask);
@@ -765,7 +820,7 @@ __global__ void __launch_bounds__(128) tri_multisect_kernel(const double* __rest
     if (!done) {
       const double nl = nlo > 0 ? xlo : lo;
       const double nh = nlo < L ? xhi : hi;
-      if (nl == lo && nh == hi)
+      if (nl == lo && nh == hi && it >= nfirst)
         done = true;  // no representable progress
       else {
         lo = nl;
@@ -1095,6 +1150,7 @@ inline int bt_columns(int n, size_t* smem) {
 struct TriScratch {
   zd *xw, *u, *next, *tau, *dots, *g, *W, *P;
   double *sparts, *e, *d, *ds, *e2, *bounds;
+  float *dsf, *e2f;
   TriCol* col;
   int *Aex, *exv;
   int4* Aq;
@@ -1124,6 +1180,8 @@ struct TriScratch {
     ds = reinterpret_cast<double*>(take(n * sizeof(double)));
     e2 = reinterpret_cast<double*>(take(n * sizeof(double)));
     bounds = reinterpret_cast<double*>(take(4 * sizeof(double)));
+    dsf = reinterpret_cast<float*>(take(n * sizeof(float)));
+    e2f = reinterpret_cast<float*>(take(n * sizeof(float)));
     Aex = reinterpret_cast<int*>(take(nt * sizeof(int)));
     exv = reinterpret_cast<int*>(take(n * sizeof(int)));
     bytes = (size_t)(p - reinterpret_cast<unsigned char*>(base));
@@ -1216,10 +1274,11 @@ cudaError_t launch_dense_eig(zd* A, int n, int lda, bool upper_only, double* W, 
   const cudaError_t err = tridiagonalise(A, n, lda, t, s);
   if (err != cudaSuccess) return err;
   tri_finish_kernel<<<1, 1024, 0, s>>>(A, n, lda, d, e, bounds); ++g_launch_count;
-  tri_scale_kernel<<<(n + 255) / 256, 256, 0, s>>>(d, e, n, bounds, ds, e2); ++g_launch_count;
+  tri_scale_kernel<<<(n + 255) / 256, 256, 0, s>>>(d, e, n, bounds, ds, e2, t.dsf, t.e2f); ++g_launch_count;
   int L = 1;  // about two warps per SM
   while (L < 32 && (long)n * L < 152L * 64) L *= 2;
-  tri_multisect_kernel<<<(unsigned)(((long)n * L + 127) / 128), 128, 0, s>>>(ds, e2, n, bounds, W, L); ++g_launch_count;
+  tri_multisect_kernel<<<(unsigned)(((long)n * L + 127) / 128), 128, 0, s>>>(ds, e2, n, t.dsf, t.e2f, bounds, W,
+                                                                             L); ++g_launch_count;
   if (Z) {
     double* Zt = reinterpret_cast<double*>(vscratch);
     double* work = Zt + (size_t)n * n;
