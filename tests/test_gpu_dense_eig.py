@@ -55,7 +55,7 @@ def test_eigenpairs(ctx, n, kind):
     assert np.abs(Z.conj().T @ Z - np.eye(n)).max() <= 1e-8
 
 
-@pytest.mark.parametrize("scale", [1e-150, 1e-100, 1e150])
+@pytest.mark.parametrize("scale", [1e-154, 1e-150, 1e-100, 1e150])
 @pytest.mark.parametrize("n", [33, 130])
 def test_scaled_eigenvalues(ctx, n, scale):
     A = matrix(n, "random") * scale

@@ -64,9 +64,12 @@ __device__ __forceinline__ double pow2(int e) {
   return scalbn(1.0, e);
 }
 // an exact sum of products hh 2^56 + cr 2^28 of groups with exponents adding to e, as a double
-// (2^28 alone may lie below the range of doubles where 2^56 does not)
-__device__ __forceinline__ double from_sums(long long hh, long long cr, double s56) {
-  return fma((double)cr, 0x1p-28, (double)hh) * s56;
+// (2^28 alone may lie below the range of doubles where 2^56 does not; for products near its end s56 is 2^60 too large
+// and the sum, at least 2^-28 or zero, is taken down before it, by its exponent field)
+__device__ __forceinline__ double from_sums(long long hh, long long cr, double s56, bool down) {
+  double t = fma((double)cr, 0x1p-28, (double)hh);
+  if (down && t != 0.0) t = __hiloint2double(__double2hiint(t) - (60 << 20), __double2loint(t));
+  return t * s56;
 }
 __device__ __forceinline__ void mac(long long& hh, long long& cr, int ah, int al, int bh, int bl) {
   hh += (long long)ah * bh;
@@ -403,13 +406,15 @@ __global__ void __launch_bounds__(256, 3) tri_symv_kernel(zd* __restrict__ A, in
   __syncthreads();
   const int second = tid / kT, out = (second ? C : R) * kT + row;
   if (tid < 2 * kT && out < n) {
-    const double s56 = pow2(Aex[t] + (second ? exR : exC) - 2 * kQ + 56);
+    const int e56 = Aex[t] + (second ? exR : exC) - 2 * kQ + 56;
+    const bool down = e56 < -960 && e56 > -1200;
+    const double s56 = pow2(e56 + (down ? 60 : 0));
     const long long* q = sums + second * 16 * kT + row;
     long long v[4];
 #pragma unroll
     for (int c = 0; c < 4; ++c) v[c] = (q[c * kT] + q[(4 + c) * kT]) + (q[(8 + c) * kT] + q[(12 + c) * kT]);
     const int slot = second ? (R == C ? nT : R) : C;
-    P[(size_t)slot * n + out] = mk<double>(from_sums(v[0], v[1], s56), from_sums(v[2], v[3], s56));
+    P[(size_t)slot * n + out] = mk<double>(from_sums(v[0], v[1], s56, down), from_sums(v[2], v[3], s56, down));
   }
 }
 
