@@ -213,11 +213,12 @@ __global__ void __launch_bounds__(256) gram_pair_partial_kernel(const cplx<S>* _
 // pair spreads over 36 CTAs).  Every component is added in the row order of gram_partial_kernel with the same
 // operations, so the partials are bitwise those of one CTA per part.  Pair of 48 columns: 2,304 rows 868 -> 75 us
 // (12 parts: 12 CTAs before; a floor of 68), 34,560 rows 1,727 -> 1,063 us (a floor of 1,010); X^H [W P] there
-// 388 -> 128 us (112).
+// 388 -> 128 us (112).  With PAIR and upper (columns q = p): on and above the diagonal only, for products that need not
+// keep the bits of both triangles; 34,560 rows 1,063 -> 587 us.
 template <int NC, int NE, bool PAIR>
 __global__ void __launch_bounds__(256) gram64_kernel(const zd* __restrict__ A, int lda, int p, const zd* __restrict__ B,
                                                      int ldb, int q, int nrow, double* __restrict__ partial,
-                                                     int rows_per_part, int npart, BatchMap bm, int RT) {
+                                                     int rows_per_part, int npart, BatchMap bm, int RT, int upper) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int W = p + q, tid = threadIdx.x;
   zd* rows = reinterpret_cast<zd*>(smem_raw);  // two stages of RT rows: [2][RT][p of A, then q of B]
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(256) gram64_kernel(const zd* __restrict__ A, i
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
   // entry t of this thread: columns ia of A and jb of the staged row (A's again for the first matrix of a pair)
-  const int n = p * q, items = (PAIR ? 2 : 1) * n * (NC == 1 ? 2 : 1);
+  const int n = p * q, ne = PAIR && upper ? p * (p + 1) / 2 : n, items = (PAIR ? 2 : 1) * ne * (NC == 1 ? 2 : 1);
   int ia[NE], jb[NE], im[NE];
   double re[NE], imv[NE];
 #pragma unroll
@@ -246,10 +247,18 @@ __global__ void __launch_bounds__(256) gram64_kernel(const zd* __restrict__ A, i
       im[t] = x >= items / 2;
       x -= im[t] * (items / 2);
     }
-    const bool second = !PAIR || x >= n;
-    if (PAIR && second) x -= n;
-    ia[t] = x / q;
-    jb[t] = x - ia[t] * q + (second ? p : 0);
+    const bool second = !PAIR || x >= ne;
+    if (PAIR && second) x -= ne;
+    if (PAIR && upper) {  // row ia <= column j of the packed upper triangle
+      int j = (int)((sqrtf(8.0f * (float)x + 1.0f) - 1.0f) * 0.5f);  // corrected exactly below
+      while ((j + 1) * (j + 2) / 2 <= x) ++j;
+      while (j * (j + 1) / 2 > x) --j;
+      ia[t] = x - j * (j + 1) / 2;
+      jb[t] = j + (second ? p : 0);
+    } else {
+      ia[t] = x / q;
+      jb[t] = x - ia[t] * q + (second ? p : 0);
+    }
     re[t] = imv[t] = 0.0;
   }
   const long nst = (r_end - r_begin + RT - 1) / RT;
@@ -307,15 +316,15 @@ __global__ void __launch_bounds__(256) gram64_kernel(const zd* __restrict__ A, i
 // Entries in twos where that still gives every SM eight CTAs, single ones where it gives six, else components.
 template <bool PAIR>
 cudaError_t run_gram64(const zd* A, int lda, int p, const zd* B, int ldb, int q, int nrow, double* partial, int rpp,
-                       int npart, cudaStream_t s, const BatchMap& bm) {
-  const int n = (PAIR ? 2 : 1) * p * q;
+                       int npart, cudaStream_t s, const BatchMap& bm, bool upper = false) {
+  const int n = (PAIR ? 2 : 1) * (upper ? p * (p + 1) / 2 : p * q);
   auto run = [&](auto kernel, int per_thread, int nt, int total, int rt) {
     const size_t smem = (size_t)2 * rt * (p + q) * sizeof(zd);
     const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(kernel), smem);
     if (e != cudaSuccess) return e;
     const int chunk = per_thread * nt;
     kernel<<<dim3(npart, (total + chunk - 1) / chunk), nt, smem, s>>>(A, lda, p, B, ldb, q, nrow, partial, rpp, npart,
-                                                                      bm, rt);
+                                                                      bm, rt, upper ? 1 : 0);
     ++g_launch_count;
     return cudaGetLastError();
   };
@@ -468,9 +477,10 @@ __global__ void __launch_bounds__(256) sum_partials_herm_kernel(const double* __
 // out[e] = sum over b of partial[b][e] over the parts of system blockIdx.y (out at a stride of out_stride per
 // system): a CTA owns 32 consecutive e (sum_parts_cta).
 // With out2: blockIdx.z = 1 sums the second set of partials (npart parts further on) into out2.
+// With herm: herm x herm Hermitian matrices of which the partials hold the upper triangles.
 __global__ void __launch_bounds__(256) sum_partials_kernel(const double* __restrict__ partial, int npart, int n,
                                                            double* __restrict__ out, BatchMap bm, long out_stride,
-                                                           double* __restrict__ out2 = nullptr) {
+                                                           double* __restrict__ out2 = nullptr, int herm = 0) {
   __shared__ double red[8][33];
   const int e = blockIdx.x * 32 + (threadIdx.x & 31);
   const int sys = blockIdx.y;
@@ -478,9 +488,18 @@ __global__ void __launch_bounds__(256) sum_partials_kernel(const double* __restr
     partial += (size_t)npart * n;
     out = out2;
   }
+  int src = e;
+  bool conj = false;
+  if (herm > 0 && e < n) {
+    const int i = e / 2 / herm, j = e / 2 - i * herm;
+    if (i > j) {
+      src = 2 * (j * herm + i) + (e & 1);
+      conj = e & 1;
+    }
+  }
   if (bm_frozen(bm, sys)) return;
-  const double t = sum_parts_cta(partial, npart, n, e, sys, bm, red);
-  if (threadIdx.x < 32 && e < n) out[(size_t)sys * out_stride + e] = t;
+  const double t = sum_parts_cta(partial, npart, n, src, sys, bm, red);
+  if (threadIdx.x < 32 && e < n) out[(size_t)sys * out_stride + e] = conj ? -t : t;
 }
 
 // ----------------------------------------------------------------------------- update: Out = beta Out + S C
@@ -1294,7 +1313,8 @@ cudaError_t launch_gram(const cplx<S>* A, int lda, int p, const cplx<S>* B, int 
 
 template <class S>
 cudaError_t launch_gram_pair(const cplx<S>* A, const cplx<S>* B, int ld, int p, int nrow, zd* outM, zd* outG,
-                             double* partial, int npart, cudaStream_t s, const BatchMap& bm, long out_stride) {
+                             double* partial, int npart, cudaStream_t s, const BatchMap& bm, long out_stride,
+                             bool upper) {
   if (p > 48) return cudaErrorInvalidValue;
   if (bm.parts) npart = bm.nparts;
   const int rpp = (nrow + npart - 1) / npart;
@@ -1310,7 +1330,7 @@ cudaError_t launch_gram_pair(const cplx<S>* A, const cplx<S>* B, int ld, int p, 
     }
   }
   if constexpr (sizeof(S) == 8) {
-    const cudaError_t e = run_gram64<true>(A, ld, p, B, ld, p, nrow, partial, rpp, npart, s, bm);
+    const cudaError_t e = run_gram64<true>(A, ld, p, B, ld, p, nrow, partial, rpp, npart, s, bm, upper);
     if (e != cudaSuccess) return e;
   } else {
     const int ti = (p + 15) / 16;
@@ -1325,7 +1345,8 @@ cudaError_t launch_gram_pair(const cplx<S>* A, const cplx<S>* B, int ld, int p, 
   // both sets in one launch (the G partials keep the part numbering, npart parts further on)
   sum_partials_kernel<<<dim3((n + 31) / 32, bm.nsys, 2), 256, 0, s>>>(partial, npart, n,
                                                                        reinterpret_cast<double*>(outM), bm,
-                                                                       2 * out_stride, reinterpret_cast<double*>(outG));
+                                                                       2 * out_stride, reinterpret_cast<double*>(outG),
+                                                                       sizeof(S) == 8 && upper ? p : 0);
   ++g_launch_count;
   return cudaGetLastError();
 }
@@ -1509,7 +1530,7 @@ cudaError_t launch_init_guess(cplx<S>* X, int ldx, int nrow, int m, const int* i
   template cudaError_t launch_gram<S>(const cplx<S>*, int, int, const cplx<S>*, int, int, int, zd*, double*, int,  \
                                       cudaStream_t, const BatchMap&, long);                                       \
   template cudaError_t launch_gram_pair<S>(const cplx<S>*, const cplx<S>*, int, int, int, zd*, zd*, double*, int,    \
-                                           cudaStream_t, const BatchMap&, long);                                   \
+                                           cudaStream_t, const BatchMap&, long, bool);                                   \
   template cudaError_t launch_update<S>(const cplx<S>*, int, int, const zd*, int, int, int, cplx<S>*, int, double, \
                                         double, cudaStream_t, const BatchMap&, long);                             \
   template cudaError_t launch_orth_update<S>(const cplx<S>*, const cplx<S>*, int, int, const zd*, cplx<S>*,        \

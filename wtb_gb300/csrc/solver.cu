@@ -321,12 +321,12 @@ struct Small {
 template <class S>
 int rayleigh_ritz(const cplx<S>* Sb, const cplx<S>* ASb, int ld, int nb, int m, int nrow, double tau, Small& sm,
                   double* partial, int npart, DevStatus* st, cudaStream_t s, std::string* msg, bool small_in_fp64,
-                  const BatchMap& bm, long nn, long ts) {
+                  const BatchMap& bm, long nn, long ts, bool upper = false) {
   (void)st;
   if (nb <= 48) {
     // both Grams in one pass over the basis (bitwise the same sums as two separate launches; with 33..48 FP32
-    // columns the upper triangles only, the lower ones their conjugates)
-    CK(launch_gram_pair<S>(Sb, ASb, ld, nb, nrow, sm.M, sm.G, partial, npart, s, bm, nn));
+    // columns, and with upper, the upper triangles only, the lower ones their conjugates)
+    CK(launch_gram_pair<S>(Sb, ASb, ld, nb, nrow, sm.M, sm.G, partial, npart, s, bm, nn, upper));
   } else {
     CK(launch_gram<S>(Sb, ld, nb, Sb, ld, nb, nrow, sm.M, partial, npart, s, bm, nn));
     CK(launch_gram<S>(Sb, ld, nb, ASb, ld, nb, nrow, sm.G, partial, npart, s, bm, nn));
@@ -784,7 +784,8 @@ int lobpcg_solve_batch(Operator<S>& op, const double* diag, const BatchLayout& L
   Small smi = sm;
   smi.theta = th_dev;
   auto rr_and_update = [&]() -> int {
-    int r = rayleigh_ritz<S>(Sb, ASb, ld, nb, m, nrow, tau, smi, partial, npart, st, s, msg, false, bm, nn, nb);
+    int r = rayleigh_ritz<S>(Sb, ASb, ld, nb, m, nrow, tau, smi, partial, npart, st, s, msg, false, bm, nn, nb,
+                             op.hermitian_grams());
     if (r) return r;
     CK(raise_smem_limit(reinterpret_cast<const void*>(lob_update_kernel<S>), upd_smem));
     lob_update_kernel<S><<<upd_grid, 256, upd_smem, s>>>(Sb, ASb, ld, m, sm.C, nrow, bm, nn);

@@ -92,6 +92,8 @@ struct Operator {
   // on: the next applications define the reported eigenvalues (final Rayleigh-Ritz); an operator may use
   // a slower, more accurate accumulation for them
   virtual void set_final(bool on) { (void)on; }
+  // true where the FP64 Rayleigh-Ritz Grams may be formed from their upper triangles alone
+  virtual bool hermitian_grams() const { return false; }
   // true while launches are being captured into a graph (no event timing then)
   bool capturing = false;
   // everything a captured application depends on besides buffer contents (configuration and addresses)
@@ -191,6 +193,9 @@ struct MatFreeOperator : Operator<S> {
     npairs = npairs_refine;
     return true;
   }
+  // The product's solves keep the bits of both triangles (make_operator says why); those with the FFT's rounding do not:
+  // M = S^H S and G = S^H H S are Hermitian to rounding, and half of either is half of the FP64 work.
+  bool hermitian_grams() const override { return kind == GEMM_FFT_F64; }
   void signature(std::vector<uint64_t>* sig) const override {
     const uint64_t v[] = {2, (uint64_t)kind, (uint64_t)nk, (uint64_t)nv, (uint64_t)nc, (uint64_t)w, (uint64_t)nbmax,
                           (uint64_t)nslices, (uint64_t)npairs, (uint64_t)npairs_refine, (uint64_t)kchunk_final,

@@ -256,11 +256,12 @@ template <class S>
 cudaError_t launch_gram(const cplx<S>* A, int lda, int p, const cplx<S>* B, int ldb, int q, int nrow,
                         zd* out, double* partial, int npart, cudaStream_t s, const BatchMap& bm = BatchMap(),
                         long out_stride = 0);
-// outM = A^H A and outG = A^H B in one pass over the rows (p <= 48 columns); partial holds 2 * npart p p doubles
+// outM = A^H A and outG = A^H B in one pass over the rows (p <= 48 columns); partial holds 2 * npart p p doubles.
+// upper (FP64): the upper triangles, and their conjugates below (B = H A with H Hermitian)
 template <class S>
 cudaError_t launch_gram_pair(const cplx<S>* A, const cplx<S>* B, int ld, int p, int nrow, zd* outM, zd* outG,
                              double* partial, int npart, cudaStream_t s, const BatchMap& bm = BatchMap(),
-                             long out_stride = 0);
+                             long out_stride = 0, bool upper = false);
 // outM, outG: the sums over npart parts of the two partial sets [part][n] at partial and partial + npart n
 cudaError_t launch_sum_partials_pair(const double* partial, int npart, int n, zd* outM, zd* outG, cudaStream_t s,
                                      const BatchMap& bm, long out_stride);
