@@ -121,12 +121,14 @@ struct TriCol {
 };
 
 // Programmatic dependent launch: a kernel's CTAs start once every CTA of the one before has called launch_next, and
-// wait_previous returns once that kernel has completed.
+// wait_previous returns once that kernel has completed.  What that kernel writes changes while this one runs, so no
+// pointer of K1, K2 and the functions they call is restrict: such a pointer's loads may be taken from the read-only path
+// or moved above the wait.
 __device__ __forceinline__ void wait_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // alpha = -(tau/2) sum_b dots[b], the sum split over one warp's lanes in a fixed order.
-__device__ __forceinline__ zd her2_alpha(const zd* __restrict__ dots, int ndots, zd tau) {
+__device__ __forceinline__ zd her2_alpha(const zd* dots, int ndots, zd tau) {
   zd d = mk<double>(0.0, 0.0);
   for (int b = threadIdx.x & 31; b < ndots; b += 32) d = cadd(d, dots[b]);
   for (int o = 16; o > 0; o >>= 1) {
@@ -164,14 +166,14 @@ constexpr int kNextRows = 16;  // rows of the next column of a CTA of K1
 //   at m = 2,304 where the FP64 product took 55; small ones by the chain of waits and FP64 sums, 7 to 9 us; 11.9 us
 //   averaged over the columns of n = 2,304 (14.1 with four real products, two CTAs an SM and one CTA per v and w).
 //   Within a panel the tiles' elements are on their way before the kernel before has finished.
-__global__ void __launch_bounds__(256, 3) tri_symv_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
-                                                       zd* __restrict__ W, const zd* __restrict__ u,
-                                                       const zd* __restrict__ xw, const zd* __restrict__ dots,
-                                                       const double* __restrict__ sparts, int ndots,
-                                                       const int4* __restrict__ Aq, const int* __restrict__ Aex,
-                                                       TriCol* __restrict__ col, zd* __restrict__ tau_out,
-                                                       double* __restrict__ e_out, zd* __restrict__ g, int nch,
-                                                       zd* __restrict__ next, int nnext, zd* __restrict__ P) {
+__global__ void __launch_bounds__(256, 3) tri_symv_kernel(zd* A, int n, int lda, int j, int i,
+                                                       zd* W, const zd* u,
+                                                       const zd* xw, const zd* dots,
+                                                       const double* sparts, int ndots,
+                                                       const int4* Aq, const int* Aex,
+                                                       TriCol* col, zd* tau_out,
+                                                       double* e_out, zd* g, int nch,
+                                                       zd* next, int nnext, zd* P) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double s_s;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -427,15 +429,15 @@ __global__ void __launch_bounds__(256, 3) tri_symv_kernel(zd* __restrict__ A, in
 // is done by nine lanes of one warp.  7.1 us averaged over the columns of n = 2,304 (8.1 with the sums of next formed
 // here); the two kernels took the place of three (32 us a column) that brought the next column up to date by
 // themselves: n = 2,304 84 -> 71 ms, and 65 with both as they are.
-__global__ void __launch_bounds__(16 * (kRows + 2)) tri_x_kernel(zd* __restrict__ A, int n, int lda, int j, int i,
-                                                                 const zd* __restrict__ next,
-                                                                 const zd* __restrict__ W,
-                                                                 const zd* __restrict__ P,
-                                                                 const TriCol* __restrict__ col,
-                                                                 const zd* __restrict__ g, int nch,
-                                                                 zd* __restrict__ u,
-                                                                 zd* __restrict__ xw, zd* __restrict__ dots,
-                                                                 double* __restrict__ sparts) {
+__global__ void __launch_bounds__(16 * (kRows + 2)) tri_x_kernel(zd* A, int n, int lda, int j, int i,
+                                                                 const zd* next,
+                                                                 const zd* W,
+                                                                 const zd* P,
+                                                                 const TriCol* col,
+                                                                 const zd* g, int nch,
+                                                                 zd* u,
+                                                                 zd* xw, zd* dots,
+                                                                 double* sparts) {
   __shared__ zd gv[kNB], gw[kNB], sx[kRows + 1];
   const int tid = threadIdx.x, lane = tid & 15, half = tid / 16, j0 = j - i;
   wait_previous();
