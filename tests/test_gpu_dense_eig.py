@@ -61,3 +61,10 @@ def test_scaled_eigenvalues(ctx, n, scale):
     A = matrix(n, "random") * scale
     W, ref = ctx.zheev(A), np.linalg.eigvalsh(A)
     assert np.abs(W - ref).max() <= n * EPS * np.abs(ref).max()
+
+
+# columns a CTA of the back-transformation and slices of a column: 1 and 256, 2 and 128, 3 and 85 (no multiple of the eight
+# lanes that add them up)
+@pytest.mark.parametrize("n", [608, 609, 1216, 1217, 1300, 1368])
+def test_eigenpairs_by_columns_a_block(ctx, n):
+    test_eigenpairs(ctx, n, "random")

@@ -31,3 +31,10 @@ def test_early_started_kernels_take_no_restrict_pointers():
                 if re.search(r"\b%s\(" % callee, body):
                     assert "__restrict__" not in callee_params, (name, callee)
     assert early >= 2  # the dense reduction's two kernels a column
+
+
+def test_shuffle_masks_are_not_taken_from_the_active_lanes():
+    """Which lanes are active after a loop of different trip counts is the compiler's choice: a mask names its lanes."""
+    for path in SOURCES:
+        with open(path) as f:
+            assert "__activemask" not in f.read(), path

@@ -1068,7 +1068,7 @@ __global__ void __launch_bounds__(kBtThreads) tri_backtransform_kernel(const zd*
         sr += red[0][q * kc + cc];
         si += red[1][q * kc + cc];
       }
-      const unsigned m = __activemask();
+      const unsigned m = 0xffu << (tid & 24);  // the column's eight lanes: their trip counts above may differ
       for (int o = 4; o > 0; o >>= 1) {
         sr += __shfl_xor_sync(m, sr, o);
         si += __shfl_xor_sync(m, si, o);
