@@ -983,7 +983,8 @@ __global__ void __launch_bounds__(32) tri_invit_kernel(const double* __restrict_
 }
 
 // The reflectors quantised in place for the back-transformation: v_j(1:) (rows j + 2 ..) of column j as int4 with the
-// exponent exv[j]; v_j(0) = 1 is implied.  One CTA per column.
+// exponent exv[j]; v_j(0) = 1 is implied.  One CTA per column.  A column's sum v^H z of the high limbs is at most
+// 2^55 sqrt(2 n) (z has unit length): one bit less in v keeps it in 64 bits beyond 16,384 rows.
 __global__ void __launch_bounds__(256) tri_quantise_kernel(zd* __restrict__ A, int n, int lda, int* __restrict__ exv) {
   __shared__ int s_f;
   const int j = blockIdx.x, tid = threadIdx.x;
@@ -995,7 +996,7 @@ __global__ void __launch_bounds__(256) tri_quantise_kernel(zd* __restrict__ A, i
   f = __reduce_max_sync(0xffffffffu, f);
   if ((tid & 31) == 0) atomicMax(&s_f, f);
   __syncthreads();
-  const int ex = group_ex(s_f);
+  const int ex = group_ex(s_f) + (n > 16384 ? 1 : 0);
   if (tid == 0) exv[j] = ex;
   int4* q = reinterpret_cast<int4*>(v);
   for (int r = j + 2 + tid; r < n; r += 256) q[r] = quantise(v[r], ex);
@@ -1010,7 +1011,13 @@ __global__ void __launch_bounds__(256) tri_quantise_kernel(zd* __restrict__ A, i
 // to 2^-56 of its terms.  Bound by the integer multiply-adds (24 an entry and reflector; the FP64 form 8 on a pipe
 // a twelfth as fast).  n = 1,520: 38.9 -> 16.1 ms.
 // Z(i, k) = Z[i * n + k] (row-major), conjugated at the end when the solver worked on conj(H).
-constexpr int kBtThreads = 256;
+// A row adds up to 2^56.6 to a low sum, so it is carried into the high one every kBtFold rows of a thread; columns in
+// shared memory have at most 50 and go without (the nested loop took n = 1,520 from 50.5 to 52.3 ms).
+constexpr int kBtThreads = 256, kBtFold = 64;
+__device__ __forceinline__ void carry(long long& hh, long long& cr) {
+  hh += cr >> 28;
+  cr &= (1ll << 28) - 1;
+}
 __global__ void __launch_bounds__(kBtThreads) tri_backtransform_kernel(const zd* __restrict__ A, int n, int lda,
                                                                        const zd* __restrict__ tau,
                                                                        const int* __restrict__ exv,
@@ -1045,17 +1052,25 @@ __global__ void __launch_bounds__(kBtThreads) tri_backtransform_kernel(const zd*
     const int i0 = j + 2 + ((sl - (j + 2)) % nsl + nsl) % nsl;  // this thread's first row from j + 2 on
     const bool head = on && (j + 1) % nsl == sl;                // it owns row j + 1
     long long rh = 0, rc = 0, ih = 0, ic = 0;
-    if (on)
-      for (int i = i0; i < n; i += nsl) {  // conj(v) z
-        const int4 a = v[i];
-        const longlong2 zi = z[i * ldz];
-        const int xl = (int)zi.x, yl = (int)zi.y;
-        const int xh = (int)(zi.x >> 32) + (xl < 0), yh = (int)(zi.y >> 32) + (yl < 0);
-        const int xs = xl >> 4, ys = yl >> 4;
-        mac(rh, rc, a.x, a.y, xh, xs);
-        mac(rh, rc, a.z, a.w, yh, ys);
-        mac(ih, ic, a.x, a.y, yh, ys);
-        mac(ih, ic, -a.z, -a.w, xh, xs);
+    auto row = [&](int i) {  // conj(v) z
+      const int4 a = v[i];
+      const longlong2 zi = z[i * ldz];
+      const int xl = (int)zi.x, yl = (int)zi.y;
+      const int xh = (int)(zi.x >> 32) + (xl < 0), yh = (int)(zi.y >> 32) + (yl < 0);
+      const int xs = xl >> 4, ys = yl >> 4;
+      mac(rh, rc, a.x, a.y, xh, xs);
+      mac(rh, rc, a.z, a.w, yh, ys);
+      mac(ih, ic, a.x, a.y, yh, ys);
+      mac(ih, ic, -a.z, -a.w, xh, xs);
+    };
+    if (on && in_smem)
+      for (int i = i0; i < n; i += nsl) row(i);
+    else if (on)
+      for (int i = i0; i < n;) {
+        const int i1 = (int)min((long)n, i + (long)kBtFold * nsl);
+        for (; i < i1; i += nsl) row(i);
+        carry(rh, rc);
+        carry(ih, ic);
       }
     red[0][tid] = rh + ((rc + (1ll << 27)) >> 28);
     red[1][tid] = ih + ((ic + (1ll << 27)) >> 28);
