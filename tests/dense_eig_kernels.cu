@@ -1,5 +1,11 @@
-// The back-transformation's kernels by themselves, for test_gpu_dense_eig_kernels.py.
+// The back-transformation's kernels and its rule by themselves, for test_gpu_dense_eig_kernels.py and
+// test_dense_eig_rule.py.
 #include "k_dense_eig.cu"
+
+extern "C" int block_columns(int n) {
+  size_t smem = 0;
+  return wtb::bt_columns(n, &smem);
+}
 
 // v: n complex per column (row r of v_j at v[j * n + r], rows j + 2 on read; quantised in place), ncol columns; tau: n - 1;
 // Zt: n x n, Z: n x n complex; the first `blocks` blocks of kc columns.

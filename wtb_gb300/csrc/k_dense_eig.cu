@@ -1147,17 +1147,21 @@ __global__ void __launch_bounds__(kBtThreads) tri_backtransform_kernel(const zd*
 }
 
 // Columns a CTA of the back-transformation: the fewest rounds of CTAs times columns, with the ~2,500 clocks of a
-// reflector's reduction hidden where several CTAs share an SM.  0: the columns do not fit shared memory.
+// reflector's reduction hidden where several CTAs share an SM, and the fewer columns where two counts tie.  0: the
+// columns do not fit shared memory.  Measured with 1 to 8 columns at 34 sizes from 300 to 4,096: the least time, or
+// within 14 % of it (0.72 ms with 1, 0.68 with 2 at 300; 2.44, 2.12 at 700; 10.5, 11.2 and 8.0 with 3 at 1,300; 13.5, 14.4
+// and 16.4 at 1,459; 18.7, 16.6 and 17.5 at 1,600; 46.2, 54.8 and 59.6 at 2,304).
 inline int bt_columns(int n, size_t* smem) {
   int best = 0;
   double cost = 0.0;
   for (int kc = 1; kc <= 16; ++kc) {
     const size_t b = (size_t)n * kc * sizeof(longlong2);
     if (b > 200 * 1024) break;
-    const int res = (int)std::min<size_t>(4, (220 * 1024) / (b + 6 * 1024));
+    // an SM's 228 KB, of which a CTA takes its columns, 4.75 KB for the sums and 1 KB for the system
+    const int res = (int)std::min<size_t>(4, (228 * 1024) / (b + 5888));
     const long ctas = (n + kc - 1) / kc, rounds = (ctas + 152L * res - 1) / (152L * res);
     const double work = 0.5 * n * kc * 24.0 / 21.0, t = rounds * std::max(res * work, work + 2500.0);
-    if (!best || t < cost) {
+    if (!best || t < cost * (1.0 - 1e-9)) {
       best = kc;
       cost = t;
       *smem = b;
