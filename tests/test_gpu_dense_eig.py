@@ -68,3 +68,17 @@ def test_scaled_eigenvalues(ctx, n, scale):
 @pytest.mark.parametrize("n", [608, 609, 1216, 1217, 1300, 1368])
 def test_eigenpairs_by_columns_a_block(ctx, n):
     test_eigenpairs(ctx, n, "random")
+
+
+# A row c without couplings and rows [[c, b], [b, a]], c one of the points at which the bisection for the pair's upper
+# eigenvalue counts: both pivots there are zero exactly.  (c, b, a), beside rows 1 and -1.
+@pytest.mark.parametrize("c,b,a", [("0x1.187f742108421p-3", "0x1p-10", "-0x1.23c53b869337cp-4"),
+                                   ("0x1.83600b18c6319p-7", "0x1p-11", "-0x1.bc6fe52111fc6p-3"),
+                                   ("0x1.c5b08aa5294a5p-2", "0x1p-11", "0x1.87a34f57a09a0p-5"),
+                                   ("0x1.38a4315ad6b5bp-5", "0x1p-10", "-0x1.e29bfe55f4160p-3")])
+def test_counts_at_two_zero_pivots(ctx, c, b, a):
+    c, b, a = (float.fromhex(x) for x in (c, b, a))
+    A = np.diag([1.0, -1.0, c, c, a]).astype(complex)
+    A[3, 4] = A[4, 3] = b
+    W, ref = ctx.zheev(A), np.linalg.eigvalsh(A)
+    assert np.abs(W - ref).max() <= 5 * EPS * np.abs(ref).max()

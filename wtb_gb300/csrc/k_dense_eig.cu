@@ -700,16 +700,20 @@ __global__ void __launch_bounds__(1024) tri_finish_kernel(const zd* __restrict__
 // (the leading minors; Givens' recurrence, each p_i the exact one of a T whose entries differ by a few ulp).  One
 // multiply-add of latency and three FP64 instructions a row, against a division's chain of 460 clocks and eleven
 // instructions for the ratios q_i = p_{i+1} / p_i (all eigenvalues at n = 2,304: 20 -> 6.9 ms).  T is scaled to entries of at
-// most 1, so that the pair (p_i, p_{i-1}) can lose at most 53 bits a row and gain two: every eighth row rescales it by a power of two.  A zero counts as
-// of the other sign than its predecessor (a zero pivot replaced by a small negative one).
+// most 1.  A zero p_i counts as of the other sign than its predecessor (a zero pivot replaced by a small negative one) and
+// goes on as -2^-110 of it, and a difference d_i - x below 2^-54 as -2^-54 (T off by a quarter of an ulp of its norm), so
+// that a row takes the pair (p_i, p_{i-1}) down by at most 110 bits and up by two: every eighth row rescales it by a
+// power of two.  (A zero that went on at a size of its own made a pivot of any size where its predecessor was small, and
+// the count wrong by one: a row of [[c, b], [b, a]] beside an uncoupled row c, at x = c.)
 __device__ __forceinline__ int sturm_count(const double* __restrict__ d, const double* __restrict__ e2, int n,
                                            double x) {
   auto nonzero = [](double p, double before) {
     return (__double_as_longlong(p) << 1) == 0
-               ? __hiloint2double((__double2hiint(before) & 0x80000000) ^ (int)0xb3700000, 0)  // -+ 2^-200
+               ? __hiloint2double((__double2hiint(before) ^ (int)0x80000000) - (110 << 20), __double2loint(before))
                : p;
   };
-  double p0 = 1.0, p1 = nonzero(d[0] - x, 1.0);
+  auto pivot = [](double t) { return (__double2hiint(t) & 0x7fffffff) < (1023 - 54) << 20 ? -0x1p-54 : t; };
+  double p0 = 1.0, p1 = pivot(d[0] - x);
   int cnt = (unsigned)__double2hiint(p1) >> 31;
   for (int i0 = 1; i0 < n; i0 += 8) {
     const int e = (max((__double2hiint(p0) >> 20) & 0x7ff, (__double2hiint(p1) >> 20) & 0x7ff));
@@ -719,7 +723,7 @@ __device__ __forceinline__ int sturm_count(const double* __restrict__ d, const d
     const int i1 = min(i0 + 8, n);
 #pragma unroll 8
     for (int i = i0; i < i1; ++i) {
-      const double p = nonzero(fma(d[i] - x, p1, -(e2[i - 1] * p0)), p1);
+      const double p = nonzero(fma(pivot(d[i] - x), p1, -(e2[i - 1] * p0)), p1);
       cnt += (unsigned)(__double2hiint(p) ^ __double2hiint(p1)) >> 31;
       p0 = p1;
       p1 = p;
@@ -728,7 +732,8 @@ __device__ __forceinline__ int sturm_count(const double* __restrict__ d, const d
   return cnt;
 }
 
-// The same in FP32, rescaled every fourth row (24 bits a row).
+// The same in FP32, rescaled every fourth row (24 bits a row); a zero goes on as 2^-40, since these counts only say where
+// to look first.
 __device__ __forceinline__ int sturm_count(const float* __restrict__ d, const float* __restrict__ e2, int n, float x) {
   auto nonzero = [](float p, float before) {
     return p == 0.0f ? __int_as_float((__float_as_int(before) & 0x80000000) ^ (int)0xab800000) : p;  // -+ 2^-40
