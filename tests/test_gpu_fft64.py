@@ -50,3 +50,24 @@ def test_operator_matches_the_oracle(built, ngrid, fft):
                                    (3, 49, 1), (100, 2, 1), (64, 5, 1), (13, 4, 3)])
 def test_pruned_and_twiddled_factors(built, ngrid):
     test_operator_matches_the_oracle(built, ngrid, True)
+
+
+# one application and the adjoint's linear solves do not depend on the number of excitons, nor does the form they take
+@pytest.mark.parametrize("nev", [6, 7, 12])
+def test_applications_whatever_the_excitons(built, nev):
+    s = make_system(5, 4, "hex", 3, 1.5, (6, 6, 1))
+    p = BSEParams(ngrid=(9, 8, 1), nc=2, nv=1, coultype="V2DRK", ediel=(1.0, 4.0, 1.0), r0=40.0, nev=nev)
+    ctx = api.Context(0)
+    ctx.set_hr(s)
+    ctx.bsesolver(p, precision="fp64", op="matfree")
+    rng = np.random.default_rng(1)
+    X = rng.normal(size=(p.dim, 3)) + 1j * rng.normal(size=(p.dim, 3))
+    Y = ctx.bse_matvec(p, X, precision="fp64", op="matfree")
+    assert ctx.operator_form() == "FP64 FFT convolution"
+    p.nev = 1
+    assert np.array_equal(Y, ctx.bse_matvec(p, X, precision="fp64", op="matfree"))
+    p.nev = nev
+    ctx.bsesolver(p, precision="fp64", op="matfree")
+    ctx.bse_backward(p, np.ones(nev), np.ones(nev), precision="fp64")
+    assert ctx.operator_form() == "FP64 FFT convolution"
+    ctx.close()

@@ -57,6 +57,7 @@ int ctx_check_status(wtb_ctx* c);
 double ctx_vcell3d(const wtb_ctx* c);  // |a1 . (a2 x a3)| of the lattice (vcell3D)
 CoulParams ctx_coul_params(wtb_ctx* c, const wtb_bse_params* p);
 int ctx_coulomb_table(wtb_ctx* c, const wtb_bse_params* p, double* V, int ldv, bool deriv_r0);
+// for single applications and linear solves (make_operator with eigensolve = false)
 int ctx_make_operator(wtb_ctx* c, const wtb_bse_params* p, int nbmax, OpBundle* ob, const std::string& tag,
                       bool deriv_r0);
 int ctx_stage_system(wtb_ctx* c, const wtb_bse_params* p);

@@ -334,8 +334,10 @@ int auto_block(const wtb_bse_params* p, int dim, bool fp64) {
 // tag: suffix of the buffers holding the V table and its forms (a second operator, e.g. the dV/dr0 one,
 // must not overwrite the first); deriv_r0: build the operator of dV/dr0 with no diagonal term.
 // tune: choose the contraction's column tile by timing (not for the operators a batch contracts jointly)
+// eigensolve: the operator of a solve for p->nev excitons; single applications and the adjoint's linear solves do not
+// depend on p->nev, so neither does the form they take
 int make_operator(wtb_ctx* c, const wtb_bse_params* p, int nbmax, OpBundle* ob, const std::string& tag = "",
-                  bool deriv_r0 = false, bool tune = true) {
+                  bool deriv_r0 = false, bool tune = true, bool eigensolve = true) {
   const int nk = c->nk, nv = c->nv, nc = c->nc, w = c->w;
   const int dim = nk * nc * nv;
   cudaError_t err = cudaSuccess;
@@ -421,7 +423,8 @@ int make_operator(wtb_ctx* c, const wtb_bse_params* p, int nbmax, OpBundle* ob, 
   Fft64Plan plan64;
   double col64 = 0.0;
   const bool three_d = p->ngrid[0] > 1 && p->ngrid[1] > 1 && p->ngrid[2] > 1;
-  if (p->op == WTB_OP_MATFREE && fp64 && mesh && (three_d || p->nev <= 6 || nk >= 1800) && !(fft_env && std::strcmp(fft_env, "0") == 0) &&
+  const bool rule = !eigensolve || three_d || p->nev <= 6 || nk >= 1800;
+  if (p->op == WTB_OP_MATFREE && fp64 && mesh && rule && !(fft_env && std::strcmp(fft_env, "0") == 0) &&
       fft64_plan(p->ngrid[0], p->ngrid[1], p->ngrid[2], &plan64, &col64)) {
     const double* dbl = c->ws.find<double>("recip", 9);
     if (!dbl) return set_err(c, WTB_ESTATE, "reciprocal vectors not staged");
@@ -635,7 +638,7 @@ int ctx_coulomb_table(wtb_ctx* c, const wtb_bse_params* p, double* V, int ldv, b
 }
 int ctx_make_operator(wtb_ctx* c, const wtb_bse_params* p, int nbmax, OpBundle* ob, const std::string& tag,
                       bool deriv_r0) {
-  return make_operator(c, p, nbmax, ob, tag, deriv_r0);
+  return make_operator(c, p, nbmax, ob, tag, deriv_r0, true, false);
 }
 }  // namespace wtb
 
@@ -1732,7 +1735,7 @@ int wtb_bse_matvec(wtb_ctx* c, const wtb_bse_params* p, int ncol, const double* 
   zf* y32 = c->ws.get<zf>("mv_y32", (size_t)dim * ncol, &err);
   CKC(err);
   OpBundle ob;
-  CKR(make_operator(c, p, std::min(ncol, 16), &ob));
+  CKR(make_operator(c, p, std::min(ncol, 16), &ob, "", false, true, false));
   // a single application: the operator's accurate accumulation, as in the eigensolver's final step
   if (ob.o64) ob.o64->set_final(true);
   if (ob.o32) ob.o32->set_final(true);
