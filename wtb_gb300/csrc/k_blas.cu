@@ -930,7 +930,7 @@ __global__ void init_guess_kernel(cplx<S>* X, int ldx, int nrow, int m, const in
 }
 
 // Lowest nwant eigenpairs of the Hermitian part of the leading n x n block of Ag (n = *nptr if nptr, capped
-// at nmax), in precision S, by the tridiagonal route of small_eig.cuh.  evals[k] ascending; evecs (nmax rows,
+// at nmax), in FP32 (S = float; FP64 below), by the tridiagonal route of small_eig.cuh.  evals[k] ascending; evecs (nmax rows,
 // leading dimension ldv): column k for k < min(nwant, n); rows >= n and the columns of missing eigenpairs
 // are zero, and a missing eigenvalue is 1e30 (a direction the orthonormalisation dropped).
 template <class S>
@@ -990,10 +990,10 @@ __global__ void __launch_bounds__(256) heev_small_kernel(const zd* __restrict__ 
   }
 }
 
-// The same in FP64, one cluster of kClu CTAs per system (tridiag_cluster64), bitwise the results of one CTA: every CTA
-// forms T's eigenvalues and eigenvectors (all hold T) and every kClu-th eigenvector of A.
-// 48 x 48, 16 vectors: 597 -> 378 us; 78 x 78, 26 vectors: 1,628 -> 700 us; 16 x 16: 141 -> 124 us.  The serial chains
-// of FP64 roots and divisions are what is left.
+// The same in FP64, one cluster of kClu CTAs per system (tridiag_cluster64): every CTA forms T's eigenvalues and
+// eigenvectors (all hold T) and every kClu-th eigenvector of A.  Against one CTA per system 48 x 48, 16 vectors:
+// 597 -> 378 us; 78 x 78, 26 vectors: 1,628 -> 700 us; 16 x 16: 141 -> 124 us.  The serial chains of FP64 roots and
+// divisions are what is left.
 __global__ void __cluster_dims__(kClu, 1, 1) __launch_bounds__(256)
     heev_cluster64_kernel(const zd* __restrict__ Ag, int lda, const int* __restrict__ nptr, int nmax, int nwant,
                           double* __restrict__ evals, zd* __restrict__ evecs, int ldv, BatchMap bm, long a_stride,
@@ -1433,30 +1433,29 @@ cudaError_t launch_heev_small(const zd* A, int lda, const int* nptr, int nmax, i
                               long v_stride) {
   if (nmax < 1 || nmax > 96 || nwant < 0 || nwant > nmax) return cudaErrorInvalidValue;
   if constexpr (sizeof(S) == 8) {
-    // a cluster where its CTAs can have an SM each (with more systems the SMs are full of one-CTA problems, and
-    // what every CTA of a cluster repeats would be lost) and its layout fits (one warp of vectors, 90 columns)
+    // the layout holds one warp of vectors of 90 columns (the solver asks for 26 of 78 at most)
     const size_t smem = (size_t)nmax * (nmax + 1) * sizeof(zd) + (size_t)3 * nmax * sizeof(zd) +
                         (size_t)(5 * nmax + 5) * sizeof(double) +
                         (size_t)4 * ((nmax + 1) * nwant + 1) * sizeof(double) + (size_t)(nwant + 4) * sizeof(int) + 64;
-    if (bm.nsys * kClu <= 152 && nwant <= 32 && smem <= 224 * 1024) {
-      cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(heev_cluster64_kernel), smem);
-      if (e != cudaSuccess) return e;
-      heev_cluster64_kernel<<<bm.nsys * kClu, 256, smem, s>>>(A, lda, nptr, nmax, nwant, evals, evecs, ldv, bm,
-                                                              a_stride, e_stride, v_stride);
-      ++g_launch_count;
-      return cudaGetLastError();
-    }
+    if (nwant > 32 || smem > 224 * 1024) return cudaErrorInvalidValue;
+    cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(heev_cluster64_kernel), smem);
+    if (e != cudaSuccess) return e;
+    heev_cluster64_kernel<<<bm.nsys * kClu, 256, smem, s>>>(A, lda, nptr, nmax, nwant, evals, evecs, ldv, bm, a_stride,
+                                                            e_stride, v_stride);
+    ++g_launch_count;
+    return cudaGetLastError();
+  } else {
+    const size_t smem = (size_t)nmax * (nmax + 1) * sizeof(cplx<S>) + (size_t)2 * nmax * sizeof(cplx<S>) +
+                        (size_t)(4 * nmax + 4) * sizeof(S) + (size_t)3 * ((nmax + 1) * nwant + 1) * sizeof(S) +
+                        (size_t)(nwant + 4) * sizeof(int) + 64;
+    if (smem > 220 * 1024) return cudaErrorInvalidValue;
+    cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(heev_small_kernel<S>), smem);
+    if (e != cudaSuccess) return e;
+    heev_small_kernel<S><<<bm.nsys, 256, smem, s>>>(A, lda, nptr, nmax, nwant, evals, evecs, ldv, bm, a_stride, e_stride,
+                                                    v_stride);
+    ++g_launch_count;
+    return cudaGetLastError();
   }
-  const size_t smem = (size_t)nmax * (nmax + 1) * sizeof(cplx<S>) + (size_t)2 * nmax * sizeof(cplx<S>) +
-                      (size_t)(4 * nmax + 4) * sizeof(S) + (size_t)3 * ((nmax + 1) * nwant + 1) * sizeof(S) +
-                      (size_t)(nwant + 4) * sizeof(int) + 64;
-  if (smem > 220 * 1024) return cudaErrorInvalidValue;
-  cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(heev_small_kernel<S>), smem);
-  if (e != cudaSuccess) return e;
-  heev_small_kernel<S><<<bm.nsys, 256, smem, s>>>(A, lda, nptr, nmax, nwant, evals, evecs, ldv, bm, a_stride, e_stride,
-                                                  v_stride);
-  ++g_launch_count;
-  return cudaGetLastError();
 }
 
 template <class S>

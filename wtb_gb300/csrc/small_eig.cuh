@@ -226,7 +226,7 @@ __device__ void tridiag_cta(cplx<S>* A, int lda, int n, S* d, S* e, cplx<S>* tau
   __syncthreads();
 }
 
-// Step 1 in FP64 on a cluster of kClu CTAs of 256 threads, bitwise the results of tridiag_cta<double>.  One SM issues an
+// Step 1 in FP64 on a cluster of kClu CTAs of 256 threads, its sums in tridiag_cta's order.  One SM issues an
 // FP64 warp instruction every 19 clocks and a warp one every 64, and the 32,000 of them of a 48 x 48 problem took
 // tridiag_cta 280 us on its SM.  Here row a of A belongs to CTA a mod kClu, which forms its entries of p = tau A22 v (eight
 // lanes a row: the four interleaved sums of tridiag_cta's two lanes, real and imaginary parts apart, added in its
@@ -235,8 +235,8 @@ __device__ void tridiag_cta(cplx<S>* A, int lda, int n, S* d, S* e, cplx<S>* tau
 // barriers a step.  On return every CTA holds d, e, tau and the reflectors (row j right of the diagonal).
 // p, w: n complex, q: n doubles.
 constexpr int kClu = 8;
-// a b + c d with the first product fused: which product of a sum the compiler fuses is written out here, as
-// tridiag_cta<double> has it, so that the two give the same bits whatever surrounds them.
+// a b + c d with the first product fused: which product of a sum is fused is written out, so that the bits do not depend
+// on what the compiler finds around it.
 __device__ __forceinline__ double ab_cd(double a, double b, double c, double d) { return fma(a, b, __dmul_rn(c, d)); }
 __device__ inline void tridiag_cluster64(zd* A, int lda, int n, double* d, double* e, zd* tau, zd* p, zd* w, double* q) {
   namespace cg = cooperative_groups;
