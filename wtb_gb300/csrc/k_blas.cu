@@ -210,8 +210,8 @@ __global__ void __launch_bounds__(256) gram_pair_partial_kernel(const cplx<S>* _
 // SM has entries to add up, not the loads: the grid is reduction part x chunk of the output's entries, each CTA
 // which stages its part's rows for 256 threads of NE entries (NC = 2), or for small problems of one real component of an
 // entry (NC = 1: a part's chain of 192 rows then takes two multiply-adds a row, and a single part of a 48-column
-// pair spreads over 36 CTAs).  Every component is added in the row order of gram_partial_kernel with the same
-// operations, so the partials are bitwise those of one CTA per part.  Pair of 48 columns: 2,304 rows 868 -> 75 us
+// pair spreads over 36 CTAs).  Every component is one chain of fused multiply-adds over its part's rows, so the bits of
+// a part do not depend on the split.  Pair of 48 columns: 2,304 rows 868 -> 75 us
 // (12 parts: 12 CTAs before; a floor of 68), 34,560 rows 1,727 -> 1,063 us (a floor of 1,010); X^H [W P] there
 // 388 -> 128 us (112).  With PAIR and upper (columns q = p): on and above the diagonal only, for products that need not
 // keep the bits of both triangles; 34,560 rows 1,063 -> 587 us.
