@@ -697,8 +697,10 @@ std::vector<Length> lengths(int n) {
   for (int a : kR)
     for (int b : kR) {
       const int P = a * b;
-      // one factor alone makes one item a row: up to 5 points only (16 alone on an 8 x 8 mesh cost
-      // its full run 4.25 instead of 4.03 ms)
+      // one factor alone makes one item a row and most lanes idle: up to 5 points only.  1,024 columns with and without
+      // two factors in their place, of 29 meshes with a dimension of at most 8: 6 x 6 20.6 and 57.8 us, 8 x 8 24.9 and
+      // 115.5, 8 x 1 10.6 and 29.0, 30 x 8 100.7 and 151.1, 4^3 63.6 and 78.2, 8^3 337 and 357, 7^3 and 24 x 24 x 2 the
+      // same; only with the short one beside two longer ones a single factor is ahead, 12 x 12 x 4 422 and 380
       if (a == 1 || (b == 1 && a > 5) || P < 2 * n - 1) continue;
       const bool ct = b > 1 && std::gcd(a, b) != 1;
       long in = dft_cost(a), out = in;
