@@ -82,3 +82,14 @@ def test_counts_at_two_zero_pivots(ctx, c, b, a):
     A[3, 4] = A[4, 3] = b
     W, ref = ctx.zheev(A), np.linalg.eigvalsh(A)
     assert np.abs(W - ref).max() <= 5 * EPS * np.abs(ref).max()
+
+
+# Eigenvalues +-g/2 of rows [[0, g/2], [g/2, 0]] beside an uncoupled row 1.  The reduction changes nothing, and the rounding of
+# the elimination is an ulp of g, so each vector is that of the matrix with its last diagonal entry off by at most the
+# smallest pivot, 2^-56 of the norm, which turns it by half of that over g; 64 ulp for the normalisation and the rest.
+@pytest.mark.parametrize("g", [3e-7, 5e-7, 1e-6, 2e-6, 3e-6, 5e-6, 7e-6, 1e-5, 2e-5, 4e-5])
+def test_vectors_of_close_eigenvalues(ctx, g):
+    A = np.diag([1.0, 0.0, 0.0]).astype(complex)
+    A[1, 2] = A[2, 1] = g / 2
+    Z = np.asarray(ctx.zheev_vectors(A)[1])
+    assert np.abs(Z.conj().T @ Z - np.eye(3)).max() <= 2.0 ** -56 * (1 + 1e-12) / g + 64 * EPS
