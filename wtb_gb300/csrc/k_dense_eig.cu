@@ -700,33 +700,49 @@ __global__ void __launch_bounds__(1024) tri_finish_kernel(const zd* __restrict__
 // (the leading minors; Givens' recurrence, each p_i the exact one of a T whose entries differ by a few ulp).  One
 // multiply-add of latency and three FP64 instructions a row, against a division's chain of 460 clocks and eleven
 // instructions for the ratios q_i = p_{i+1} / p_i (all eigenvalues at n = 2,304: 20 -> 6.9 ms).  T is scaled to entries of at
-// most 1.  A zero p_i counts as of the other sign than its predecessor (a zero pivot replaced by a small negative one) and
-// goes on as -2^-110 of it, and a difference d_i - x below 2^-54 as -2^-54 (T off by a quarter of an ulp of its norm), so
-// that a row takes the pair (p_i, p_{i-1}) down by at most 110 bits and up by two: every eighth row rescales it by a
-// power of two.  (A zero that went on at a size of its own made a pivot of any size where its predecessor was small, and
-// the count wrong by one: a row of [[c, b], [b, a]] beside an uncoupled row c, at x = c.)
+// most 1.  A row takes the pair (p_i, p_{i-1}) up by at most two bits; every eighth row rescales it by a power of two.  A
+// zero p_i counts as of the other sign than its predecessor (a zero pivot replaced by a small negative one) and goes on at
+// the end of the range, far below a predecessor of an ordinary size.  Eight rows that leave the pair below 2^-900, after a
+// zero without couplings or differences d_i - x of nearly nothing, are done again with zeros as -2^-110 of their
+// predecessor and differences below 2^-54 as -2^-54 (T off by a quarter of an ulp of its norm): 110 bits a row at most.  (A
+// zero of a size of its own beside a predecessor as small made the count wrong by one: a row of [[c, b], [b, a]] beside an
+// uncoupled row c, at x = c.)
 __device__ __forceinline__ int sturm_count(const double* __restrict__ d, const double* __restrict__ e2, int n,
                                            double x) {
-  auto nonzero = [](double p, double before) {
-    return (__double_as_longlong(p) << 1) == 0
-               ? __hiloint2double((__double2hiint(before) ^ (int)0x80000000) - (110 << 20), __double2loint(before))
-               : p;
-  };
+  auto zero = [](double p) { return (__double_as_longlong(p) << 1) == 0; };
   auto pivot = [](double t) { return (__double2hiint(t) & 0x7fffffff) < (1023 - 54) << 20 ? -0x1p-54 : t; };
   double p0 = 1.0, p1 = pivot(d[0] - x);
   int cnt = (unsigned)__double2hiint(p1) >> 31;
+  auto field = [&]() { return max((__double2hiint(p0) >> 20) & 0x7ff, (__double2hiint(p1) >> 20) & 0x7ff); };
+  auto next = [&](double p) {
+    cnt += (unsigned)(__double2hiint(p) ^ __double2hiint(p1)) >> 31;
+    p0 = p1;
+    p1 = p;
+  };
+  int e = field();
   for (int i0 = 1; i0 < n; i0 += 8) {
-    const int e = (max((__double2hiint(p0) >> 20) & 0x7ff, (__double2hiint(p1) >> 20) & 0x7ff));
     const double sc = __hiloint2double((2046 - e) << 20, 0);  // 2^(1023 - e): the larger one to [1, 2)
     p0 *= sc;
     p1 *= sc;
-    const int i1 = min(i0 + 8, n);
+    const double q0 = p0, q1 = p1;
+    const int c0 = cnt, i1 = min(i0 + 8, n);
 #pragma unroll 8
     for (int i = i0; i < i1; ++i) {
-      const double p = nonzero(fma(pivot(d[i] - x), p1, -(e2[i - 1] * p0)), p1);
-      cnt += (unsigned)(__double2hiint(p) ^ __double2hiint(p1)) >> 31;
-      p0 = p1;
-      p1 = p;
+      const double p = fma(d[i] - x, p1, -(e2[i - 1] * p0));
+      next(zero(p) ? __hiloint2double((__double2hiint(p1) & 0x80000000) ^ (int)0x80100000, 0) : p);  // -+ 2^-1022
+    }
+    e = field();
+    if (e < 1023 - 900) {
+      p0 = q0;
+      p1 = q1;
+      cnt = c0;
+#pragma unroll 1
+      for (int i = i0; i < i1; ++i) {
+        const double p = fma(pivot(d[i] - x), p1, -(e2[i - 1] * p0));
+        const int neg = __double2hiint(p1) ^ (int)0x80000000;
+        next(zero(p) ? __hiloint2double(neg - (110 << 20), __double2loint(p1)) : p);
+      }
+      e = field();
     }
   }
   return cnt;
