@@ -437,8 +437,10 @@ int wtb_batch_timings(const wtb_batch* batch, double* t_ms);
 int wtb_autotune_report(char* buf, int len);
 
 /* The contraction form of the context's last BSE operator: WTB_FORM_NONE (dense operator, or none built),
- * the split-BF16 tensor-core product, the FP32 or FP64 CUDA-core product, or the FP32 FFT convolution that
- * the FP32 matrix-free operator uses on a two-dimensional Monkhorst-Pack mesh of at most 64 x 64 points. */
+ * the split-BF16 tensor-core product, the FP32 or FP64 CUDA-core product, the FP32 FFT convolution that
+ * the FP32 matrix-free operator uses on a two-dimensional Monkhorst-Pack mesh of at most 64 x 64 points, or the
+ * FP64 one on a mesh of one to three dimensions (up to 80 x 80, 18^3 or 120 points): in applications and the
+ * adjoint's linear solves, and in solves of 3D meshes, of at most 6 excitons, or of 1,800 k-points and more. */
 enum { WTB_FORM_NONE = 0, WTB_FORM_TC_BF16 = 1, WTB_FORM_SIMT_F32 = 2, WTB_FORM_SIMT_F64 = 3, WTB_FORM_FFT_F32 = 4,
        WTB_FORM_FFT_F64 = 5 };
 int wtb_operator_form(const wtb_ctx* ctx);

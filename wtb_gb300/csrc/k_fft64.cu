@@ -22,9 +22,12 @@
 //      times S, inverse over dimension 1, over dimension 2; the m1 x m2 results on the mesh go back to the rows;
 //   C. inverse rows; the m3 results on the mesh go to T.
 // The second factor of dimension 1, the product with S and the inverse's first factor stay in registers.
-// Measured per 16-column application: 2.45 ms at 48 x 45, w = 12 (2,304 columns of 0.49 M FP64 instructions; the FP64
+// Measured per 16-column application: 2.45 ms at 48 x 45, w = 12 (2,304 columns of 0.52 M FP64 instructions; the FP64
 // pipe busy 79 % of the cycles; without the pruned stages and 96 points 3.04 ms of 0.61 M; the product 37.3 ms), 4.20 ms
 // at 11^3, w = 16 (4.48 and 24.5 ms).
+//
+// All rows of a column stay in one CTA's shared memory, so a mesh has a plan up to 80 x 80 (60 x 113, 120 x 56), 18^3 and
+// 120 points in one dimension; larger ones take the product.
 #include "wtb_internal.h"
 
 #include <algorithm>

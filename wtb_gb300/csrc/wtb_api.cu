@@ -410,18 +410,19 @@ int make_operator(wtb_ctx* c, const wtb_bse_params* p, int nbmax, OpBundle* ob, 
   c->last_form = WTB_FORM_NONE;
   // FP64 matrix-free operator on a Monkhorst-Pack mesh of any dimension: the same contraction in FP64, faster than the
   // product at every size measured (9.0 against 75 us at 2 x 2 and w = 6, 17 / 76 at 6 x 6, 79 / 212 at 12 x 12 and
-  // w = 8, 105 / 144 at 5^3, 2.45 / 37.3 ms at 48 x 45 and w = 12) and no less accurate: an application is off by 2.7e-16 of
-  // its norm at 24 x 24 where the product is by 4.4e-16, 3.8 / 6.2 at 48 x 45, 3.4 / 6.9 at 11^3.
+  // w = 8, 105 / 144 at 5^3, 2.45 / 37.3 ms at 48 x 45 and w = 12) and no less accurate: an application is off by
+  // 2.7e-16 of its norm at 24 x 24 where the product is by 4.4e-16, 3.8 / 6.2 at 48 x 45, 3.4 / 6.9 at 11^3.
   // Solves do not all take it, which is a choice about the digits beyond a solve's accuracy, not a bound of either form.
-  // Over 1,320 strained systems (2D 24 x 24 to 60 x 60, 3D 24 x 24 x 2 to 14^3, 4 to 14 excitons) both forms give the same
-  // energies to 2e-14 eV, and activities equally far from the 64-bit values, 2e-9 to 3e-7 relative, as a residual of 1e-8
-  // leaves them.  Between the forms activities differ by up to 1.4e-10 on 3D meshes, where solves take 4 to 8
-  // iterations (2.6e-9 in one of 25 further systems at 11^3), and in 2D by more the more iterations a solve takes (the search directions of its early converged
-  // columns are rounding noise, which the late ones use): below 1,800 points up to 6e-10 at 24 x 24; at 38 x 39 and 42 x 42
-  // by over 1e-9 (7e-9 at most) in none of the systems with w = 8 and 12 and up to 38 % with w = 10 for 4 and 6 excitons,
-  // in up to 81 % (1.4e-8) for 7 to 14; above by up to 5e-8.  2D solves for more than 6 excitons below 1,800 points keep the
-  // product and so the digits they had, at 2 to 8 times the cost (24 x 24 25 against 12 ms, 42 x 42 173 to 480 against 29 to
-  // 66); from 1,800 points on, where the product takes 0.2 to 2.3 s a solve, and for few excitons speed goes first.
+  // Over 1,320 strained systems (2D 24 x 24 to 60 x 60, 3D 24 x 24 x 2 to 14^3, 4 to 14 excitons) both forms give the
+  // same energies to 2e-14 eV, and activities equally far from the 64-bit values, 2e-9 to 3e-7 relative, as a residual of
+  // 1e-8 leaves them.  Between the forms activities differ by up to 1.4e-10 on 3D meshes, where solves take 4 to 8
+  // iterations (2.6e-9 in one of 25 further systems at 11^3), and in 2D by more the more iterations a solve takes (the
+  // search directions of its early converged columns are rounding noise, which the late ones use): below 1,800 points up
+  // to 6e-10 at 24 x 24; at 38 x 39 and 42 x 42 by over 1e-9 (7e-9 at most) in none of the systems with w = 8 and 12 and
+  // up to 38 % with w = 10 for 4 and 6 excitons, in up to 81 % (1.4e-8) for 7 to 14; above by up to 5e-8.  2D solves for
+  // more than 6 excitons below 1,800 points keep the product and so the digits they had, at 2 to 8 times the cost
+  // (24 x 24 25 against 12 ms, 42 x 42 173 to 480 against 29 to 66); from 1,800 points on, where the product takes 0.2 to
+  // 2.3 s a solve, and for few excitons speed goes first.
   const bool fp64 = p->precision == WTB_PREC_FP64;
   const bool mesh = c->mesh_mp && p->ngrid[0] == c->ngrid[0] && p->ngrid[1] == c->ngrid[1] &&
                     p->ngrid[2] == c->ngrid[2] && (long)p->ngrid[0] * p->ngrid[1] * p->ngrid[2] == nk;
