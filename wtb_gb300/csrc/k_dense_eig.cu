@@ -799,7 +799,7 @@ __global__ void tri_scale_kernel(const double* __restrict__ d, const double* __r
 // The first 20 bits come from FP32 counts of the rounded T (an FP32 instruction costs a sixtieth): their bracket,
 // widened by 2^-18 for the rounding (entries of at most 1, each off by a few 2^-24), is only where the first FP64
 // points lie, from its one end to the other inside the Gershgorin interval; the FP64 counts decide.  n = 1,520:
-// 4.6 -> 3.6 ms.
+// 4.6 -> 3.8 ms, 2,304: 6.9 -> 5.4.
 __global__ void __launch_bounds__(128) tri_multisect_kernel(const double* __restrict__ d,
                                                             const double* __restrict__ e2, int n,
                                                             const float* __restrict__ df,
@@ -1033,7 +1033,7 @@ __global__ void __launch_bounds__(256) tri_quantise_kernel(zd* __restrict__ A, i
 // v f run as exact integer sums (kQ above; the two 32-bit halves of z are its limbs, the lower one shortened to 28
 // bits; f quantised with an exponent of its own), f = tau v^H z itself in FP64.  Rounding: 2^-61 an update and entry, where FP64 has 2^-53 of the entry; v^H z
 // to 2^-56 of its terms.  Bound by the integer multiply-adds (24 an entry and reflector; the FP64 form 8 on a pipe
-// a twelfth as fast).  n = 1,520: 38.9 -> 16.1 ms.
+// a twelfth as fast).  n = 1,520: 38.9 -> 15.3 ms.
 // Z(i, k) = Z[i * n + k] (row-major), conjugated at the end when the solver worked on conj(H).
 // A row adds up to 2^56.6 to a low sum, so it is carried into the high one every kBtFold rows of a thread; columns in
 // shared memory have at most 50 and go without (the nested loop took n = 1,520 from 50.5 to 52.3 ms).
